@@ -6,22 +6,39 @@
 // decomposition on split fragments: Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br,
 // four DMMAs per 16x8 complex tile step.
 //
-// CTA tile 64x64 (complex), K step 16, double-buffered cp.async pipeline (one
-// barrier per 128 DMMAs of a warp; 80 KB, two CTAs per SM), 4 warps each
-// owning a 32x32 complex warp tile (2 x 4 DMMA tiles, real and imaginary
-// accumulators: 64 doubles per thread).  Tiles stay complex-interleaved in
-// shared memory so one 16-byte load yields both parts of an element; the
-// padded row strides (20 / 66 complex) make every 8-lane fragment load hit 8
-// distinct 16-byte bank groups.
+// K step 16, double-buffered cp.async pipeline, 4 warps, and two CTA tiles:
+//   64x64, warp tile 32x32, two CTAs per SM (80 KB each)
+//   32x32, warp tile 16x16, four CTAs per SM (40 KB each)
+// Bound by the DMMA pipe (87-90 % active in either form where the tiles fill
+// whole waves), so the choice is the one with the shorter last wave: see
+// launch_zgemm.  Per output element both run the same DMMA sequence, so the
+// result does not depend on the tile.
+//
+// Tried and not kept: three real products instead of four (Gauss's identity,
+// in either variant): 9 % faster at b = 256 (0.565 against 0.623 ms for 148
+// matrices; the fragment sums hold the shared FP64 pipe), but the surface
+// Green's functions of the decimation then end 1.3 times (1.16 times with the
+// chains cut in two) further from an extended-precision result.
+// Tiles stay complex-interleaved in shared memory so one 16-byte load yields
+// both parts of an element; the padded row strides (20 and 66 / 34 complex) make
+// every 8-lane fragment load hit 8 distinct 16-byte bank groups.
+#include <algorithm>
+
 #include "kernels.h"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, STAGES = 2, THREADS = 128;
-constexpr int LD_KMAJOR = BK + 4;   // tile stored [row][k]: 20 complex = 320 B rows
-constexpr int LD_MMAJOR = BM + 2;   // tile stored [k][row]: 66 complex = 1056 B rows
-constexpr int TILE_ELEMS = (BM * LD_KMAJOR > BK * LD_MMAJOR) ? BM * LD_KMAJOR : BK * LD_MMAJOR;
-constexpr int SMEM_BYTES = STAGES * 2 * TILE_ELEMS * (int)sizeof(cplx);
+constexpr int BK = 16, STAGES = 2, THREADS = 128;
+constexpr int LD_KMAJOR = BK + 4;  // tile stored [row][k]: 20 complex = 320 B rows
+
+template <int TILE>
+struct Cfg {
+  static constexpr int W = TILE / 2, MI = W / 16, NI = W / 8;  // warp tile W x W: MI x NI DMMA tiles
+  static constexpr int LD_MMAJOR = TILE + 2;                   // tile stored [k][row]: 66 / 34 complex
+  static constexpr int ELEMS = TILE * LD_KMAJOR > BK * LD_MMAJOR ? TILE * LD_KMAJOR : BK * LD_MMAJOR;
+  static constexpr int SMEM_BYTES = STAGES * 2 * ELEMS * (int)sizeof(cplx);
+  static constexpr int CTAS_PER_SM = TILE == 64 ? 2 : 4;
+};
 
 __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double b0) {
   asm volatile(
@@ -53,11 +70,11 @@ struct Params {
   const cplx* diag_shift;
 };
 
-// Load one K-slice of op(A) (BM x BK) into shared memory.
-template <int OPA>
+// Load one K-slice of op(A) (TILE x BK) into shared memory.
+template <int TILE, int OPA>
 __device__ __forceinline__ void load_a(cplx* sm, const Params& p, const cplx* a, int m0, int k0, int tid) {
 #pragma unroll
-  for (int r = 0; r < (BM * BK) / THREADS; ++r) {
+  for (int r = 0; r < (TILE * BK) / THREADS; ++r) {
     int idx = tid + r * THREADS;
     if (OPA == OP_N) {
       int row = idx / BK, col = idx % BK;  // A stored m x k
@@ -66,27 +83,27 @@ __device__ __forceinline__ void load_a(cplx* sm, const Params& p, const cplx* a,
       const cplx* src = ok ? a + (int64_t)gm * p.lda + gk : a;
       cp_async16(sm + row * LD_KMAJOR + col, src, ok);
     } else {
-      int krow = idx / BM, mcol = idx % BM;  // A stored k x m
+      int krow = idx / TILE, mcol = idx % TILE;  // A stored k x m
       int gk = k0 + krow, gm = m0 + mcol;
       bool ok = gm < p.m && gk < p.k;
       const cplx* src = ok ? a + (int64_t)gk * p.lda + gm : a;
-      cp_async16(sm + krow * LD_MMAJOR + mcol, src, ok);
+      cp_async16(sm + krow * Cfg<TILE>::LD_MMAJOR + mcol, src, ok);
     }
   }
 }
 
-// Load one K-slice of op(B) (BK x BN) into shared memory.
-template <int OPB>
+// Load one K-slice of op(B) (BK x TILE) into shared memory.
+template <int TILE, int OPB>
 __device__ __forceinline__ void load_b(cplx* sm, const Params& p, const cplx* b, int n0, int k0, int tid) {
 #pragma unroll
-  for (int r = 0; r < (BN * BK) / THREADS; ++r) {
+  for (int r = 0; r < (TILE * BK) / THREADS; ++r) {
     int idx = tid + r * THREADS;
     if (OPB == OP_N) {
-      int krow = idx / BN, ncol = idx % BN;  // B stored k x n
+      int krow = idx / TILE, ncol = idx % TILE;  // B stored k x n
       int gk = k0 + krow, gn = n0 + ncol;
       bool ok = gn < p.n && gk < p.k;
       const cplx* src = ok ? b + (int64_t)gk * p.ldb + gn : b;
-      cp_async16(sm + krow * LD_MMAJOR + ncol, src, ok);
+      cp_async16(sm + krow * Cfg<TILE>::LD_MMAJOR + ncol, src, ok);
     } else {
       int nrow = idx / BK, kcol = idx % BK;  // B stored n x k
       int gn = n0 + nrow, gk = k0 + kcol;
@@ -97,50 +114,87 @@ __device__ __forceinline__ void load_b(cplx* sm, const Params& p, const cplx* b,
   }
 }
 
-template <int OPA>
+template <int TILE, int OPA>
 __device__ __forceinline__ cplx frag_a(const cplx* sm, int m, int k) {
   if (OPA == OP_N) return sm[m * LD_KMAJOR + k];
-  cplx v = sm[k * LD_MMAJOR + m];
+  cplx v = sm[k * Cfg<TILE>::LD_MMAJOR + m];
   return make_double2(v.x, -v.y);
 }
-template <int OPB>
+template <int TILE, int OPB>
 __device__ __forceinline__ cplx frag_b(const cplx* sm, int k, int n) {
-  if (OPB == OP_N) return sm[k * LD_MMAJOR + n];
+  if (OPB == OP_N) return sm[k * Cfg<TILE>::LD_MMAJOR + n];
   cplx v = sm[n * LD_KMAJOR + k];
   return make_double2(v.x, -v.y);
 }
 
-template <int OPA, int OPB>
-__global__ void __launch_bounds__(THREADS, 2) zgemm_dmma_kernel(Params p) {
+// One K step of 4: fragments of lane (g, t) at rows / columns m + 16 mi (+ 8),
+// n + 8 ni and depth k, four DMMAs per complex tile.
+template <int TILE, int OPA, int OPB>
+__device__ __forceinline__ void mma_step(const cplx* sa, const cplx* sb, int m, int n, int k,
+                                         double (&acc_re)[Cfg<TILE>::MI][Cfg<TILE>::NI][4],
+                                         double (&acc_im)[Cfg<TILE>::MI][Cfg<TILE>::NI][4]) {
+  using C = Cfg<TILE>;
+  cplx af[C::MI][2], bf[C::NI];
+#pragma unroll
+  for (int mi = 0; mi < C::MI; ++mi) {
+    af[mi][0] = frag_a<TILE, OPA>(sa, m + mi * 16, k);
+    af[mi][1] = frag_a<TILE, OPA>(sa, m + mi * 16 + 8, k);
+  }
+#pragma unroll
+  for (int ni = 0; ni < C::NI; ++ni) bf[ni] = frag_b<TILE, OPB>(sb, k, n + ni * 8);
+  // first product of every accumulator, then the second (the order
+  // within each accumulator is unchanged: Ar Br, -Ai Bi / Ar Bi, Ai Br)
+#pragma unroll
+  for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < C::NI; ++ni) {
+      dmma(acc_re[mi][ni], af[mi][0].x, af[mi][1].x, bf[ni].x);
+      dmma(acc_im[mi][ni], af[mi][0].x, af[mi][1].x, bf[ni].y);
+    }
+#pragma unroll
+  for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < C::NI; ++ni) {
+      dmma(acc_re[mi][ni], -af[mi][0].y, -af[mi][1].y, bf[ni].y);
+      dmma(acc_im[mi][ni], af[mi][0].y, af[mi][1].y, bf[ni].x);
+    }
+}
+
+template <int TILE, int OPA, int OPB>
+__global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_kernel(Params p) {
+  using C = Cfg<TILE>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wm0 = (warp >> 1) * 32, wn0 = (warp & 1) * 32;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int wm0 = (warp >> 1) * C::W, wn0 = (warp & 1) * C::W;
+  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
   const int ktiles = (p.k + BK - 1) / BK;
+  // a warp tile outside the matrix only copies (small tile: the wide one is
+  // taken where the tiles are full)
+  const bool has_tile = m0 + wm0 < p.m && n0 + wn0 < p.n;
 
   for (int64_t e = blockIdx.z; e < p.batch; e += gridDim.z) {
     if (p.active && !p.active[e]) continue;
     const cplx* a = p.a + e * p.sa;
     const cplx* b = p.b + e * p.sb;
 
-    double acc_re[2][4][4], acc_im[2][4][4];
+    double acc_re[C::MI][C::NI][4], acc_im[C::MI][C::NI][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < C::MI; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < C::NI; ++j)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc_re[i][j][q] = acc_im[i][j][q] = 0.0;
 
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
       if (s < ktiles) {
-        cplx* sa = smem + s * 2 * TILE_ELEMS;
-        load_a<OPA>(sa, p, a, m0, s * BK, tid);
-        load_b<OPB>(sa + TILE_ELEMS, p, b, n0, s * BK, tid);
+        cplx* sa = smem + s * 2 * C::ELEMS;
+        load_a<TILE, OPA>(sa, p, a, m0, s * BK, tid);
+        load_b<TILE, OPB>(sa + C::ELEMS, p, b, n0, s * BK, tid);
       }
       cp_async_commit();
     }
@@ -151,41 +205,25 @@ __global__ void __launch_bounds__(THREADS, 2) zgemm_dmma_kernel(Params p) {
       {
         int nk = kt + STAGES - 1;
         if (nk < ktiles) {
-          cplx* sa = smem + (nk % STAGES) * 2 * TILE_ELEMS;
-          load_a<OPA>(sa, p, a, m0, nk * BK, tid);
-          load_b<OPB>(sa + TILE_ELEMS, p, b, n0, nk * BK, tid);
+          cplx* sa = smem + (nk % STAGES) * 2 * C::ELEMS;
+          load_a<TILE, OPA>(sa, p, a, m0, nk * BK, tid);
+          load_b<TILE, OPB>(sa + C::ELEMS, p, b, n0, nk * BK, tid);
         }
         cp_async_commit();
       }
-      const cplx* sa = smem + (kt % STAGES) * 2 * TILE_ELEMS;
-      const cplx* sb = sa + TILE_ELEMS;
-#pragma unroll
-      for (int kk = 0; kk < BK; kk += 4) {
-        cplx af[2][2], bf[4];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
-          af[mi][0] = frag_a<OPA>(sa, wm0 + mi * 16 + g, kk + t);
-          af[mi][1] = frag_a<OPA>(sa, wm0 + mi * 16 + g + 8, kk + t);
-        }
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) bf[ni] = frag_b<OPB>(sb, kk + t, wn0 + ni * 8 + g);
-        // first product of every accumulator, then the second (the order
-        // within each accumulator is unchanged: Ar Br, -Ai Bi / Ar Bi, Ai Br)
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) {
-            dmma(acc_re[mi][ni], af[mi][0].x, af[mi][1].x, bf[ni].x);
-            dmma(acc_im[mi][ni], af[mi][0].x, af[mi][1].x, bf[ni].y);
-          }
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) {
-            dmma(acc_re[mi][ni], -af[mi][0].y, -af[mi][1].y, bf[ni].y);
-            dmma(acc_im[mi][ni], af[mi][0].y, af[mi][1].y, bf[ni].x);
-          }
+      if (TILE == 32 && !has_tile) continue;
+      const cplx* sa = smem + (kt % STAGES) * 2 * C::ELEMS;
+      const cplx* sb = sa + C::ELEMS;
+      if (TILE == 32 && (kt + 1) * BK > p.k) {
+        // steps past k hold zeros and are left out
+#pragma unroll 1
+        for (int kk = 0; kk < p.k - kt * BK; kk += 4)
+          mma_step<TILE, OPA, OPB>(sa, sb, wm0 + g, wn0 + g, kk + t, acc_re, acc_im);
+        continue;
       }
+#pragma unroll
+      for (int kk = 0; kk < BK; kk += 4)
+        mma_step<TILE, OPA, OPB>(sa, sb, wm0 + g, wn0 + g, kk + t, acc_re, acc_im);
     }
     cp_async_wait<0>();
     __syncthreads();
@@ -195,9 +233,9 @@ __global__ void __launch_bounds__(THREADS, 2) zgemm_dmma_kernel(Params p) {
     const cplx* c = p.c ? p.c + e * p.sc : nullptr;
     const cplx* c2 = p.c2 ? p.c2 + e * p.sc2 : nullptr;
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi) {
+    for (int mi = 0; mi < C::MI; ++mi) {
 #pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
+      for (int ni = 0; ni < C::NI; ++ni) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           int row = m0 + wm0 + mi * 16 + g + ((q >> 1) << 3);
@@ -215,12 +253,38 @@ __global__ void __launch_bounds__(THREADS, 2) zgemm_dmma_kernel(Params p) {
   }
 }
 
-template <int OPA, int OPB>
+template <int TILE, int OPA, int OPB>
 void launch_t(const Params& p, cudaStream_t stream) {
+  constexpr int smem = Cfg<TILE>::SMEM_BYTES;
   // opt-in to the large shared-memory carve-out (per device)
-  qtx_opt_in_smem((const void*)zgemm_dmma_kernel<OPA, OPB>, SMEM_BYTES);
-  dim3 grid(ceil_div_u(p.n, BN), ceil_div_u(p.m, BM), (unsigned)(p.batch < 65535 ? p.batch : 65535));
-  zgemm_dmma_kernel<OPA, OPB><<<grid, THREADS, SMEM_BYTES, stream>>>(p);
+  qtx_opt_in_smem((const void*)zgemm_dmma_kernel<TILE, OPA, OPB>, smem);
+  dim3 grid(ceil_div_u(p.n, TILE), ceil_div_u(p.m, TILE), (unsigned)(p.batch < 65535 ? p.batch : 65535));
+  zgemm_dmma_kernel<TILE, OPA, OPB><<<grid, THREADS, smem, stream>>>(p);
+}
+
+// The tile whose waves finish first.  A full wave of 64x64 tiles covers twice
+// the outputs of a full wave of 32x32 ones in twice the time, less about
+// 1.5 % (b = 256, 148 matrices, 8.0 waves: 0.614 ms against 0.623 ms).  A
+// nearly empty last wave costs more than that: 32x32 / 64x64 tiles take
+// 9.0 / 17.4 us for 32 matrices of b = 64, 17.9 / 24.0 us for 24 of b = 100,
+// 66 / 86 us for 100 of b = 128, 0.796 / 0.878 ms for 24 of b = 512; 84 / 81
+// us for 16 of b = 256 (two waves against one).
+bool wide_tile(const Params& p) {
+  if (p.m > 32 * 65535) return true;  // grid.y
+  int dev = 0, sms = 0;
+  QTX_CUDA_TRY(cudaGetDevice(&dev));
+  QTX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  auto waves = [&](int64_t tile, int64_t resident) {
+    const int64_t tiles = ((p.m + tile - 1) / tile) * ((p.n + tile - 1) / tile) * p.batch;
+    return (tiles + resident * sms - 1) / (resident * sms);
+  };
+  return 0.985 * 2.0 * (double)waves(64, Cfg<64>::CTAS_PER_SM) <= (double)waves(32, Cfg<32>::CTAS_PER_SM);
+}
+
+template <int OPA, int OPB>
+void launch_op(const Params& p, cudaStream_t stream) {
+  if (wide_tile(p)) launch_t<64, OPA, OPB>(p, stream);
+  else launch_t<32, OPA, OPB>(p, stream);
 }
 
 }  // namespace
@@ -236,9 +300,9 @@ void launch_zgemm(const GemmCall& g, cudaStream_t stream) {
   p.d = g.d.ptr; p.ldd = g.d.ld; p.sd = g.d.stride; p.alpha = g.alpha;
   p.active = g.active;
   p.diag_shift = g.diag_shift;
-  if (g.op_a == OP_N && g.op_b == OP_N) launch_t<OP_N, OP_N>(p, stream);
-  else if (g.op_a == OP_N && g.op_b == OP_C) launch_t<OP_N, OP_C>(p, stream);
-  else if (g.op_a == OP_C && g.op_b == OP_N) launch_t<OP_C, OP_N>(p, stream);
-  else launch_t<OP_C, OP_C>(p, stream);
+  if (g.op_a == OP_N && g.op_b == OP_N) launch_op<OP_N, OP_N>(p, stream);
+  else if (g.op_a == OP_N && g.op_b == OP_C) launch_op<OP_N, OP_C>(p, stream);
+  else if (g.op_a == OP_C && g.op_b == OP_N) launch_op<OP_C, OP_N>(p, stream);
+  else launch_op<OP_C, OP_C>(p, stream);
   qtx_check_launch("zgemm_dmma_kernel");
 }

@@ -59,6 +59,26 @@ def test_zgemm_matches_torch(m, n, k, op_a, op_b):
     assert _rel(d, ref) < 1e-13
 
 
+@pytest.mark.parametrize("op_a,op_b", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("n,batch", [(63, 296), (64, 296), (97, 148), (128, 148), (161, 296)])
+def test_zgemm_result_does_not_depend_on_the_tile(n, batch, op_a, op_b):
+    """A single product takes the 32 x 32 tile, a batch that fills whole waves
+    of the GPU the 64 x 64 one; both run the same sequence per element, so the
+    results agree bit for bit (edges of both tiles, one row or column past
+    them included)."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a, b = (torch.randn(batch, n, n, dtype=torch.complex128, device="cuda", generator=g) for _ in range(2))
+    big = torch.empty_like(a)
+    _zgemm(n, n, n, batch, 1.0 + 0.5j, a, op_a, b, op_b, 0j, None, big)
+    one = torch.empty_like(a[:1])
+    for e in (0, batch - 1):
+        _zgemm(n, n, n, 1, 1.0 + 0.5j, a[e:e + 1].contiguous(), op_a, b[e:e + 1].contiguous(), op_b, 0j, None, one)
+        assert torch.equal(one[0], big[e])
+    want = (1.0 + 0.5j) * (a.mH if op_a else a) @ (b.mH if op_b else b)
+    # two chains of 2 n products each, rounded once a step
+    assert _rel(big, want.cpu().numpy()) < 4 * n * 2.0**-53
+
+
 def test_zgemm_broadcast_operand():
     g = torch.Generator().manual_seed(5)
     a = _crand(g, 1, 48, 48)
