@@ -22,6 +22,7 @@ inline unsigned grid_for(int64_t work) {
 // out = s + w^H - w, square n x n; tiles of 32x32 for the transposed read
 __global__ void skew_combine_kernel(int n, int64_t batch, const cplx* s, int64_t lds, int64_t ss, const cplx* w,
                                     int64_t ldw, int64_t sw, cplx* out, int64_t ldo, int64_t so) {
+  qtx_grid_dependency();
   __shared__ cplx tile[32][33];
   const int tiles = (n + 31) / 32;
   const int64_t total = batch * tiles * tiles;
@@ -55,6 +56,7 @@ __global__ void skew_combine_kernel(int n, int64_t batch, const cplx* s, int64_t
 // coalesced.  The same arithmetic per element as sub_herm_kernel.
 __global__ void __launch_bounds__(256)
     sub_herm_tiled_kernel(int n, int64_t batch, cplx* x, int64_t ld, int64_t sx) {
+  qtx_grid_dependency();
   __shared__ cplx ta[32][33], tb[32][33];
   const int nt = (n + 31) / 32;
   // triangular index -> (ti, tj), ti <= tj, row-major over the upper triangle
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(256)
 // x <- x - x^H in place (small blocks): each thread owns the pair (r, c), (c, r)
 // with r <= c
 __global__ void sub_herm_kernel(int n, int64_t batch, cplx* x, int64_t ld, int64_t sx) {
+  qtx_grid_dependency();
   const int64_t pairs = (int64_t)n * (n + 1) / 2;
   const int64_t total = batch * pairs;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -119,6 +122,7 @@ __global__ void sub_herm_kernel(int n, int64_t batch, cplx* x, int64_t ld, int64
 __global__ void axpby_kernel(int rows, int cols, int64_t batch, cplx alpha, const cplx* x, int64_t ldx, int64_t sx,
                              cplx beta, const cplx* y, int64_t ldy, int64_t sy, cplx* out, int64_t ldo, int64_t so,
                              const int* active) {
+  qtx_grid_dependency();
   const int64_t per = (int64_t)rows * cols;
   const int64_t total = batch * per;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -137,6 +141,7 @@ __global__ void axpby_kernel(int rows, int cols, int64_t batch, cplx alpha, cons
 // `rows`/`cols` are the shape of the STORED block)
 __global__ void block_scatter_kernel(int rows, int cols, int64_t batch, const cplx* x, int64_t ldx, int64_t sx,
                                      int mode, cplx* data, int64_t stride, int64_t nnz, const int32_t* index) {
+  qtx_grid_dependency();
   const int64_t total = batch * nnz;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t e = t / nnz;
@@ -161,6 +166,7 @@ __global__ void block_scatter_kernel(int rows, int cols, int64_t batch, const cp
 
 __global__ void block_gather_kernel(int rows, int cols, int64_t batch, const cplx* data, int64_t stride, int64_t nnz,
                                     const int32_t* index, cplx* out, int64_t ldo, int64_t so) {
+  qtx_grid_dependency();
   // zero the dense block first (grid-stride), then scatter the entries
   const int64_t per = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < batch * per; t += (int64_t)gridDim.x * blockDim.x) {
@@ -171,6 +177,7 @@ __global__ void block_gather_kernel(int rows, int cols, int64_t batch, const cpl
 }
 __global__ void block_gather_fill_kernel(int rows, int cols, int64_t batch, const cplx* data, int64_t stride,
                                          int64_t nnz, const int32_t* index, cplx* out, int64_t ldo, int64_t so) {
+  qtx_grid_dependency();
   const int64_t total = batch * nnz;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t e = t / nnz;
@@ -211,6 +218,7 @@ __device__ cplx block_sum(cplx v) {
 
 __global__ void trace_product_kernel(int rows, int cols, int64_t batch, const cplx* x, int64_t ldx, int64_t sx,
                                      const cplx* y, int64_t ldy, int64_t sy, cplx scale, cplx* tr, int accumulate) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     cplx acc = cmk(0, 0);
     for (int q = threadIdx.x; q < rows * cols; q += blockDim.x) {
@@ -227,6 +235,7 @@ __global__ void trace_product_kernel(int rows, int cols, int64_t batch, const cp
 
 __global__ void trace_product_h_kernel(int rows, int cols, int64_t batch, const cplx* x, int64_t ldx, int64_t sx,
                                        const cplx* y, int64_t ldy, int64_t sy, cplx* tr) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     cplx acc = cmk(0, 0);
     for (int q = threadIdx.x; q < rows * cols; q += blockDim.x) {
@@ -252,6 +261,7 @@ __device__ __forceinline__ double sr_norm_term(cplx av, cplx bv) {
 __global__ void __launch_bounds__(SRN_THREADS)
     sr_norm_kernel(int n, int64_t batch, const cplx* a, int64_t lda, int64_t sa, const cplx* b, int64_t ldb,
                    int64_t sb, double tol, int* active, int* iterations, int* num_active) {
+  qtx_grid_dependency();
   const int nn = n * n;
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     if (!active[e]) continue;
@@ -286,6 +296,7 @@ __global__ void __launch_bounds__(SRN_THREADS)
 
 __global__ void assemble_diag_kernel(int n, int64_t batch, const cplx* h, const double* energies, double eta,
                                      cplx* out, int64_t ldo, int64_t so) {
+  qtx_grid_dependency();
   const int64_t per = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < batch * per; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t e = t / per;
@@ -302,6 +313,7 @@ __global__ void assemble_diag_kernel(int n, int64_t batch, const cplx* h, const 
 }
 
 __global__ void neg_herm_kernel(int n, const cplx* h, cplx* out) {
+  qtx_grid_dependency();
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * n; q += gridDim.x * blockDim.x) {
     int r = q / n, c = q % n;
     cplx v = h[(int64_t)c * n + r];
@@ -312,6 +324,7 @@ __global__ void neg_herm_kernel(int n, const cplx* h, cplx* out) {
 __global__ void obc_lg_kernel(int n, int64_t batch, const cplx* s, int64_t lds, int64_t ss, const double* occ,
                               cplx* sl, int64_t ldl, int64_t sls, cplx* sg, int64_t ldg, int64_t sgs, cplx* gam,
                               int64_t ldgam, int64_t sgam) {
+  qtx_grid_dependency();
   const int64_t per = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < batch * per; t += (int64_t)gridDim.x * blockDim.x) {
     int64_t e = t / per;
@@ -332,11 +345,13 @@ __global__ void obc_lg_kernel(int n, int64_t batch, const cplx* s, int64_t lds, 
 }
 
 __global__ void fermi_kernel(int64_t batch, const double* energies, double mu, double kt, double* occ) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch; e += (int64_t)gridDim.x * blockDim.x)
     occ[e] = 1.0 / (1.0 + exp((energies[e] - mu) / kt));
 }
 
 __global__ void fill_int_kernel(int* p, int64_t count, int value) {
+  qtx_grid_dependency();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x)
     p[t] = value;
 }
@@ -348,6 +363,7 @@ template <int OPX, int OPY>
 __global__ void block_combine_kernel(int rows, int cols, int64_t batch, cplx alpha, const cplx* x, int64_t ldx,
                                      int64_t sx, cplx beta, const cplx* y, int64_t ldy, int64_t sy, cplx* out,
                                      int64_t ldo, int64_t so) {
+  qtx_grid_dependency();
   __shared__ cplx tx[32][33];
   __shared__ cplx ty[32][33];
   const int tiles_c = (cols + 31) / 32;
@@ -388,6 +404,7 @@ __global__ void block_combine_kernel(int rows, int cols, int64_t batch, cplx alp
 // entry, out[2] = src[0].  (A cudaMemcpy of a status word queues behind any
 // large device-to-host copy in flight on the copy engine.)
 __global__ void flag_reduce_kernel(const int* src, int64_t n, int* out) {
+  qtx_grid_dependency();
   __shared__ unsigned long long first;
   if (threadIdx.x == 0) first = ~0ull;
   __syncthreads();
@@ -409,6 +426,7 @@ __global__ void flag_reduce_kernel(const int* src, int64_t n, int* out) {
 // Slice k is entries [slices[2k], slices[2k] + slices[2k + 1]) of every row.
 __global__ void block_nonzero_kernel(const int64_t* slices, const cplx* data, int64_t stride, int64_t rows,
                                      int* flags) {
+  qtx_grid_dependency();
   const int k = blockIdx.y;
   const int64_t off = slices[2 * k], nnz = slices[2 * k + 1];
   if (off < 0 || nnz <= 0) return;
@@ -429,11 +447,13 @@ __global__ void block_nonzero_kernel(const int64_t* slices, const cplx* data, in
 }
 
 __global__ void copy_int_kernel(int* dst, int64_t dst_stride, const int* src, int64_t src_stride, int64_t count) {
+  qtx_grid_dependency();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x)
     dst[t * dst_stride] = src[t * src_stride];
 }
 
 __global__ void real_part_kernel(int64_t count, const cplx* src, double* dst) {
+  qtx_grid_dependency();
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < count; t += (int64_t)gridDim.x * blockDim.x)
     dst[t] = src[t].x;
 }
@@ -444,6 +464,7 @@ namespace {
 // abs_res[e] = ||x_ref - x||_F, rel_res[e] = abs_res[e] / ||x_ref||_F
 __global__ void residual_norm_kernel(int n, int64_t batch, const cplx* xr, int64_t sr, const cplx* x, int64_t sx,
                                      double* abs_res, double* rel_res) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     double d2 = 0, r2 = 0;
     for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
@@ -464,14 +485,15 @@ __global__ void residual_norm_kernel(int n, int64_t batch, const cplx* xr, int64
 void launch_residual_norm(int n, int64_t batch, MatView x_ref, MatView x, double* abs_res, double* rel_res,
                           cudaStream_t stream) {
   unsigned g = (unsigned)(batch < 65535 ? batch : 65535);
-  residual_norm_kernel<<<g, TB, 0, stream>>>(n, batch, x_ref.ptr, x_ref.stride, x.ptr, x.stride, abs_res, rel_res);
+  qtx_launch(residual_norm_kernel, g, TB, 0, stream, n, batch, x_ref.ptr, x_ref.stride, x.ptr, x.stride, abs_res,
+             rel_res);
   qtx_check_launch("residual_norm_kernel");
 }
 
 void launch_skew_combine(int n, int64_t batch, MatView s, MatView w, MutView out, cudaStream_t stream) {
   int tiles = (n + 31) / 32;
-  skew_combine_kernel<<<grid_for(batch * tiles * tiles * TB), TB, 0, stream>>>(
-      n, batch, s.ptr, s.ld, s.stride, w.ptr, w.ld, w.stride, out.ptr, out.ld, out.stride);
+  qtx_launch(skew_combine_kernel, grid_for(batch * tiles * tiles * TB), TB, 0, stream, n, batch, s.ptr, s.ld,
+             s.stride, w.ptr, w.ld, w.stride, out.ptr, out.ld, out.stride);
   qtx_check_launch("skew_combine_kernel");
 }
 
@@ -481,65 +503,66 @@ void launch_sub_herm_inplace(int n, int64_t batch, MutView x, cudaStream_t strea
     const int nt = (n + 31) / 32;
     const unsigned pairs = (unsigned)(nt * (nt + 1) / 2);
     const unsigned gy = (unsigned)(batch < 65535 ? batch : 65535);
-    sub_herm_tiled_kernel<<<dim3(pairs, gy), 256, 0, stream>>>(n, batch, x.ptr, x.ld, x.stride);
+    qtx_launch(sub_herm_tiled_kernel, dim3(pairs, gy), 256, 0, stream, n, batch, x.ptr, x.ld, x.stride);
     qtx_check_launch("sub_herm_tiled_kernel");
     return;
   }
-  sub_herm_kernel<<<grid_for(batch * (int64_t)n * (n + 1) / 2), TB, 0, stream>>>(n, batch, x.ptr, x.ld, x.stride);
+  qtx_launch(sub_herm_kernel, grid_for(batch * (int64_t)n * (n + 1) / 2), TB, 0, stream, n, batch, x.ptr, x.ld,
+             x.stride);
   qtx_check_launch("sub_herm_kernel");
 }
 
 void launch_axpby(int rows, int cols, int64_t batch, cplx alpha, MatView x, cplx beta, MatView y, MutView out,
                   cudaStream_t stream, const int* active) {
-  axpby_kernel<<<grid_for(batch * (int64_t)rows * cols), TB, 0, stream>>>(
-      rows, cols, batch, alpha, x.ptr, x.ld, x.stride, beta, y.ptr, y.ld, y.stride, out.ptr, out.ld, out.stride,
-      active);
+  qtx_launch(axpby_kernel, grid_for(batch * (int64_t)rows * cols), TB, 0, stream, rows, cols, batch, alpha, x.ptr,
+             x.ld, x.stride, beta, y.ptr, y.ld, y.stride, out.ptr, out.ld, out.stride, active);
   qtx_check_launch("axpby_kernel");
 }
 
 namespace {
 __global__ void energy_shift_kernel(int64_t batch, const double* energies, double eta, cplx* shift) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < batch; e += (int64_t)gridDim.x * blockDim.x)
     shift[e] = cmk(energies[e], eta);
 }
 }  // namespace
 
 void launch_energy_shift(int64_t batch, const double* energies, double eta, cplx* shift, cudaStream_t stream) {
-  energy_shift_kernel<<<grid_for(batch), TB, 0, stream>>>(batch, energies, eta, shift);
+  qtx_launch(energy_shift_kernel, grid_for(batch), TB, 0, stream, batch, energies, eta, shift);
   qtx_check_launch("energy_shift_kernel");
 }
 
 void launch_block_scatter(int rows, int cols, int64_t batch, MatView x, int mode, cplx* data, int64_t stride,
                           int64_t nnz, const int32_t* index, cudaStream_t stream) {
   if (nnz <= 0) return;
-  block_scatter_kernel<<<grid_for(batch * nnz), TB, 0, stream>>>(rows, cols, batch, x.ptr, x.ld, x.stride, mode,
-                                                                 data, stride, nnz, index);
+  qtx_launch(block_scatter_kernel, grid_for(batch * nnz), TB, 0, stream, rows, cols, batch, x.ptr, x.ld, x.stride,
+             mode, data, stride, nnz, index);
   qtx_check_launch("block_scatter_kernel");
 }
 
 void launch_block_gather(int rows, int cols, int64_t batch, const cplx* data, int64_t stride, int64_t nnz,
                          const int32_t* index, MutView out, cudaStream_t stream) {
-  block_gather_kernel<<<grid_for(batch * (int64_t)rows * cols), TB, 0, stream>>>(rows, cols, batch, data, stride,
-                                                                                nnz, index, out.ptr, out.ld,
-                                                                                out.stride);
+  qtx_launch(block_gather_kernel, grid_for(batch * (int64_t)rows * cols), TB, 0, stream, rows, cols, batch, data,
+             stride, nnz, index, out.ptr, out.ld, out.stride);
   qtx_check_launch("block_gather_kernel");
   if (nnz <= 0) return;
-  block_gather_fill_kernel<<<grid_for(batch * nnz), TB, 0, stream>>>(rows, cols, batch, data, stride, nnz, index,
-                                                                     out.ptr, out.ld, out.stride);
+  qtx_launch(block_gather_fill_kernel, grid_for(batch * nnz), TB, 0, stream, rows, cols, batch, data, stride, nnz,
+             index, out.ptr, out.ld, out.stride);
   qtx_check_launch("block_gather_fill_kernel");
 }
 
 void launch_trace_product(int rows, int cols, int64_t batch, MatView x, MatView y, cplx scale, cplx* tr,
                           bool accumulate, cudaStream_t stream) {
   unsigned g = (unsigned)(batch < 65535 ? batch : 65535);
-  trace_product_kernel<<<g, TB, 0, stream>>>(rows, cols, batch, x.ptr, x.ld, x.stride, y.ptr, y.ld, y.stride, scale,
-                                             tr, accumulate ? 1 : 0);
+  qtx_launch(trace_product_kernel, g, TB, 0, stream, rows, cols, batch, x.ptr, x.ld, x.stride, y.ptr, y.ld, y.stride,
+             scale, tr, accumulate ? 1 : 0);
   qtx_check_launch("trace_product_kernel");
 }
 
 void launch_trace_product_h(int rows, int cols, int64_t batch, MatView x, MatView y, cplx* tr, cudaStream_t stream) {
   unsigned g = (unsigned)(batch < 65535 ? batch : 65535);
-  trace_product_h_kernel<<<g, TB, 0, stream>>>(rows, cols, batch, x.ptr, x.ld, x.stride, y.ptr, y.ld, y.stride, tr);
+  qtx_launch(trace_product_h_kernel, g, TB, 0, stream, rows, cols, batch, x.ptr, x.ld, x.stride, y.ptr, y.ld,
+             y.stride, tr);
   qtx_check_launch("trace_product_h_kernel");
 }
 
@@ -547,45 +570,44 @@ void launch_trace_product_h(int rows, int cols, int64_t batch, MatView x, MatVie
 void launch_sr_norm_update(int n, int64_t batch, MatView alpha, MatView beta, double tol, int* active,
                            int* iterations, int* num_active, cudaStream_t stream) {
   unsigned g = (unsigned)(batch < 65535 ? batch : 65535);
-  sr_norm_kernel<<<g, SRN_THREADS, 0, stream>>>(n, batch, alpha.ptr, alpha.ld, alpha.stride, beta.ptr, beta.ld,
-                                                beta.stride, tol, active, iterations, num_active);
+  qtx_launch(sr_norm_kernel, g, SRN_THREADS, 0, stream, n, batch, alpha.ptr, alpha.ld, alpha.stride, beta.ptr,
+             beta.ld, beta.stride, tol, active, iterations, num_active);
   qtx_check_launch("sr_norm_kernel");
 }
 
 void launch_assemble_diag(int n, int64_t batch, const cplx* h, const double* energies, double eta, MutView out,
                           cudaStream_t stream) {
-  assemble_diag_kernel<<<grid_for(batch * (int64_t)n * n), TB, 0, stream>>>(n, batch, h, energies, eta, out.ptr,
-                                                                            out.ld, out.stride);
+  qtx_launch(assemble_diag_kernel, grid_for(batch * (int64_t)n * n), TB, 0, stream, n, batch, h, energies, eta,
+             out.ptr, out.ld, out.stride);
   qtx_check_launch("assemble_diag_kernel");
 }
 
 void launch_neg_herm(int n, const cplx* h, cplx* out, cudaStream_t stream) {
-  neg_herm_kernel<<<grid_for((int64_t)n * n), TB, 0, stream>>>(n, h, out);
+  qtx_launch(neg_herm_kernel, grid_for((int64_t)n * n), TB, 0, stream, n, h, out);
   qtx_check_launch("neg_herm_kernel");
 }
 
 void launch_obc_lesser_greater(int n, int64_t batch, MatView sigma_r, const double* occ, MutView sl, MutView sg,
                                MutView gamma, cudaStream_t stream) {
-  obc_lg_kernel<<<grid_for(batch * (int64_t)n * n), TB, 0, stream>>>(n, batch, sigma_r.ptr, sigma_r.ld,
-                                                                     sigma_r.stride, occ, sl.ptr, sl.ld, sl.stride,
-                                                                     sg.ptr, sg.ld, sg.stride, gamma.ptr, gamma.ld,
-                                                                     gamma.stride);
+  qtx_launch(obc_lg_kernel, grid_for(batch * (int64_t)n * n), TB, 0, stream, n, batch, sigma_r.ptr, sigma_r.ld,
+             sigma_r.stride, occ, sl.ptr, sl.ld, sl.stride, sg.ptr, sg.ld, sg.stride, gamma.ptr, gamma.ld,
+             gamma.stride);
   qtx_check_launch("obc_lg_kernel");
 }
 
 void launch_fermi(int64_t batch, const double* energies, double mu, double kt, double* occ, cudaStream_t stream) {
-  fermi_kernel<<<grid_for(batch), TB, 0, stream>>>(batch, energies, mu, kt, occ);
+  qtx_launch(fermi_kernel, grid_for(batch), TB, 0, stream, batch, energies, mu, kt, occ);
   qtx_check_launch("fermi_kernel");
 }
 
 void launch_fill_int(int* p, int64_t count, int value, cudaStream_t stream) {
   if (count <= 0) return;
-  fill_int_kernel<<<grid_for(count), TB, 0, stream>>>(p, count, value);
+  qtx_launch(fill_int_kernel, grid_for(count), TB, 0, stream, p, count, value);
   qtx_check_launch("fill_int_kernel");
 }
 
 void launch_flag_reduce(const int* src, int64_t n, int* mapped_out, cudaStream_t stream) {
-  flag_reduce_kernel<<<1, 256, 0, stream>>>(src, n, mapped_out);
+  qtx_launch(flag_reduce_kernel, 1, 256, 0, stream, src, n, mapped_out);
   qtx_check_launch("flag_reduce_kernel");
 }
 
@@ -596,17 +618,17 @@ void launch_block_combine(int rows, int cols, int64_t batch, cplx alpha, MatView
   const dim3 grid(tiles, (unsigned)std::min<int64_t>(batch, 65535));
   const cplx* yp = y.ptr;
   if (op_x == OP_N && op_y == OP_N)
-    block_combine_kernel<0, 0><<<grid, 256, 0, stream>>>(rows, cols, batch, alpha, x.ptr, x.ld, x.stride, beta, yp,
-                                                         y.ld, y.stride, out.ptr, out.ld, out.stride);
+    qtx_launch(block_combine_kernel<0, 0>, grid, 256, 0, stream, rows, cols, batch, alpha, x.ptr, x.ld, x.stride,
+               beta, yp, y.ld, y.stride, out.ptr, out.ld, out.stride);
   else if (op_x == OP_C && op_y == OP_N)
-    block_combine_kernel<1, 0><<<grid, 256, 0, stream>>>(rows, cols, batch, alpha, x.ptr, x.ld, x.stride, beta, yp,
-                                                         y.ld, y.stride, out.ptr, out.ld, out.stride);
+    qtx_launch(block_combine_kernel<1, 0>, grid, 256, 0, stream, rows, cols, batch, alpha, x.ptr, x.ld, x.stride,
+               beta, yp, y.ld, y.stride, out.ptr, out.ld, out.stride);
   else if (op_x == OP_N && op_y == OP_C)
-    block_combine_kernel<0, 1><<<grid, 256, 0, stream>>>(rows, cols, batch, alpha, x.ptr, x.ld, x.stride, beta, yp,
-                                                         y.ld, y.stride, out.ptr, out.ld, out.stride);
+    qtx_launch(block_combine_kernel<0, 1>, grid, 256, 0, stream, rows, cols, batch, alpha, x.ptr, x.ld, x.stride,
+               beta, yp, y.ld, y.stride, out.ptr, out.ld, out.stride);
   else
-    block_combine_kernel<1, 1><<<grid, 256, 0, stream>>>(rows, cols, batch, alpha, x.ptr, x.ld, x.stride, beta, yp,
-                                                         y.ld, y.stride, out.ptr, out.ld, out.stride);
+    qtx_launch(block_combine_kernel<1, 1>, grid, 256, 0, stream, rows, cols, batch, alpha, x.ptr, x.ld, x.stride,
+               beta, yp, y.ld, y.stride, out.ptr, out.ld, out.stride);
   qtx_check_launch("block_combine_kernel");
 }
 
@@ -614,20 +636,20 @@ void launch_block_nonzero(int num_slices, const int64_t* slices, const cplx* dat
                           int* flags, cudaStream_t stream) {
   if (num_slices <= 0 || rows <= 0) return;
   const unsigned gx = (unsigned)std::min<int64_t>(rows, 256);
-  block_nonzero_kernel<<<dim3(gx, (unsigned)num_slices), TB, 0, stream>>>(slices, data, stride, rows, flags);
+  qtx_launch(block_nonzero_kernel, dim3(gx, (unsigned)num_slices), TB, 0, stream, slices, data, stride, rows, flags);
   qtx_check_launch("block_nonzero_kernel");
 }
 
 void launch_copy_int(int* dst, int64_t dst_stride, const int* src, int64_t src_stride, int64_t count,
                      cudaStream_t stream) {
   if (count <= 0) return;
-  copy_int_kernel<<<grid_for(count), TB, 0, stream>>>(dst, dst_stride, src, src_stride, count);
+  qtx_launch(copy_int_kernel, grid_for(count), TB, 0, stream, dst, dst_stride, src, src_stride, count);
   qtx_check_launch("copy_int_kernel");
 }
 
 void launch_real_part(int64_t count, const cplx* src, double* dst, cudaStream_t stream) {
   if (count <= 0) return;
-  real_part_kernel<<<grid_for(count), TB, 0, stream>>>(count, src, dst);
+  qtx_launch(real_part_kernel, grid_for(count), TB, 0, stream, count, src, dst);
   qtx_check_launch("real_part_kernel");
 }
 
@@ -635,6 +657,7 @@ namespace {
 __global__ void keldysh_combine_kernel(int n, int64_t batch, const cplx* xl, int64_t ldl, int64_t sl, const cplx* xr,
                                        int64_t ldr, int64_t sr, const double* occ_l, const double* occ_r,
                                        double sign_r, int sym, cplx* out_l, int64_t so_l, cplx* out_g, int64_t so_g) {
+  qtx_grid_dependency();
   const int64_t per = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < batch * per; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t e = t / per;
@@ -659,6 +682,7 @@ __global__ void keldysh_combine_kernel(int n, int64_t batch, const cplx* xl, int
 __global__ void keldysh_density_kernel(int n, int64_t batch, const cplx* xl, int64_t ldl, int64_t sl, const cplx* xr,
                                        int64_t ldr, int64_t sr, const double* occ_l, const double* occ_r,
                                        double* density, double* hole, int64_t out_stride, int out_col) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     const double fl = occ_l[e], fr = occ_r[e];
     double dl = 0, dg = 0;
@@ -680,9 +704,8 @@ void launch_keldysh_combine(int n, int64_t batch, MatView xl, MatView xr, const 
                             double sign_r, bool sym, cplx* out_l, int64_t stride_l, cplx* out_g, int64_t stride_g,
                             cudaStream_t stream) {
   if (!out_l && !out_g) return;
-  keldysh_combine_kernel<<<grid_for(batch * (int64_t)n * n), TB, 0, stream>>>(
-      n, batch, xl.ptr, xl.ld, xl.stride, xr.ptr, xr.ld, xr.stride, occ_l, occ_r, sign_r, sym ? 1 : 0, out_l, stride_l,
-      out_g, stride_g);
+  qtx_launch(keldysh_combine_kernel, grid_for(batch * (int64_t)n * n), TB, 0, stream, n, batch, xl.ptr, xl.ld,
+             xl.stride, xr.ptr, xr.ld, xr.stride, occ_l, occ_r, sign_r, sym ? 1 : 0, out_l, stride_l, out_g, stride_g);
   qtx_check_launch("keldysh_combine_kernel");
 }
 
@@ -690,14 +713,15 @@ void launch_keldysh_density(int n, int64_t batch, MatView xl, MatView xr, const 
                             double* density, double* hole, int64_t out_stride, int out_col, cudaStream_t stream) {
   if (!density && !hole) return;
   const unsigned g = (unsigned)(batch < 65535 ? batch : 65535);
-  keldysh_density_kernel<<<g, TB, 0, stream>>>(n, batch, xl.ptr, xl.ld, xl.stride, xr.ptr, xr.ld, xr.stride, occ_l,
-                                                occ_r, density, hole, out_stride, out_col);
+  qtx_launch(keldysh_density_kernel, g, TB, 0, stream, n, batch, xl.ptr, xl.ld, xl.stride, xr.ptr, xr.ld, xr.stride,
+             occ_l, occ_r, density, hole, out_stride, out_col);
   qtx_check_launch("keldysh_density_kernel");
 }
 
 namespace {
 __global__ void block_dos_kernel(int n, int64_t batch, const cplx* g, int64_t ld, int64_t sg, double* out,
                                  int64_t out_stride, int out_col) {
+  qtx_grid_dependency();
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     double acc = 0;
     for (int r = threadIdx.x; r < n; r += blockDim.x) acc += g[e * sg + (int64_t)r * ld + r].y;
@@ -719,6 +743,7 @@ __global__ void __launch_bounds__(LC_THREADS)
     layer_current_kernel(int n, int64_t batch, const cplx* xl, int64_t ldl, int64_t sl, const cplx* xr,
                          int64_t ldr, int64_t sr, const double* occ_l, const double* occ_r, double sign_r,
                          const cplx* h, cplx* out, int64_t out_stride, int out_col) {
+  qtx_grid_dependency();
   const int nn = n * n;
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     const double fl = occ_l[e], frs = sign_r * occ_r[e];
@@ -751,7 +776,7 @@ void launch_block_dos(int n, int64_t batch, MatView g, double* out, int64_t out_
                       cudaStream_t stream) {
   if (!out) return;
   const unsigned grid = (unsigned)(batch < 65535 ? batch : 65535);
-  block_dos_kernel<<<grid, TB, 0, stream>>>(n, batch, g.ptr, g.ld, g.stride, out, out_stride, out_col);
+  qtx_launch(block_dos_kernel, grid, TB, 0, stream, n, batch, g.ptr, g.ld, g.stride, out, out_stride, out_col);
   qtx_check_launch("block_dos_kernel");
 }
 
@@ -760,7 +785,7 @@ void launch_layer_current(int n, int64_t batch, MatView xl, MatView xr, const do
                           cudaStream_t stream) {
   if (!out) return;
   const unsigned grid = (unsigned)(batch < 65535 ? batch : 65535);
-  layer_current_kernel<<<grid, LC_THREADS, 0, stream>>>(n, batch, xl.ptr, xl.ld, xl.stride, xr.ptr, xr.ld, xr.stride,
-                                                        occ_l, occ_r, sign_r, coupling, out, out_stride, out_col);
+  qtx_launch(layer_current_kernel, grid, LC_THREADS, 0, stream, n, batch, xl.ptr, xl.ld, xl.stride, xr.ptr, xr.ld,
+             xr.stride, occ_l, occ_r, sign_r, coupling, out, out_stride, out_col);
   qtx_check_launch("layer_current_kernel");
 }

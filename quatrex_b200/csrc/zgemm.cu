@@ -162,6 +162,7 @@ __device__ __forceinline__ void mma_step(const cplx* sa, const cplx* sb, int m, 
 
 template <int TILE, int OPA, int OPB>
 __global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_kernel(Params p) {
+  qtx_grid_dependency();
   using C = Cfg<TILE>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
@@ -259,7 +260,7 @@ void launch_t(const Params& p, cudaStream_t stream) {
   // opt-in to the large shared-memory carve-out (per device)
   qtx_opt_in_smem((const void*)zgemm_dmma_kernel<TILE, OPA, OPB>, smem);
   dim3 grid(ceil_div_u(p.n, TILE), ceil_div_u(p.m, TILE), (unsigned)(p.batch < 65535 ? p.batch : 65535));
-  zgemm_dmma_kernel<TILE, OPA, OPB><<<grid, THREADS, smem, stream>>>(p);
+  qtx_launch(zgemm_dmma_kernel<TILE, OPA, OPB>, grid, THREADS, smem, stream, p);
 }
 
 // The tile whose waves finish first.  A full wave of 64x64 tiles covers twice

@@ -104,6 +104,7 @@ template <int S, int NPARTS>
 __global__ void __launch_bounds__(256) ozaki_split_rows_kernel(int R, int K, int64_t batch, const cplx* base, int64_t si,
                                                           int64_t sk, int64_t sb, int conj, int KT, int TR, int* expo,
                                                           signed char* out) {
+  qtx_grid_dependency();
   constexpr int NSEG = NPARTS * S;  // 1 KiB segments per chunk: A 2S, B 4S
   __shared__ __align__(16) uint32_t stage[NSEG * 256];
   __shared__ double wmax[8][8];
@@ -207,6 +208,7 @@ template <int S, int NPARTS>
 __global__ void __launch_bounds__(256) ozaki_split_k_kernel(int R, int K, int64_t batch, const cplx* base, int64_t si,
                                                             int64_t sk, int64_t sb, int conj, int KT, int TR,
                                                             int* expo, signed char* out) {
+  qtx_grid_dependency();
   constexpr int NSEG = NPARTS * S;  // 512-byte segments per chunk (16 rows)
   __shared__ __align__(16) signed char stage[NSEG * 512];
   __shared__ double rscale[SPLIT_KROWS];
@@ -301,10 +303,10 @@ void launch_split(int S, cudaStream_t stream, int R, int K, int64_t batch, const
 #define QTX_SPLIT_CASE(SS)                                                                                      \
   case SS:                                                                                                     \
     if (rows_adjacent)                                                                                         \
-      ozaki_split_rows_kernel<SS, NPARTS><<<grid, 256, 0, stream>>>(R, K, batch, base, si, sk, sb, conj, KT, TR, \
+      qtx_launch(ozaki_split_rows_kernel<SS, NPARTS>, grid, 256, 0, stream, R, K, batch, base, si, sk, sb, conj, KT, TR, \
                                                                     expo, out);                                \
     else                                                                                                       \
-      ozaki_split_k_kernel<SS, NPARTS><<<grid, 256, 0, stream>>>(R, K, batch, base, si, sk, sb, conj, KT, TR,    \
+      qtx_launch(ozaki_split_k_kernel<SS, NPARTS>, grid, 256, 0, stream, R, K, batch, base, si, sk, sb, conj, KT, TR,    \
                                                                  expo, out);                                   \
     break;
   switch (S) {
@@ -440,6 +442,7 @@ struct OzParams {
 // 32w..32w+31), release the tensor memory with tmem_empty and then write the
 // FP64 results while the next tile's MMAs already run.
 __global__ void __launch_bounds__(THREADS, 1) ozaki_gemm_kernel(OzParams p) {
+  qtx_grid_dependency();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const int S = p.S;
   const int abytes = a_block_bytes(S), bbytes = b_block_bytes(S);
@@ -738,7 +741,7 @@ void launch_zgemm_mixed(const GemmCall& g, cudaStream_t stream) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t ntiles = g.batch * (int64_t)Mt * Nt;
   const unsigned grid = (unsigned)std::min<int64_t>(ntiles, sms);
-  ozaki_gemm_kernel<<<grid, THREADS, smem, stream>>>(p);
+  qtx_launch(ozaki_gemm_kernel, grid, THREADS, smem, stream, p);
   qtx_check_launch("ozaki_gemm_kernel");
   cudaFreeAsync(buf, stream);
 }

@@ -502,8 +502,9 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
 
 template <int TPR, int RPT, int CPT, int ROT>
 __global__ void __launch_bounds__(THREADS, 1)
-    zinv_gj_kernel(int n, int64_t batch, const cplx* __restrict__ a_base, int64_t lda, int64_t sa,
+    zinv_gj_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa,
                    cplx* x_base, int64_t ldx, int64_t sx, int* info, const int* active) {
+  qtx_grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const InvShape shp = inv_shape(n);
   const int W = shp.w, WP = shp.wp, CW = shp.cw;
@@ -762,9 +763,10 @@ struct SplitScratch {
 
 template <int TPR, int RPT, int CPT, int ROT>
 __global__ void __launch_bounds__(THREADS, 1)
-    zinv_split_panel_kernel(int n, int64_t batch, const cplx* __restrict__ a_base, int64_t lda, int64_t sa,
+    zinv_split_panel_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa,
                             cplx* x_base, int64_t ldx, int64_t sx, int k0, SplitScratch sc, int* info,
                             const int* active) {
+  qtx_grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const InvShape shp = inv_shape(n);
   const int W = shp.w, WP = shp.wp;
@@ -811,6 +813,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 __global__ void __launch_bounds__(256)
     zinv_split_rows_kernel(int n, int64_t batch, const cplx* x_base, int64_t ldx, int64_t sx, int k0, int W,
                            SplitScratch sc, const int* active) {
+  qtx_grid_dependency();
   const int j = blockIdx.x;
   for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
     if (active && !active[e]) continue;
@@ -838,6 +841,7 @@ inline size_t split_update_smem(int W) {
 __global__ void __launch_bounds__(SPLIT_THREADS, 2)
     zinv_split_update_kernel(int n, int64_t batch, cplx* x_base, int64_t ldx, int64_t sx, int k0, int w, int W,
                              SplitScratch sc, const int* active) {
+  qtx_grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* Prow = reinterpret_cast<cplx*>(smem_raw);  // P rows of the CTA's outputs, swizzled, 32 columns
   cplx* R = Prow + SPLIT_ROWS * 32;                 // w x SPLIT_LDR
@@ -997,6 +1001,7 @@ inline size_t split_unscramble_smem(int n) {
 __global__ void __launch_bounds__(THREADS)
     zinv_split_unscramble_kernel(int n, int64_t batch, cplx* x_base, int64_t ldx, int64_t sx, SplitScratch sc,
                                  const int* active) {
+  qtx_grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const size_t iw = (n * sizeof(int) + 15) & ~size_t(15);
   int* colsrc = reinterpret_cast<int*>(smem_raw);
@@ -1059,8 +1064,8 @@ void launch_inv_r(int n, int64_t batch, MatView a, MutView x, int* info, const i
                   cudaStream_t stream) {
   qtx_opt_in_smem((const void*)zinv_gj_kernel<TPR, RPT, CPT, ROT>, smem);
   int grid = (int)(batch < 65535 ? batch : 65535);
-  zinv_gj_kernel<TPR, RPT, CPT, ROT><<<grid, THREADS, smem, stream>>>(n, batch, a.ptr, a.ld, a.stride, x.ptr,
-                                                                       x.ld, x.stride, info, active);
+  qtx_launch(zinv_gj_kernel<TPR, RPT, CPT, ROT>, grid, THREADS, smem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr,
+             x.ld, x.stride, info, active);
 }
 
 template <int TPR, int RPT, int CPT>
@@ -1101,16 +1106,15 @@ void launch_split_r(int n, int64_t batch, MatView a, MutView x, int* info, const
   const int nslab = (n + SPLIT_CW - 1) / SPLIT_CW, ngroups = (n + SPLIT_ROWS - 1) / SPLIT_ROWS;
   for (int k0 = 0; k0 < n; k0 += W) {
     const int w = std::min(W, n - k0);
-    zinv_split_panel_kernel<TPR, RPT, CPT, ROT><<<gb, THREADS, psmem, stream>>>(n, batch, a.ptr, a.ld, a.stride,
-                                                                               x.ptr, x.ld, x.stride, k0, sc, info,
-                                                                               active);
-    zinv_split_rows_kernel<<<dim3(w, gb), 256, 0, stream>>>(n, batch, x.ptr, x.ld, x.stride, k0, W, sc, active);
-    zinv_split_update_kernel<<<dim3(nslab * ngroups, gb), SPLIT_THREADS, usmem, stream>>>(n, batch, x.ptr, x.ld,
-                                                                                         x.stride, k0, w, W, sc,
-                                                                                         active);
+    qtx_launch(zinv_split_panel_kernel<TPR, RPT, CPT, ROT>, gb, THREADS, psmem, stream, n, batch, a.ptr, a.ld,
+               a.stride, x.ptr, x.ld, x.stride, k0, sc, info, active);
+    qtx_launch(zinv_split_rows_kernel, dim3(w, gb), 256, 0, stream, n, batch, x.ptr, x.ld, x.stride, k0, W, sc,
+               active);
+    qtx_launch(zinv_split_update_kernel, dim3(nslab * ngroups, gb), SPLIT_THREADS, usmem, stream, n, batch, x.ptr,
+               x.ld, x.stride, k0, w, W, sc, active);
   }
-  zinv_split_unscramble_kernel<<<dim3((n + UNS_ROWS - 1) / UNS_ROWS, gb), THREADS, xsmem, stream>>>(
-      n, batch, x.ptr, x.ld, x.stride, sc, active);
+  qtx_launch(zinv_split_unscramble_kernel, dim3((n + UNS_ROWS - 1) / UNS_ROWS, gb), THREADS, xsmem, stream, n, batch,
+             x.ptr, x.ld, x.stride, sc, active);
   cudaFreeAsync(buf, stream);
 }
 
