@@ -20,12 +20,12 @@
 //     products on DMMA (mma.sync m16n8k4 f64) from a 4-stage cp.async ring of
 //     8-wide K slices; per output element the K order and the DMMA sequence
 //     are those of zgemm_dmma_kernel.
-//   * cta_inverse: Gauss-Jordan with implicit partial pivoting (LAPACK izamax
-//     rule: first row of maximal |Re| + |Im|), the matrix in registers with
-//     THREADS / BT threads per row, one barrier per column, the row and
-//     column permutations applied on the store.
+//   * cta_inverse: Gauss-Jordan with implicit partial pivoting (gj_regs.cuh),
+//     the matrix in registers with THREADS / BT threads per row, one barrier
+//     per column, the row and column permutations applied on the store.
 // There are no inter-CTA waits: the only shared state is the work counter
 // and the error flags.
+#include "gj_regs.cuh"
 #include "kernels.h"
 
 namespace {
@@ -46,16 +46,13 @@ struct GCfg {
   static constexpr int WM = BT / 2, WN = BT / WARPS_N, MI = WM / 16, NI = WN / 8;
   static constexpr int GEMM_ELEMS = ST * 2 * TILE;
   static constexpr int TPR = THREADS / BT, CPT = BT / TPR;  // inverse: threads per row, columns per thread
-  static constexpr int CAND_ELEMS = 2 * NWARPS * BT;
-  static constexpr int REGION = GEMM_ELEMS > CAND_ELEMS ? GEMM_ELEMS : CAND_ELEMS;
+  static constexpr int GJ_ELEMS = (int)(sizeof(GjRegs<TPR, CPT, NWARPS>) / sizeof(cplx)) + 1;
+  static constexpr int REGION = GEMM_ELEMS > GJ_ELEMS ? GEMM_ELEMS : GJ_ELEMS;
   static constexpr int MIN_BLOCKS = BT <= 32 ? 4 : 2;
 };
 
 template <int BT>
 struct Misc {
-  double red_v[2][GCfg<BT>::NWARPS];
-  int red_i[2][GCfg<BT>::NWARPS];
-  cplx red_piv[2][GCfg<BT>::NWARPS];  // column-k entry of each warp's candidate
   int pivs[BT];  // pivot row of each step
   int pos[BT];   // step at which each row was the pivot
   double sum[2 * GCfg<BT>::NWARPS];
@@ -247,128 +244,38 @@ __device__ __noinline__ void cta_gemm(const GArgs g, int n) {
   }
 }
 
-__device__ __forceinline__ void argmax_combine(double& v, int& i, double v2, int i2) {
-  if (v2 > v || (v2 == v && i2 < i)) {
-    v = v2;
-    i = i2;
-  }
-}
-
 // X = A^-1 (n x n, n <= BT; X must not alias A).  Returns 0, or 1 + the first
 // column whose pivot is exactly zero (the result then holds inf/NaN).
 //
-// Rows stay where they are (implicit pivoting): step k picks pivot row p_k
-// among the rows not used yet and stores the elimination in place.  The
-// row-swapping form would hold row p_k at position k, so with pos(r) the step
-// at which row r was the pivot, X[pos(r)][p_c] = M[r][c]: every thread writes
-// its own elements once, through the pivot list and its inverse.
-//
-// The in-place step is x_rc <- x_rc - (x_rk / piv) p_c for c != k and
-// -x_rk / piv at c = k.  The staged pivot row carries 1 at column k and every
-// row clears its own column-k entry when it reads it, so one branch-free
-// x - fd p covers both (the pivot row's own entries p_c / piv likewise); the
-// pivot value itself travels through shared memory.
+// The matrix in registers, TPR threads per row, eliminated by gj_eliminate (the
+// steps of zinv_regs_kernel).  Rows stay where they are; the row-swapping form
+// would hold row p_k at position k, so with pos(r) the step at which row r was
+// the pivot, X[pos(r)][p_c] = M[r][c]: every thread writes its own elements
+// once, through the pivot list and its inverse.
 template <int BT>
 __device__ __noinline__ int cta_inverse(const cplx* A, cplx* X, int n) {
   using C = GCfg<BT>;
-  cplx* cand = smem_region<BT>();
-  Misc<BT>* ms = smem_misc<BT>();
   constexpr int TPR = C::TPR, CPT = C::CPT;
-  constexpr int ROWS_PER_WARP = 32 / TPR;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto& sm = *reinterpret_cast<GjRegs<TPR, CPT, C::NWARPS>*>(smem_region<BT>());
+  Misc<BT>* ms = smem_misc<BT>();
+  const int tid = threadIdx.x;
   const int r_own = tid / TPR, c_own = tid % TPR;
-  const int grp0 = lane - c_own;  // first lane of this row's group
   cplx reg[CPT];
 #pragma unroll
   for (int j = 0; j < CPT; ++j) {
     const int c = c_own + j * TPR;
     reg[j] = (r_own < n && c < n) ? A[(int64_t)r_own * n + c] : cmk(0, 0);
   }
-  // staged rows are written at columns < n only: the rest stays zero, so the
-  // padding columns of every register row stay zero too
-  for (int q = tid; q < C::CAND_ELEMS; q += C::THREADS) cand[q] = cmk(0, 0);
-  __syncthreads();
-  bool used = r_own >= n;
-  int zero = 0;
-#pragma unroll 1
-  for (int kk = 0; kk < n; ++kk) {
-    const int kc = kk % TPR;  // lanes c_own == kc hold column kk
-    cplx colv = cmk(0, 0);
-#pragma unroll
-    for (int j = 0; j < CPT; ++j)
-      if (c_own + j * TPR == kk) {
-        colv = reg[j];
-        reg[j] = cmk(0, 0);
-      }
-    double bv = -1.0;
-    int bi = n;
-    if (c_own == kc && !used) {
-      bv = cabs1(colv);
-      bi = r_own;
-    }
-    // the warp's best row among the lanes holding column kk (lanes that share
-    // c_own differ in the bits above log2(TPR)); then lane kc tells the rest
-#pragma unroll
-    for (int off = 16; off >= TPR; off >>= 1) {
-      const double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int i2 = __shfl_xor_sync(0xffffffffu, bi, off);
-      argmax_combine(bv, bi, v2, i2);
-    }
-    bi = __shfl_sync(0xffffffffu, bi, kc);
-    const int src = grp0 + kc;
-    const cplx f = cmk(__shfl_sync(0xffffffffu, colv.x, src), __shfl_sync(0xffffffffu, colv.y, src));
-    const int par = kk & 1;
-    if (bi < n && r_own == bi) {
-      cplx* my_cand = cand + (par * C::NWARPS + warp) * BT;
-#pragma unroll
-      for (int j = 0; j < CPT; ++j) {
-        const int c = c_own + j * TPR;
-        if (c < n) my_cand[c] = reg[j];
-      }
-      if (c_own == kc) {
-        my_cand[kk] = cmk(1, 0);
-        ms->red_piv[par][warp] = colv;
-      }
-    }
-    if (lane == kc) {
-      ms->red_v[par][warp] = bv;
-      ms->red_i[par][warp] = bi;
-    }
-    __syncthreads();  // every warp's candidate row visible
-    // best over the warps: every group of NWARPS lanes holds all candidates
-    double v = ms->red_v[par][lane % C::NWARPS];
-    int p = ms->red_i[par][lane % C::NWARPS];
-#pragma unroll
-    for (int off = C::NWARPS / 2; off > 0; off >>= 1) {
-      const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
-      const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
-      argmax_combine(v, p, v2, i2);
-    }
-    // the global best is also the best of its own warp, whose row is staged
-    const int pw = p / ROWS_PER_WARP;
-    const cplx* prow = cand + (par * C::NWARPS + pw) * BT;
-    const cplx piv = ms->red_piv[par][pw];
-    if (piv.x == 0.0 && piv.y == 0.0 && !zero) zero = kk + 1;
-    const cplx d = crecip_pivot(piv);
-    if (tid == 0) ms->pivs[kk] = p;
-    if (r_own == p) {
-      used = true;
-#pragma unroll
-      for (int j = 0; j < CPT; ++j) reg[j] = cmul(prow[c_own + j * TPR], d);
-    } else {
-      const cplx fd = cmul(f, d);
-#pragma unroll
-      for (int j = 0; j < CPT; ++j) reg[j] = cfms(fd, prow[c_own + j * TPR], reg[j]);
-    }
-  }
+  const int zero = gj_eliminate<TPR, CPT, C::NWARPS>(reg, n, r_own, c_own, r_own >= n, sm, ms->pivs);
   __syncthreads();
   for (int k = tid; k < n; k += C::THREADS) ms->pos[ms->pivs[k]] = k;
   __syncthreads();
   if (r_own < n) {
     const int i = ms->pos[r_own];
+    const int turned = n / TPR;
 #pragma unroll
     for (int j = 0; j < CPT; ++j) {
-      const int c = c_own + j * TPR;
+      const int c = ((j + turned) % CPT) * TPR + c_own;
       if (c < n) X[(int64_t)i * n + ms->pivs[c]] = reg[j];
     }
   }

@@ -1,19 +1,22 @@
-// Batched complex FP64 inverse: blocked in-place Gauss-Jordan elimination with
-// partial (row) pivoting, one CTA per matrix, bulk work on the FP64 tensor path.
+// Batched complex FP64 inverse: in-place Gauss-Jordan elimination with partial
+// pivoting.  Replaces qttools.kernels.linalg.inv
+// (src/qttools/kernels/linalg/inv.py:6-40, LAPACK getrf/getri, or getrf/getrs on
+// the GPU).  Pivot choice follows the LAPACK izamax rule: the first row (in the
+// current row order) of maximal |Re| + |Im|.
 //
-// Replaces qttools.kernels.linalg.inv (src/qttools/kernels/linalg/inv.py:6-40,
-// LAPACK getrf/getri, or getrf/getrs on the GPU).  Pivot choice follows the
-// LAPACK izamax rule: the first row (in the current row order) of maximal
-// |Re| + |Im|.
+// Three forms, chosen in launch_zinv:
+//   n <= 64            zinv_regs_kernel: the whole matrix in the registers of one
+//                      CTA
+//   n <= 512           zinv_panel_kernel + zinv_update_kernel per panel of
+//                      columns, zinv_split_unscramble_kernel at the end
+//   no scratch memory  zinv_gj_kernel: one launch, one CTA per matrix
 //
-// Algorithm for an n x n matrix X (a copy of A), panel width w:
+// Algorithm of the blocked forms for an n x n matrix X (a copy of A), panel
+// width w:
 //   for each panel of columns [k0, k0 + w):
-//     1. stage the n x w panel (rows in the current order of X) into the
-//        threads' registers through shared memory and eliminate it column by
-//        column without moving rows: pick the pivot row among the rows not
-//        yet used, eliminate the column from all other rows, scale the pivot
-//        row (one barrier per column: every warp publishes its candidate row
-//        before it);
+//     1. eliminate the n x w panel in registers column by column without moving
+//        rows: pick the pivot row among the rows not yet used, eliminate the
+//        column from all other rows, scale the pivot row;
 //     2. turn the pivot sequence into the row permutation sigma that the
 //        classic row-swapping Gauss-Jordan would apply (position k0 + j takes
 //        pivot row p_j, the displaced row goes to p_j's position), and record
@@ -22,17 +25,15 @@
 //        rank-w update on DMMA (mma.sync m16n8k4 f64) tiles:
 //          X[i, c] <- [i not in panel] X[sigma(i), c]
 //                     + sum_j P[sigma(i), j] X[p_j, c]
-//        in column slabs of CW, the k0 + j pivot rows staged in shared memory
-//        (for small batches the updates of one panel run as a separate launch
-//        spread over the GPU, the split path below);
+//        in column slabs, the pivot rows staged in shared memory;
 //   finally undo the row interchanges as column interchanges in reverse order.
-// The matrix itself stays in global memory (L2 resident for a wave of
-// matrices); shared memory holds the panel (n x Wp, XOR-swizzled so that both
-// row-per-thread access and DMMA fragment loads are conflict-free), two slabs
-// of pivot rows and the permutation arrays.
+// The matrix itself stays in global memory; shared memory holds the panel
+// (n x Wp, XOR-swizzled so that both row-per-thread access and DMMA fragment
+// loads are conflict-free), slabs of pivot rows and the permutation arrays.
 #include <algorithm>
 #include <cstdlib>
 
+#include "gj_regs.cuh"
 #include "kernels.h"
 
 namespace {
@@ -160,7 +161,7 @@ __device__ inline GjSmem gj_smem_layout(unsigned char* base, int n, int wp, int 
 // permutation sigma (pos2row / row2pos, relative to the current order) and
 // the swaps perm[k0 .. k0 + w), and leave the eliminated panel in P (rows in
 // the current order).  Ends with a CTA barrier.
-template <int TPR, int RPT, int CPT, int ROT>
+template <int TPR, int RPT, int CPT>
 __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cplx* X, int64_t ldx, const GjSmem& sm,
                                          int& zero_pivot) {
   cplx* P = sm.P;
@@ -205,110 +206,30 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
       }
     const int grp0 = lane - c_own;  // first lane of this row's group (groups never straddle warps)
     // rows before k0 are the pivots of earlier panels (rows are in the new order now)
-    bool rotated = false;
     if constexpr (TPR == 1 && RPT == 1 && CPT == 32) {
-      if constexpr (ROT == 1) {
-        // Register rotation: at step kk, reg[0][j] holds panel column
-        // (kk + j) mod 32, so the step's column is always reg[0][0] (no
-        // selects over the row) and every update is unpredicated (columns
-        // at or beyond w stay zero: the published pivot rows carry zeros
-        // there).  The same pivots and the same update of every non-pivot
-        // row as the generic loop.
-        rotated = true;
-        bool used = r_own < k0;
-        auto rotate = [&]() {
-          const cplx t0 = reg[0][0];
+      // Register rotation: at step kk, reg[0][j] holds panel column
+      // (kk + j) mod 32, so the step's column is always reg[0][0] (no
+      // selects over the row) and every update is unpredicated (columns
+      // at or beyond w stay zero: the published pivot rows carry zeros
+      // there).  The same pivots and the same update of every non-pivot
+      // row as the generic loop.
+      bool used = r_own < k0;
+      auto rotate = [&]() {
+        const cplx t0 = reg[0][0];
 #pragma unroll
-          for (int j = 0; j < 31; ++j) reg[0][j] = reg[0][j + 1];
-          reg[0][31] = t0;
-        };
-#pragma unroll 1
-        for (int kk = 0; kk < w; ++kk) {
-          const int k = k0 + kk;
-          const cplx colv = reg[0][0];
-          reg[0][0] = cmk(0, 0);
-          double bv = -1.0;
-          int bi = n;
-          if (r_own < n && !used) {
-            bv = cabs1(colv);
-            bi = r_own;
-          }
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-            int i2 = __shfl_xor_sync(0xffffffffu, bi, off);
-            argmax_combine(bv, bi, v2, i2);
-          }
-          const int par = kk & 1;
-          cplx* my_cand = cand + (size_t)(par * NWARPS + warp) * WP;
-          const int slot = par * NWARPS;
-          if (r_own == bi) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) my_cand[j] = reg[0][j];
-            my_cand[0] = cmk(1, 0);
-            red_piv[slot + warp] = colv;
-          }
-          if (lane == 0) {
-            red_v[slot + warp] = bv;
-            red_i[slot + warp] = bi;
-          }
-          __syncthreads();  // candidates of every warp visible
-          double v = red_v[slot + lane % NWARPS];
-          int p = red_i[slot + lane % NWARPS];
-#pragma unroll
-          for (int off = NWARPS / 2; off > 0; off >>= 1) {
-            const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
-            const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
-            argmax_combine(v, p, v2, i2);
-          }
-          const int pw = p >> 5;  // one row per thread: row p lives in warp p / 32
-          const cplx* prow = cand + (size_t)(par * NWARPS + pw) * WP;
-          const cplx piv = red_piv[slot + pw];
-          if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k + 1;
-          const cplx d = crecip_pivot(piv);
-          if (tid == 0) pivs[kk] = p;
-          if (r_own < n) {
-            // the pivot row as 0 - (-d) p: one update formula for every
-            // row, so the warp holding the pivot row does not run two
-            // branches while the others wait at the next barrier
-            const bool is_p = r_own == p;
-            used = used || is_p;
-            const cplx fd = is_p ? cmk(-d.x, -d.y) : cmul(colv, d);
-            if (is_p) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) reg[0][j] = cmk(0, 0);
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) reg[0][j] = cfms(fd, prow[j], reg[0][j]);
-          }
-          rotate();
-        }
-        for (int extra = w; extra < 32; ++extra) rotate();  // natural column order again
-      }
-    }
-    if (rotated) {
-    } else if constexpr (CPT == 1) {
-      // One column per lane: lane c_own holds column c_own of the rows
-      // r_own + q * rstride; the factors of column kk come by shuffle from
-      // the lane that holds it, the pivot row is one shared-memory word per
-      // lane.  One barrier per column (each warp publishes its candidate's
-      // row before it).
-      uint32_t used_bits = 0;
-#pragma unroll
-      for (int q = 0; q < RPT; ++q)
-        if (r_own + q * rstride < k0) used_bits |= 1u << q;
+        for (int j = 0; j < 31; ++j) reg[0][j] = reg[0][j + 1];
+        reg[0][31] = t0;
+      };
 #pragma unroll 1
       for (int kk = 0; kk < w; ++kk) {
         const int k = k0 + kk;
-        const int src = grp0 + kk % TPR;
+        const cplx colv = reg[0][0];
+        reg[0][0] = cmk(0, 0);
         double bv = -1.0;
         int bi = n;
-        if (c_own == kk % TPR) {
-#pragma unroll
-          for (int q = 0; q < RPT; ++q) {
-            const int r = r_own + q * rstride;
-            if (r < n && !((used_bits >> q) & 1u)) argmax_combine(bv, bi, cabs1(reg[q][0]), r);
-          }
+        if (r_own < n && !used) {
+          bv = cabs1(colv);
+          bi = r_own;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -318,49 +239,49 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
         }
         const int par = kk & 1;
         cplx* my_cand = cand + (size_t)(par * NWARPS + warp) * WP;
-#pragma unroll
-        for (int q = 0; q < RPT; ++q)
-          if (r_own + q * rstride == bi && c_own < w) my_cand[c_own] = reg[q][0];
         const int slot = par * NWARPS;
+        if (r_own == bi) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) my_cand[j] = reg[0][j];
+          my_cand[0] = cmk(1, 0);
+          red_piv[slot + warp] = colv;
+        }
         if (lane == 0) {
           red_v[slot + warp] = bv;
           red_i[slot + warp] = bi;
         }
         __syncthreads();  // candidates of every warp visible
-        double v = red_v[slot];
-        int p = red_i[slot], pw = 0;
-        for (int q = 1; q < NWARPS; ++q) {
-          const double vq = red_v[slot + q];
-          const int iq = red_i[slot + q];
-          if (vq > v || (vq == v && iq < p)) {
-            v = vq;
-            p = iq;
-            pw = q;
-          }
+        double v = red_v[slot + lane % NWARPS];
+        int p = red_i[slot + lane % NWARPS];
+#pragma unroll
+        for (int off = NWARPS / 2; off > 0; off >>= 1) {
+          const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
+          const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
+          argmax_combine(v, p, v2, i2);
         }
+        const int pw = p >> 5;  // one row per thread: row p lives in warp p / 32
         const cplx* prow = cand + (size_t)(par * NWARPS + pw) * WP;
-        const cplx piv = prow[kk];
+        const cplx piv = red_piv[slot + pw];
         if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k + 1;
         const cplx d = crecip_pivot(piv);
         if (tid == 0) pivs[kk] = p;
-        const cplx pc = c_own < w ? prow[c_own] : cmk(0, 0);
-        const cplx pd = cmul(pc, d);
+        if (r_own < n) {
+          // the pivot row as 0 - (-d) p: one update formula for every
+          // row, so the warp holding the pivot row does not run two
+          // branches while the others wait at the next barrier
+          const bool is_p = r_own == p;
+          used = used || is_p;
+          const cplx fd = is_p ? cmk(-d.x, -d.y) : cmul(colv, d);
+          if (is_p) {
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          // every lane takes part in the shuffle, whatever its row
-          const double fx = __shfl_sync(0xffffffffu, reg[q][0].x, src);
-          const double fy = __shfl_sync(0xffffffffu, reg[q][0].y, src);
-          const int r = r_own + q * rstride;
-          if (r >= n || c_own >= w) continue;
-          if (r == p) {
-            used_bits |= 1u << q;
-            reg[q][0] = (c_own == kk) ? d : pd;
-          } else {
-            const cplx fd = cmul(cmk(fx, fy), d);
-            reg[q][0] = (c_own == kk) ? cmk(-fd.x, -fd.y) : cfms(fd, pc, reg[q][0]);
+            for (int j = 0; j < 32; ++j) reg[0][j] = cmk(0, 0);
           }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) reg[0][j] = cfms(fd, prow[j], reg[0][j]);
         }
+        rotate();
       }
+      for (int extra = w; extra < 32; ++extra) rotate();  // natural column order again
     } else {
       bool used[RPT];
 #pragma unroll
@@ -500,7 +421,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
     __syncthreads();
 }
 
-template <int TPR, int RPT, int CPT, int ROT>
+template <int TPR, int RPT, int CPT>
 __global__ void __launch_bounds__(THREADS, 1)
     zinv_gj_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa,
                    cplx* x_base, int64_t ldx, int64_t sx, int* info, const int* active) {
@@ -534,7 +455,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     for (int k0 = 0; k0 < n; k0 += W) {
       const int w = min(W, n - k0);
-      gj_panel<TPR, RPT, CPT, ROT>(n, k0, w, WP, X, ldx, sm, zero_pivot);
+      gj_panel<TPR, RPT, CPT>(n, k0, w, WP, X, ldx, sm, zero_pivot);
 
       // ---- 3. rank-w update of the other columns, slabs of CW columns.
       // Output position i reads X[sigma(i)], and sigma(i) is either i itself or
@@ -741,250 +662,320 @@ __global__ void __launch_bounds__(THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Split path for batches smaller than the GPU: the elimination and update of
-// zinv_gj_kernel, but every panel is two launches -- one CTA per matrix
-// eliminates the panel, then (matrix x 32-column slab x 128-row group) CTAs
-// apply its rank-w update -- so the updates of a few matrices spread over the
-// whole GPU (the column chain of the elimination stays one CTA per matrix).
-// Per matrix the panel launch leaves in global scratch the eliminated panel
-// P (n x W, rows in the order before the panel's permutation), sigma
-// (pos2row) and the column swaps; a row-copy launch adds the pivot rows
-// R = X[sigma(k0 + j)] and the panel-position rows D = X[k0 + j] (n columns
-// each); the update CTAs read R and D from the scratch, so no CTA reads a row
-// of X that another CTA of the same launch writes.
+// Blocks of up to 64: the whole matrix in registers (gj_regs.cuh), one CTA per
+// matrix, four threads per row (four warps up to 32 rows, eight up to 64).  The row and column permutations are applied on the store:
+// the row-swapping elimination would hold row p_k at position k, so with pos(r)
+// the step at which row r was the pivot, X[pos(r)][p_c] = M[r][c].
+// Bound by the chain of n dependent steps: about 1100 cycles each at 32 rows,
+// 1700 at 64.  Measured on B200, us per call with its status read: b = 32, 8
+// matrices 44 (66 with the blocked kernel), b = 64, 32 matrices 89 (147).
+template <int TPR, int CPT, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
+    zinv_regs_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa, cplx* x_base, int64_t ldx,
+                     int64_t sx, int* info, const int* active) {
+  qtx_grid_dependency();
+  __shared__ GjRegs<TPR, CPT, NW> sm;
+  __shared__ int pivs[TPR * CPT], pos[TPR * CPT];
+  const int r = threadIdx.x / TPR, cl = threadIdx.x % TPR;
+  for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
+    if (active && !active[e]) continue;
+    const cplx* A = a_base + e * sa;
+    cplx* X = x_base + e * sx;
+    cplx x[CPT];
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
+      const int c = cl + j * TPR;
+      x[j] = r < n && c < n ? A[(int64_t)r * lda + c] : cmk(0, 0);
+    }
+    const int zero = gj_eliminate<TPR, CPT, NW>(x, n, r, cl, r >= n, sm, pivs);
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += 32 * NW) pos[pivs[k]] = k;
+    __syncthreads();
+    if (r < n) {
+      cplx* row = X + (int64_t)pos[r] * ldx;
+      const int turned = n / TPR;
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) {
+        const int c = ((j + turned) % CPT) * TPR + cl;
+        if (c < n) row[pivs[c]] = x[j];
+      }
+    }
+    // sticky: callers zero info once and read it after several launches
+    if (info && threadIdx.x == 0 && zero) info[e] = zero;
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Larger blocks: every panel of 32 columns (16 above 256 rows) is two
+// launches.  zinv_panel_kernel, one CTA per matrix and a row per thread,
+// eliminates the panel in registers (gj_regs.cuh) and leaves in global scratch
+// the eliminated panel P (n x W, rows in the order before the panel's
+// permutation), sigma (pos2row) and the column swaps; zinv_update_kernel
+// applies its rank-w update to the other columns, a CTA per (matrix, 32-column
+// slab) with all n rows, so a CTA stages the pivot rows R = X[sigma(k0 + j)]
+// and the panel-position rows D = X[k0 + j] of its slab itself before it
+// writes any of them.  The column chain of the elimination runs on as many SMs
+// as there are matrices, the updates on all.
+//
+// Bounds: the panel by its chain of dependent steps (about 2000 cycles each at
+// 256 rows), the update by HBM (32 n^2 bytes per matrix and panel) once the
+// batch is larger than L2, by the DMMA rate before.  Measured on B200, ms per
+// call, against three launches per panel (the pivot rows copied by one of their
+// own) below 80-124 matrices and zinv_gj_kernel from there on:
+//     b = 100,  24 matrices 0.18 (0.28)     b = 128, 100 matrices 0.27 (0.41)
+//     b = 256,  16 matrices 0.54 (0.82)     b = 256,  64 matrices 0.84 (1.26)
+//     b = 256, 148 matrices 1.31 (1.65)     b = 300,  20 matrices 0.84 (1.43)
+//     b = 512,  24 matrices 2.62 (4.26)     b = 512, 148 matrices 9.4 (13.0)
 
 struct SplitScratch {
-  cplx* p;      // batch x n x W
-  cplx* r;      // batch x W x n
-  cplx* d;      // batch x W x n
-  int* sigma;   // batch x n
-  int* perm;    // batch x n
+  cplx* p;     // batch x n x W
+  int* sigma;  // batch x n
+  int* perm;   // batch x n
 };
 
-template <int TPR, int RPT, int CPT, int ROT>
-__global__ void __launch_bounds__(THREADS, 1)
-    zinv_split_panel_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa,
-                            cplx* x_base, int64_t ldx, int64_t sx, int k0, SplitScratch sc, int* info,
-                            const int* active) {
+inline int panel_width(int n) { return n <= 256 ? 32 : 16; }
+
+inline size_t panel_smem(int n, int W) {
+  return (size_t)n * W * sizeof(cplx) + (size_t)(2 * n + 2 * W) * sizeof(int);
+}
+
+// The panel [k0, k0 + w) of every matrix; W = TPR * CPT columns, TPR threads a
+// row, 32 NW / TPR >= n rows.
+template <int TPR, int CPT, int NW>
+__global__ void __launch_bounds__(32 * NW)
+    zinv_panel_kernel(int n, int64_t batch, const cplx* a_base, int64_t lda, int64_t sa, cplx* x_base, int64_t ldx,
+                      int64_t sx, int k0, SplitScratch sc, int* info, const int* active) {
   qtx_grid_dependency();
+  constexpr int W = TPR * CPT, NT = 32 * NW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const InvShape shp = inv_shape(n);
-  const int W = shp.w, WP = shp.wp;
-  const GjSmem sm = gj_smem_layout(smem_raw, n, WP, 0);
-  const int tid = threadIdx.x;
+  __shared__ GjRegs<TPR, CPT, NW> sm;
+  cplx* P = reinterpret_cast<cplx*>(smem_raw);  // n x W, swizzled
+  int* pos2row = reinterpret_cast<int*>(P + (size_t)n * W);
+  int* row2pos = pos2row + n;
+  int* pivs = row2pos + n;
+  int* swaps = pivs + W;
+  const int tid = threadIdx.x, row = tid / TPR, cl = tid % TPR;
   const int w = min(W, n - k0);
   for (int64_t e = blockIdx.x; e < batch; e += gridDim.x) {
     if (active && !active[e]) continue;
     cplx* X = x_base + e * sx;
+    const cplx* src = X + k0;
+    int64_t lds = ldx;
     if (k0 == 0) {
-      const cplx* A = a_base + e * sa;
-      if (A != X || lda != ldx) {
-        for (int idx = tid; idx < n * n; idx += THREADS) {
-          int r = idx / n, c = idx % n;
-          X[(int64_t)r * ldx + c] = A[(int64_t)r * lda + c];
-        }
-      }
-      __syncthreads();
+      src = a_base + e * sa;
+      lds = lda;
     }
-    int zero_pivot = 0;
-    gj_panel<TPR, RPT, CPT, ROT>(n, k0, w, WP, X, ldx, sm, zero_pivot);
-    cplx* pe = sc.p + e * (int64_t)n * W;
-    for (int idx = tid; idx < n * w; idx += THREADS) {
+    // the panel through shared memory: coalesced copies, then a row per thread
+    for (int idx = tid; idx < n * w; idx += NT) {
       const int r = idx / w, c = idx % w;
-      pe[(int64_t)r * W + c] = sm.P[pidx(r, c, WP)];
-    }
-    for (int r = tid; r < n; r += THREADS) sc.sigma[e * n + r] = sm.pos2row[r];
-    for (int kk = tid; kk < w; kk += THREADS) sc.perm[e * n + k0 + kk] = sm.perm[k0 + kk];
-    __syncthreads();  // sigma and the panel copied before the panel columns change
-    for (int idx = tid; idx < n * w; idx += THREADS) {
-      const int i = idx / w, c = idx % w;
-      X[(int64_t)i * ldx + k0 + c] = sm.P[pidx(sm.pos2row[i], c, WP)];
-    }
-    // the first exact zero pivot of the matrix (earlier panels win)
-    if (info && tid == 0 && zero_pivot && info[e] == 0) info[e] = zero_pivot;
-    __syncthreads();
-  }
-}
-
-// The pivot rows R = X[sigma(k0 + j)] and the panel-position rows
-// D = X[k0 + j] of every matrix, copied before the update moves them (one
-// CTA per row and matrix; the panel columns of X may already hold their final
-// values, the update does not read them from these copies).
-__global__ void __launch_bounds__(256)
-    zinv_split_rows_kernel(int n, int64_t batch, const cplx* x_base, int64_t ldx, int64_t sx, int k0, int W,
-                           SplitScratch sc, const int* active) {
-  qtx_grid_dependency();
-  const int j = blockIdx.x;
-  for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
-    if (active && !active[e]) continue;
-    const cplx* X = x_base + e * sx;
-    const int src = sc.sigma[e * n + k0 + j];
-    cplx* re = sc.r + (e * (int64_t)W + j) * n;
-    cplx* de = sc.d + (e * (int64_t)W + j) * n;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) {
-      re[c] = X[(int64_t)src * ldx + c];
-      de[c] = X[(int64_t)(k0 + j) * ldx + c];
-    }
-  }
-}
-
-constexpr int SPLIT_ROWS = 128;     // output rows per update CTA
-constexpr int SPLIT_THREADS = 128;  // four warps, one 32 x 32 tile each
-constexpr int SPLIT_CW = 32;        // columns per update CTA
-constexpr int SPLIT_LDR = SPLIT_CW + 2;
-
-inline size_t split_update_smem(int W) {
-  return (size_t)SPLIT_ROWS * 32 * sizeof(cplx) + (size_t)2 * W * SPLIT_LDR * sizeof(cplx) +
-         (size_t)SPLIT_ROWS * sizeof(int) + 64;
-}
-
-__global__ void __launch_bounds__(SPLIT_THREADS, 2)
-    zinv_split_update_kernel(int n, int64_t batch, cplx* x_base, int64_t ldx, int64_t sx, int k0, int w, int W,
-                             SplitScratch sc, const int* active) {
-  qtx_grid_dependency();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* Prow = reinterpret_cast<cplx*>(smem_raw);  // P rows of the CTA's outputs, swizzled, 32 columns
-  cplx* R = Prow + SPLIT_ROWS * 32;                 // w x SPLIT_LDR
-  cplx* D = R + W * SPLIT_LDR;                      // w x SPLIT_LDR
-  int* srow = reinterpret_cast<int*>(D + W * SPLIT_LDR);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int ngroups = (n + SPLIT_ROWS - 1) / SPLIT_ROWS;
-  const int slab = blockIdx.x / ngroups, grp = blockIdx.x % ngroups;
-  const int c0 = slab * SPLIT_CW, r0 = grp * SPLIT_ROWS;
-  // a slab inside the panel has nothing to update
-  if (c0 >= k0 && min(c0 + SPLIT_CW, n) <= k0 + w) return;
-  for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
-    if (active && !active[e]) continue;
-    cplx* X = x_base + e * sx;
-    const bool pairs = pair_access_ok(X, ldx, n);
-    const int* sig = sc.sigma + e * n;
-    const cplx* pe = sc.p + e * (int64_t)n * W;
-    const cplx* re = sc.r + e * (int64_t)W * n;
-    const cplx* de = sc.d + e * (int64_t)W * n;
-    for (int li = tid; li < SPLIT_ROWS; li += SPLIT_THREADS) srow[li] = r0 + li < n ? sig[r0 + li] : -1;
-    __syncthreads();
-    for (int idx = tid; idx < SPLIT_ROWS * 32; idx += SPLIT_THREADS) {
-      const int li = idx >> 5, c = idx & 31;
-      const int src = srow[li];
-      const bool ok = src >= 0 && c < w;
-      cp_async16(&Prow[pidx(li, c, 32)], ok ? &pe[(int64_t)src * W + c] : pe, ok);
-    }
-    for (int idx = tid; idx < w * SPLIT_CW; idx += SPLIT_THREADS) {
-      const int j = idx / SPLIT_CW, cc = idx % SPLIT_CW;
-      const bool ok = c0 + cc < n;
-      cp_async16(&R[j * SPLIT_LDR + cc], ok ? &re[(int64_t)j * n + c0 + cc] : re, ok);
-      cp_async16(&D[j * SPLIT_LDR + cc], ok ? &de[(int64_t)j * n + c0 + cc] : de, ok);
+      cp_async16(&P[pidx(r, c, W)], &src[(int64_t)r * lds + c], true);
     }
     cp_async_commit();
-    // one 32 x 32 tile per warp: rows r0 + 32 warp .., columns c0 ..
-    // Output position i starts from row sigma(i): itself, or a row of
-    // [k0, k0 + w) displaced by a pivot swap; positions inside the panel start
-    // from zero.  The rows that start from themselves load while the staged
-    // copies are in flight (only this CTA writes these positions of X); the
-    // displaced rows are patched from the staged D after the barrier.
-    const int lrow0 = warp * 32;
-    const bool has_tile = r0 + lrow0 < n;
-    double acc_re[2][4][4], acc_im[2][4][4];
-    int src_of[2][2];  // sigma(i), or -1 where position i starts from zero
-    if (has_tile) {
-#pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-        for (int hq = 0; hq < 2; ++hq) {
-          const int li = lrow0 + mi * 16 + g + hq * 8;
-          const int i = r0 + li;
-          const bool rv = i < n && !(i >= k0 && i < k0 + w);
-          const int src = rv ? srow[li] : -1;
-          src_of[mi][hq] = src;
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) {
-            const int c = c0 + ni * 8 + 2 * t;  // even
-            cplx y0 = cmk(0, 0), y1 = cmk(0, 0);
-            if (src == i) {
-              const cplx* p = X + (int64_t)i * ldx + c;
-              if (pairs) {
-                if (c < n) ld_pair(p, y0, y1);
-              } else {
-                if (c < n) y0 = p[0];
-                if (c + 1 < n) y1 = p[1];
-              }
-            }
-            acc_re[mi][ni][hq * 2] = y0.x;
-            acc_im[mi][ni][hq * 2] = y0.y;
-            acc_re[mi][ni][hq * 2 + 1] = y1.x;
-            acc_im[mi][ni][hq * 2 + 1] = y1.y;
-          }
-        }
+    for (int r = tid; r < n; r += NT) {
+      pos2row[r] = r;
+      row2pos[r] = r;
     }
     cp_async_wait<0>();
     __syncthreads();
-    if (has_tile) {
+    cplx x[CPT];
 #pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
+    for (int j = 0; j < CPT; ++j) {
+      const int c = cl + j * TPR;
+      x[j] = row < n && c < w ? P[pidx(row, c, W)] : cmk(0, 0);
+    }
+    // rows before k0 are the pivots of earlier panels (rows are in the new order now)
+    const int zero = gj_eliminate<TPR, CPT, NW>(x, w, row, cl, row < k0 || row >= n, sm, pivs);
+    if (row < n) {
+      const int turned = w / TPR;
 #pragma unroll
-        for (int hq = 0; hq < 2; ++hq) {
-          const int i = r0 + lrow0 + mi * 16 + g + hq * 8;
-          const int src = src_of[mi][hq];
-          if (src >= 0 && src != i) {
+      for (int j = 0; j < CPT; ++j) {
+        const int c = ((j + turned) % CPT) * TPR + cl;
+        if (c < w) P[pidx(row, c, W)] = x[j];
+      }
+    }
+    __syncthreads();
+    // row-swap semantics of the panel's pivots: position k0 + kk receives row
+    // pivs[kk], the displaced row goes to the pivot's position
+    if (tid == 0) {
+      for (int kk = 0; kk < w; ++kk) {
+        const int k = k0 + kk, p = pivs[kk];
+        const int qpos = row2pos[p], rk = pos2row[k];
+        pos2row[k] = p;
+        row2pos[p] = k;
+        pos2row[qpos] = rk;
+        row2pos[rk] = qpos;
+        swaps[kk] = qpos;
+      }
+    }
+    cplx* pe = sc.p + e * (int64_t)n * W;
+    for (int idx = tid; idx < n * w; idx += NT) {
+      const int r = idx / w, c = idx % w;
+      pe[(int64_t)r * W + c] = P[pidx(r, c, W)];
+    }
+    __syncthreads();
+    for (int r = tid; r < n; r += NT) sc.sigma[e * n + r] = pos2row[r];
+    for (int kk = tid; kk < w; kk += NT) sc.perm[e * n + k0 + kk] = swaps[kk];
+    // the panel columns of X: final values in the new row order.  (Where X is
+    // still A, k0 = 0 and out of place, the update brings the other columns.)
+    for (int idx = tid; idx < n * w; idx += NT) {
+      const int i = idx / w, c = idx % w;
+      X[(int64_t)i * ldx + k0 + c] = P[pidx(pos2row[i], c, W)];
+    }
+    // the first exact zero pivot of the matrix (earlier panels win)
+    if (info && tid == 0 && zero && info[e] == 0) info[e] = k0 + zero;
+    __syncthreads();
+  }
+}
+
+// Eight warps, 16 rows of the slab each at a time, two CTAs per SM: what
+// bounds a CTA is the latency of its loads (the start values, then the staged
+// rows), so twice the warps of a 32-row tile count for more than its reuse of R.
+constexpr int UPD_THREADS = 256;
+constexpr int UPD_ROWS = UPD_THREADS / 2;  // rows of one pass
+constexpr int UPD_CW = 32;        // columns per CTA
+constexpr int UPD_LDR = UPD_CW + 2;
+
+inline size_t update_smem(int n, int W) {
+  return (size_t)UPD_ROWS * W * sizeof(cplx) + (size_t)2 * W * UPD_LDR * sizeof(cplx) + (size_t)n * sizeof(int);
+}
+
+// Position i of the slab: [i not in panel] S[sigma(i)] + sum_j P[sigma(i), j] R[j],
+// S = X, or A for the first panel of an out-of-place call (S and X are then
+// different matrices and every element of X outside the panel is written here).
+__global__ void __launch_bounds__(UPD_THREADS, 2)
+    zinv_update_kernel(int n, int64_t batch, const cplx* s_base, int64_t lds, int64_t ss, cplx* x_base, int64_t ldx,
+                       int64_t sx, int k0, int w, int W, SplitScratch sc, const int* active) {
+  qtx_grid_dependency();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cplx* P = reinterpret_cast<cplx*>(smem_raw);  // per warp 16 rows P[sigma(i)], swizzled
+  cplx* R = P + UPD_ROWS * W;                   // w x UPD_LDR
+  cplx* D = R + W * UPD_LDR;                    // w x UPD_LDR
+  int* sig = reinterpret_cast<int*>(D + W * UPD_LDR);
+  const int g = lane >> 2, t = lane & 3;
+  cplx* Pw = P + warp * 16 * W;
+  const int c0 = blockIdx.x * UPD_CW;
+  // a slab inside the panel has nothing to update
+  if (c0 >= k0 && min(c0 + UPD_CW, n) <= k0 + w) return;
+  for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
+    if (active && !active[e]) continue;
+    const cplx* S = s_base + e * ss;
+    cplx* X = x_base + e * sx;
+    const bool pairs = pair_access_ok(X, ldx, n) && pair_access_ok(S, lds, n);
+    const cplx* pe = sc.p + e * (int64_t)n * W;
+    for (int i = tid; i < n; i += UPD_THREADS) sig[i] = sc.sigma[e * n + i];
+    __syncthreads();
+    for (int idx = tid; idx < w * UPD_CW; idx += UPD_THREADS) {
+      const int j = idx / UPD_CW, cc = idx % UPD_CW;
+      const bool ok = c0 + cc < n;
+      cp_async16(&R[j * UPD_LDR + cc], ok ? &S[(int64_t)sig[k0 + j] * lds + c0 + cc] : S, ok);
+      cp_async16(&D[j * UPD_LDR + cc], ok ? &S[(int64_t)(k0 + j) * lds + c0 + cc] : S, ok);
+    }
+    bool staged = false;
+    for (int row0 = warp * 16; row0 < n || !staged; row0 += UPD_ROWS) {
+      // the warp's own P rows (no other warp reads them)
+      for (int idx = lane; idx < 16 * W; idx += 32) {
+        const int i = row0 + idx / W, c = idx % W;
+        const bool ok = i < n && c < w;
+        cp_async16(&Pw[pidx(idx / W, c, W)], ok ? &pe[(int64_t)sig[i] * W + c] : pe, ok);
+      }
+      cp_async_commit();
+      // Rows that start from themselves load while the staged copies are in
+      // flight (only this warp writes these positions); rows displaced by a
+      // pivot swap (sigma(i) is then a row of [k0, k0 + w)) are patched from D
+      // after the barrier, positions inside the panel start from zero.
+      double acc_re[4][4], acc_im[4][4];
+      int src_of[2];  // sigma(i), -1 past the matrix
+      bool in_panel[2];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-              for (int ql = 0; ql < 2; ++ql) {
-                const int cc = ni * 8 + 2 * t + ql;
-                if (c0 + cc < n) {
-                  const cplx y = D[(src - k0) * SPLIT_LDR + cc];
-                  acc_re[mi][ni][hq * 2 + ql] = y.x;
-                  acc_im[mi][ni][hq * 2 + ql] = y.y;
-                }
-              }
-          }
-        }
-      for (int kk = 0; kk < w; kk += 4) {
-        const int kc = kk + t;
-        cplx af[2][2];
-#pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int li = lrow0 + mi * 16 + g + h * 8;
-            af[mi][h] = (kc < w) ? Prow[pidx(li, kc, 32)] : cmk(0, 0);
-          }
+      for (int hq = 0; hq < 2; ++hq) {
+        const int i = row0 + g + hq * 8;
+        in_panel[hq] = i >= k0 && i < k0 + w;
+        const int src = i < n ? sig[i] : -1;
+        src_of[hq] = src;
+        const bool own = i < n && src == i && !in_panel[hq];
 #pragma unroll
         for (int ni = 0; ni < 4; ++ni) {
-          const cplx bf = (kc < w) ? R[kc * SPLIT_LDR + ni * 8 + g] : cmk(0, 0);
-#pragma unroll
-          for (int mi = 0; mi < 2; ++mi) {
-            dmma(acc_re[mi][ni], af[mi][0].x, af[mi][1].x, bf.x);
-            dmma(acc_im[mi][ni], af[mi][0].x, af[mi][1].x, bf.y);
+          const int c = c0 + ni * 8 + 2 * t;  // even
+          cplx y0 = cmk(0, 0), y1 = cmk(0, 0);
+          if (own) {
+            const cplx* p = S + (int64_t)i * lds + c;
+            if (pairs) {
+              if (c < n) ld_pair(p, y0, y1);
+            } else {
+              if (c < n) y0 = p[0];
+              if (c + 1 < n) y1 = p[1];
+            }
           }
+          acc_re[ni][hq * 2] = y0.x;
+          acc_im[ni][hq * 2] = y0.y;
+          acc_re[ni][hq * 2 + 1] = y1.x;
+          acc_im[ni][hq * 2 + 1] = y1.y;
+        }
+      }
+      cp_async_wait<0>();
+      if (!staged) {
+        __syncthreads();
+        staged = true;
+      } else {
+        __syncwarp();
+      }
+      if (row0 >= n) break;
 #pragma unroll
-          for (int mi = 0; mi < 2; ++mi) {
-            dmma(acc_re[mi][ni], -af[mi][0].y, -af[mi][1].y, bf.y);
-            dmma(acc_im[mi][ni], af[mi][0].y, af[mi][1].y, bf.x);
-          }
+      for (int hq = 0; hq < 2; ++hq) {
+        const int i = row0 + g + hq * 8;
+        const int src = src_of[hq];
+        if (src >= 0 && src != i && !in_panel[hq]) {
+#pragma unroll
+          for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int ql = 0; ql < 2; ++ql) {
+              const int cc = ni * 8 + 2 * t + ql;
+              const cplx y = D[(src - k0) * UPD_LDR + cc];
+              acc_re[ni][hq * 2 + ql] = y.x;
+              acc_im[ni][hq * 2 + ql] = y.y;
+            }
+        }
+      }
+      for (int kk = 0; kk < w; kk += 4) {
+        const int kc = kk + t;
+        cplx af[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) af[h] = kc < w ? Pw[pidx(g + h * 8, kc, W)] : cmk(0, 0);
+        cplx bf[4];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) bf[ni] = kc < w ? R[kc * UPD_LDR + ni * 8 + g] : cmk(0, 0);
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          dmma(acc_re[ni], af[0].x, af[1].x, bf[ni].x);
+          dmma(acc_im[ni], af[0].x, af[1].x, bf[ni].y);
+        }
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          dmma(acc_re[ni], -af[0].y, -af[1].y, bf[ni].y);
+          dmma(acc_im[ni], af[0].y, af[1].y, bf[ni].x);
         }
       }
 #pragma unroll
-      for (int mi = 0; mi < 2; ++mi)
+      for (int hq = 0; hq < 2; ++hq) {
+        const int i = row0 + g + hq * 8;
+        if (i >= n) continue;
 #pragma unroll
-        for (int hq = 0; hq < 2; ++hq) {
-          const int i = r0 + lrow0 + mi * 16 + g + hq * 8;
-          if (i >= n) continue;
-#pragma unroll
-          for (int ni = 0; ni < 4; ++ni) {
-            const int c = c0 + ni * 8 + 2 * t;  // even
-            const cplx v0 = cmk(acc_re[mi][ni][hq * 2], acc_im[mi][ni][hq * 2]);
-            const cplx v1 = cmk(acc_re[mi][ni][hq * 2 + 1], acc_im[mi][ni][hq * 2 + 1]);
-            cplx* p = X + (int64_t)i * ldx + c;
-            if (pairs) {
-              if (c < n && !(c >= k0 && c < k0 + w)) st_pair(p, v0, v1);
-            } else {
-              if (c < n && !(c >= k0 && c < k0 + w)) p[0] = v0;
-              if (c + 1 < n && !(c + 1 >= k0 && c + 1 < k0 + w)) p[1] = v1;
-            }
+        for (int ni = 0; ni < 4; ++ni) {
+          const int c = c0 + ni * 8 + 2 * t;  // even
+          const cplx v0 = cmk(acc_re[ni][hq * 2], acc_im[ni][hq * 2]);
+          const cplx v1 = cmk(acc_re[ni][hq * 2 + 1], acc_im[ni][hq * 2 + 1]);
+          cplx* p = X + (int64_t)i * ldx + c;
+          if (pairs) {
+            if (c < n && !(c >= k0 && c < k0 + w)) st_pair(p, v0, v1);
+          } else {
+            if (c < n && !(c >= k0 && c < k0 + w)) p[0] = v0;
+            if (c + 1 < n && !(c + 1 >= k0 && c + 1 < k0 + w)) p[1] = v1;
           }
         }
+      }
+      __syncwarp();  // every lane is done with the warp's P rows
     }
     __syncthreads();
   }
@@ -1012,18 +1003,17 @@ __global__ void __launch_bounds__(THREADS)
   for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
     if (active && !active[e]) continue;
     cplx* X = x_base + e * sx;
-    for (int c = tid; c < n; c += THREADS) {
-      colsrc[c] = c;
-      perm[c] = sc.perm[e * n + c];
-    }
+    for (int c = tid; c < n; c += THREADS) perm[c] = sc.perm[e * n + c];
     __syncthreads();
-    if (tid == 0) {
-      for (int k = n - 1; k >= 0; --k) {
+    // undoing the swaps from the last to the first leaves column c with what
+    // the swaps, applied to its index from the first to the last, arrive at
+    for (int c = tid; c < n; c += THREADS) {
+      int y = c;
+      for (int k = 0; k < n; ++k) {
         const int q = perm[k];
-        const int tmp = colsrc[k];
-        colsrc[k] = colsrc[q];
-        colsrc[q] = tmp;
+        y = y == k ? q : (y == q ? k : y);
       }
+      colsrc[c] = y;
     }
     for (int idx = tid; idx < nr * n; idx += THREADS) {
       const int r = idx / n, c = idx % n;
@@ -1042,139 +1032,105 @@ __global__ void __launch_bounds__(THREADS)
 
 namespace {
 
-// Column loop of the 32-column panel elimination (b in 129..256),
-// QTX_INV_ROTATE: 1 (the default) the rotated register row with one update
-// formula for every row, 0 the select-based loop of the other shapes.
-// Measured on B200, b = 256, batch 148 / batch 16 (split path): select loop
-// 1.82 / 0.98 ms; rotation alone 1.72 / 0.89 ms (bit for bit the same
-// results as the select loop); rotation with the uniform pivot-row update
-// 1.67 / 0.84 ms (the pivot row then differs by FP64 rounding).  Rotation
-// with each step's updates deferred into the next step's reduction was
-// slower (more spills at 255 registers) and is not built.
-int rotate_panel() {
-  static int v = [] {
-    const char* env = getenv("QTX_INV_ROTATE");
-    return env ? atoi(env) : 1;
+template <int TPR, int RPT, int CPT>
+void launch_inv_r(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, cudaStream_t stream) {
+  const size_t smem = inv_smem_bytes(n);
+  qtx_opt_in_smem((const void*)zinv_gj_kernel<TPR, RPT, CPT>, smem);
+  int grid = (int)(batch < 65535 ? batch : 65535);
+  qtx_launch(zinv_gj_kernel<TPR, RPT, CPT>, grid, THREADS, smem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr,
+             x.ld, x.stride, info, active);
+}
+
+template <int TPR, int CPT, int NW>
+void launch_regs(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, cudaStream_t stream) {
+  const unsigned grid = (unsigned)(batch < (int64_t)1 << 30 ? batch : (int64_t)1 << 30);
+  qtx_launch(zinv_regs_kernel<TPR, CPT, NW>, grid, 32 * NW, 0, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr, x.ld,
+             x.stride, info, active);
+}
+
+// QTX_INV_SPLIT_BELOW sends batches of that many matrices or more of n > 64 to
+// the one-launch kernel (0: all of them), which takes no scratch.  The two-launch
+// panels are the faster form at every batch measured (b = 256: 1.31 against 1.65 ms for 148 matrices, 0.54 against 1.72 for 16), so by default
+// all batches take them.
+int64_t split_below() {
+  static const int64_t v = [] {
+    const char* e = getenv("QTX_INV_SPLIT_BELOW");
+    return e ? (int64_t)atoll(e) : INT64_MAX;
   }();
   return v;
 }
 
-template <int TPR, int RPT, int CPT, int ROT>
-void launch_inv_r(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, size_t smem,
-                  cudaStream_t stream) {
-  qtx_opt_in_smem((const void*)zinv_gj_kernel<TPR, RPT, CPT, ROT>, smem);
-  int grid = (int)(batch < 65535 ? batch : 65535);
-  qtx_launch(zinv_gj_kernel<TPR, RPT, CPT, ROT>, grid, THREADS, smem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr,
-             x.ld, x.stride, info, active);
+size_t split_bytes(int n, int64_t batch) {
+  return sizeof(cplx) * (size_t)batch * n * panel_width(n) + sizeof(int) * (size_t)batch * 2 * n + 256;
 }
 
-template <int TPR, int RPT, int CPT>
-void launch_inv_t(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, size_t smem,
+template <int TPR, int CPT, int NW>
+void launch_split(int n, int64_t batch, MatView a, MutView x, void* scratch, int* info, const int* active,
                   cudaStream_t stream) {
-  if constexpr (TPR == 1 && RPT == 1 && CPT == 32) {
-    const int r = rotate_panel();
-    if (r != 0) return launch_inv_r<TPR, RPT, CPT, 1>(n, batch, a, x, info, active, smem, stream);
-  }
-  launch_inv_r<TPR, RPT, CPT, 0>(n, batch, a, x, info, active, smem, stream);
-}
-
-}  // namespace
-
-namespace {
-
-template <int TPR, int RPT, int CPT, int ROT>
-void launch_split_r(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, cudaStream_t stream) {
-  const InvShape s = inv_shape(n);
-  const int W = s.w;
-  const size_t psmem = inv_smem_bytes(n) - (size_t)slab_elems(n, s) * sizeof(cplx);
-  const size_t usmem = split_update_smem(W);
-  const size_t xsmem = split_unscramble_smem(n);
-  qtx_opt_in_smem((const void*)zinv_split_panel_kernel<TPR, RPT, CPT, ROT>, psmem);
-  qtx_opt_in_smem((const void*)zinv_split_update_kernel, usmem);
+  constexpr int W = TPR * CPT;
+  const unsigned gb = (unsigned)(batch < 65535 ? batch : 65535);
+  const unsigned nslab = (n + UPD_CW - 1) / UPD_CW;
+  const size_t psmem = panel_smem(n, W), usmem = update_smem(n, W), xsmem = split_unscramble_smem(n);
+  qtx_opt_in_smem((const void*)zinv_panel_kernel<TPR, CPT, NW>, psmem);
+  qtx_opt_in_smem((const void*)zinv_update_kernel, usmem);
   qtx_opt_in_smem((const void*)zinv_split_unscramble_kernel, xsmem);
-  const size_t bytes = sizeof(cplx) * (size_t)batch * (3 * (size_t)n * W) + sizeof(int) * (size_t)batch * 2 * n + 256;
-  unsigned char* buf = static_cast<unsigned char*>(qtx_malloc_async(bytes, stream));
-  if (!buf) throw QtxError(QTX_E_NOMEM, "qtx inverse: scratch allocation failed");
   SplitScratch sc;
-  sc.p = reinterpret_cast<cplx*>(buf);
-  sc.r = sc.p + (size_t)batch * n * W;
-  sc.d = sc.r + (size_t)batch * W * n;
-  sc.sigma = reinterpret_cast<int*>(sc.d + (size_t)batch * W * n);
+  sc.p = reinterpret_cast<cplx*>(scratch);
+  sc.sigma = reinterpret_cast<int*>(sc.p + (size_t)batch * n * W);
   sc.perm = sc.sigma + (size_t)batch * n;
 
-  const unsigned gb = (unsigned)(batch < 65535 ? batch : 65535);
-  const int nslab = (n + SPLIT_CW - 1) / SPLIT_CW, ngroups = (n + SPLIT_ROWS - 1) / SPLIT_ROWS;
   for (int k0 = 0; k0 < n; k0 += W) {
     const int w = std::min(W, n - k0);
-    qtx_launch(zinv_split_panel_kernel<TPR, RPT, CPT, ROT>, gb, THREADS, psmem, stream, n, batch, a.ptr, a.ld,
-               a.stride, x.ptr, x.ld, x.stride, k0, sc, info, active);
-    qtx_launch(zinv_split_rows_kernel, dim3(w, gb), 256, 0, stream, n, batch, x.ptr, x.ld, x.stride, k0, W, sc,
-               active);
-    qtx_launch(zinv_split_update_kernel, dim3(nslab * ngroups, gb), SPLIT_THREADS, usmem, stream, n, batch, x.ptr,
-               x.ld, x.stride, k0, w, W, sc, active);
+    qtx_launch(zinv_panel_kernel<TPR, CPT, NW>, gb, 32 * NW, psmem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr, x.ld,
+               x.stride, k0, sc, info, active);
+    // the first update reads A itself, so an out-of-place call needs no copy
+    const MatView from = k0 == 0 ? a : MatView(x);
+    qtx_launch(zinv_update_kernel, dim3(nslab, gb), UPD_THREADS, usmem, stream, n, batch, from.ptr, from.ld,
+               from.stride, x.ptr, x.ld, x.stride, k0, w, W, sc, active);
   }
   qtx_launch(zinv_split_unscramble_kernel, dim3((n + UNS_ROWS - 1) / UNS_ROWS, gb), THREADS, xsmem, stream, n, batch,
              x.ptr, x.ld, x.stride, sc, active);
-  cudaFreeAsync(buf, stream);
-}
-
-template <int TPR, int RPT, int CPT>
-void launch_split_t(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, cudaStream_t stream) {
-  if constexpr (TPR == 1 && RPT == 1 && CPT == 32) {
-    const int r = rotate_panel();
-    if (r != 0) return launch_split_r<TPR, RPT, CPT, 1>(n, batch, a, x, info, active, stream);
-  }
-  launch_split_r<TPR, RPT, CPT, 0>(n, batch, a, x, info, active, stream);
-}
-
-// Batches below split_below(n) matrices take the split path (the fused
-// kernel keeps one matrix per SM, so a small batch leaves most SMs idle
-// during the updates).  Crossovers measured on B200 (kernel_bench inv, fused
-// vs split): b = 128 between 64 and 100 matrices, b = 256 at about 105
-// (1.61 vs 1.57 ms at 100, 1.63 vs 1.74 ms at 120), b = 512 between 100 and
-// 148 (12.7 vs 10.9 ms at 100, 13.0 vs 14.9 ms at 148).  QTX_INV_SPLIT_BELOW
-// sets one threshold for every size (0: never split).
-int64_t split_below(int n) {
-  static const int64_t env = [] {
-    const char* v = getenv("QTX_INV_SPLIT_BELOW");
-    return v ? (int64_t)atoll(v) : (int64_t)-1;
-  }();
-  if (env >= 0) return env;
-  return n <= 128 ? 80 : (n <= 256 ? 110 : 124);
 }
 
 }  // namespace
 
 size_t zinv_workspace_bytes(int n, int64_t batch) {
-  if (n <= 64 || n > 512 || batch >= split_below(n)) return 0;
-  const size_t W = (size_t)inv_shape(n).w;
-  return sizeof(cplx) * (size_t)batch * 3 * (size_t)n * W + sizeof(int) * (size_t)batch * 2 * n + 256;
+  return n <= 64 || n > 512 || batch >= split_below() ? 0 : split_bytes(n, batch);
 }
 
 void launch_zinv(int n, int64_t batch, MatView a, MutView x, int* info, const int* active, cudaStream_t stream,
                  bool may_allocate) {
   if (n <= 0 || batch <= 0) return;
   if (n > 512) throw QtxError(QTX_E_UNSUPPORTED, "qtx inverse: block size above 512");
-  const size_t smem = inv_smem_bytes(n);
+  if (n <= 32) {
+    launch_regs<4, 8, 4>(n, batch, a, x, info, active, stream);
+    qtx_check_launch("zinv_regs_kernel");
+    return;
+  }
+  if (n <= 64) {
+    launch_regs<4, 16, 8>(n, batch, a, x, info, active, stream);
+    qtx_check_launch("zinv_regs_kernel");
+    return;
+  }
+  // without scratch (not allowed, or none left) the one-launch kernel runs
+  void* scratch =
+      may_allocate && batch < split_below() ? qtx_malloc_async(split_bytes(n, batch), stream) : nullptr;
+  if (scratch) {
+    if (n <= 128) launch_split<2, 16, 8>(n, batch, a, x, scratch, info, active, stream);
+    else if (n <= 256) launch_split<1, 32, 8>(n, batch, a, x, scratch, info, active, stream);
+    else if (n <= 384) launch_split<1, 16, 12>(n, batch, a, x, scratch, info, active, stream);
+    else launch_split<1, 16, 16>(n, batch, a, x, scratch, info, active, stream);
+    qtx_check_launch("zinv_panel_kernel");
+    cudaFreeAsync(scratch, stream);
+    return;
+  }
   const InvShape s = inv_shape(n);
   // every panel row / column must be owned by the elimination mapping
   const int rpt = (n + (THREADS / s.tpr) - 1) / (THREADS / s.tpr);
   const int cpt = (s.w + s.tpr - 1) / s.tpr;
-  if (may_allocate && n > 64 && batch < split_below(n)) {
-    if (s.tpr == 1 && rpt == 1 && cpt <= 32) launch_split_t<1, 1, 32>(n, batch, a, x, info, active, stream);
-    else if (s.tpr == 1 && rpt == 2 && cpt <= 16) launch_split_t<1, 2, 16>(n, batch, a, x, info, active, stream);
-    else if (s.tpr == 2 && rpt == 1 && cpt <= 16) launch_split_t<2, 1, 16>(n, batch, a, x, info, active, stream);
-    else throw QtxError(QTX_E_UNSUPPORTED, "qtx inverse: block size outside the supported shapes");
-    qtx_check_launch("zinv_split");
-    return;
-  }
-  // (threads per row, rows per thread) -> instance with enough register columns
-  if (s.tpr == 1 && rpt == 1 && cpt <= 32) launch_inv_t<1, 1, 32>(n, batch, a, x, info, active, smem, stream);
-  else if (s.tpr == 1 && rpt == 2 && cpt <= 16) launch_inv_t<1, 2, 16>(n, batch, a, x, info, active, smem, stream);
-  else if (s.tpr == 2 && rpt == 1 && cpt <= 16) launch_inv_t<2, 1, 16>(n, batch, a, x, info, active, smem, stream);
-  else if (s.tpr == 4 && rpt == 1 && cpt <= 4) launch_inv_t<4, 1, 4>(n, batch, a, x, info, active, smem, stream);
-  else if (s.tpr == 8 && rpt == 1 && cpt <= 4) launch_inv_t<8, 1, 4>(n, batch, a, x, info, active, smem, stream);
-  else if (s.tpr == 16 && rpt == 1 && cpt <= 1) launch_inv_t<16, 1, 1>(n, batch, a, x, info, active, smem, stream);
+  if (s.tpr == 1 && rpt == 1 && cpt <= 32) launch_inv_r<1, 1, 32>(n, batch, a, x, info, active, stream);
+  else if (s.tpr == 1 && rpt == 2 && cpt <= 16) launch_inv_r<1, 2, 16>(n, batch, a, x, info, active, stream);
+  else if (s.tpr == 2 && rpt == 1 && cpt <= 16) launch_inv_r<2, 1, 16>(n, batch, a, x, info, active, stream);
   else throw QtxError(QTX_E_UNSUPPORTED, "qtx inverse: block size outside the supported shapes");
   qtx_check_launch("zinv_gj_kernel");
 }

@@ -108,6 +108,49 @@ def test_inverse_matches_lapack(n):
     _lib.check(st, ctx, "inv")
     assert _rel(ta, ref) < 1e-10
 
+@pytest.mark.parametrize("n,batch", [(32, 3), (33, 3), (63, 2), (65, 3), (160, 2), (192, 160), (256, 20), (384, 2),
+                                     (385, 2), (511, 2)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_inverse_register_and_panel_shapes(n, batch, in_place):
+    """Edges of the register kernels (32 and 64 rows) and of the panel kernels
+    (128, 256 and 384 rows; 32- and 16-column panels with a remainder), with
+    few and with many matrices per launch (the update's two CTA shapes)."""
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
+    a[:, np.arange(n), np.arange(n)] += np.sqrt(n)
+    ta = torch.from_numpy(a[:, np.roll(np.arange(n), n // 3)].copy()).cuda()
+    want = torch.linalg.inv(ta)
+    x = ta.clone() if in_place else torch.empty_like(ta)
+    lib = _lib.load()
+    ctx = _lib.context(0)
+    src = x if in_place else ta
+    _lib.check(lib.qtx_inv(ctx, n, batch, src.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
+    torch.cuda.synchronize()
+    # elimination with partial pivoting: error of order n u times the condition number
+    cond = float(torch.linalg.cond(ta).max())
+    assert _rel(x, want.cpu().numpy()) < 4 * n * 2.0**-53 * cond
+
+
+@pytest.mark.parametrize("n", [16, 32, 64, 128])
+def test_inverse_of_tied_pivots(n):
+    """Hadamard matrices: in the first steps every candidate of a column has
+    the same |Re| + |Im| (ties over all the bits the search compares), and
+    rows scaled by 1 + k 2^-50 tie in the high word only; H^-1 = H^T / n."""
+    h = np.ones((1, 1))
+    while h.shape[0] < n:
+        h = np.block([[h, h], [h, -h]])
+    scale = 1.0 + np.arange(n) * 2.0**-50
+    a = np.stack([h, scale[:, None] * h]).astype(np.complex128)
+    ta = torch.from_numpy(a).cuda()
+    x = torch.empty_like(ta)
+    lib = _lib.load()
+    ctx = _lib.context(0)
+    _lib.check(lib.qtx_inv(ctx, n, 2, ta.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
+    torch.cuda.synchronize()
+    want = np.stack([h.T / n, h.T / (n * scale[None, :])])
+    # orthogonal up to scale (condition number 1), growth factor n
+    assert _rel(x, want) < 4 * n * 2.0**-53
+
 
 @pytest.mark.parametrize("n", [96, 200, 256, 300])
 def test_inverse_split_and_fused_paths_agree(n):
