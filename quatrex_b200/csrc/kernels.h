@@ -35,6 +35,10 @@ struct GemmCall {
   const cplx* diag_shift = nullptr;
 };
 void launch_zgemm(const GemmCall& g, cudaStream_t stream);
+// Independent products in one launch (ZGEMM_GROUP_MAX at a time): no product
+// may write what another one of the group reads or writes.
+constexpr int ZGEMM_GROUP_MAX = 8;
+void launch_zgemm_group(const GemmCall* calls, int count, cudaStream_t stream);
 
 // Mixed-precision variant of the same contract: FP64 operands split into
 // 7-bit integer slices whose products run on tcgen05 kind::i8 with exact

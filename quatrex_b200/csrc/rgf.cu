@@ -325,6 +325,13 @@ struct Btd {
   bool dense(int k) const { return !index(k) && !empty(k); }
 };
 
+// A block of `m` is gathered from (or scattered to) a sparse pattern.
+bool has_sparse_block(const Btd& m) {
+  for (int k = 0; k < 3 * m.nb() - 2; ++k)
+    if (!m.empty(k) && !m.dense(k)) return true;
+  return false;
+}
+
 void validate_desc(const qtx_btd_desc* d, const char* name) {
   if (!d) throw QtxError(QTX_E_INVAL, std::string(name) + ": missing block descriptor");
   if (d->num_blocks < 1) throw QtxError(QTX_E_INVAL, std::string(name) + ": num_blocks < 1");
@@ -396,17 +403,52 @@ MatView obc_view(const void* const* arr, int i, int b, int64_t e0) {
   return MatView{p + e0 * (int64_t)b * b, b, (int64_t)b * b};
 }
 
-void gemm(int m, int n, int k, int64_t batch, cplx alpha, MatView a, int op_a, MatView b, int op_b, MutView d,
-          cudaStream_t s, MatView c = MatView{}, cplx beta = ZERO, MatView c2 = MatView{}, cplx gamma = ZERO,
-          const int* active = nullptr, const cplx* diag_shift = nullptr, int precision = QTX_PREC_FP64) {
+GemmCall gemm_call(int m, int n, int k, int64_t batch, cplx alpha, MatView a, int op_a, MatView b, int op_b, MutView d,
+                   MatView c = MatView{}, cplx beta = ZERO, MatView c2 = MatView{}, cplx gamma = ZERO,
+                   const int* active = nullptr, const cplx* diag_shift = nullptr) {
   GemmCall g;
   g.m = m; g.n = n; g.k = k; g.batch = batch;
   g.a = a; g.op_a = op_a; g.b = b; g.op_b = op_b;
   g.c = c; g.beta = beta; g.c2 = c2; g.gamma = gamma;
   g.d = d; g.alpha = alpha; g.active = active; g.diag_shift = diag_shift;
-  TimedScope ts(0, 8.0 * m * n * (double)k * batch, s);
-  if (precision == QTX_PREC_MIXED && mixed_supported(g)) launch_zgemm_mixed(g, s);
-  else launch_zgemm(g, s);
+  return g;
+}
+
+// Independent block products of one step of a recursion, in one launch (the
+// mixed form runs them one by one).  A small product leaves most of the GPU
+// idle and costs its latency whatever else runs beside it (32 matrices of
+// b = 64 are 128 tiles of 592 resident ones); at large sizes the products of
+// a step share their operands in L2 and a single last wave.  The results do
+// not depend on the grouping.
+struct GemmGroup {
+  cudaStream_t s;
+  int precision;
+  std::vector<GemmCall> calls;
+  GemmGroup(cudaStream_t stream, int prec = QTX_PREC_FP64) : s(stream), precision(prec) {}
+  void add(const GemmCall& g) { calls.push_back(g); }
+  void run() {
+    if (precision == QTX_PREC_MIXED) {
+      for (const GemmCall& g : calls) {
+        TimedScope ts(0, 8.0 * g.m * g.n * (double)g.k * g.batch, s);
+        if (mixed_supported(g)) launch_zgemm_mixed(g, s);
+        else launch_zgemm(g, s);
+      }
+    } else if (!calls.empty()) {
+      double flops = 0;
+      for (const GemmCall& g : calls) flops += 8.0 * g.m * g.n * (double)g.k * g.batch;
+      TimedScope ts(0, flops, s);
+      launch_zgemm_group(calls.data(), (int)calls.size(), s);
+    }
+    calls.clear();
+  }
+};
+
+void gemm(int m, int n, int k, int64_t batch, cplx alpha, MatView a, int op_a, MatView b, int op_b, MutView d,
+          cudaStream_t s, MatView c = MatView{}, cplx beta = ZERO, MatView c2 = MatView{}, cplx gamma = ZERO,
+          const int* active = nullptr, const cplx* diag_shift = nullptr, int precision = QTX_PREC_FP64) {
+  GemmGroup g(s, precision);
+  g.add(gemm_call(m, n, k, batch, alpha, a, op_a, b, op_b, d, c, beta, c2, gamma, active, diag_shift));
+  g.run();
 }
 
 // Block inverse with timing (8 n^3 algorithmic flops per matrix: getrf + getri).
@@ -537,17 +579,15 @@ void selected_inv_impl(qtx_ctx* ctx, const Btd& a, const void* const* obc_r, con
       const int j = i + 1, bi = sizes[i], bj = sizes[j];
       MatView a_ji = in_block(a, j, i, e0, ne, T[5], ws);
       MatView a_ij = in_block(a, i, j, e0, ne, T[6], ws);
-      // X_ji = -(X_jj A_ji) x_i
-      gemm(bj, bi, bj, ne, ONE, x.view(j), OP_N, a_ji, OP_N, tv(0, bi), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           precision);
-      gemm(bj, bi, bi, ne, MONE, tv(0, bi), OP_N, x.view(i), OP_N, tv(1, bi), s, {}, ZERO, {}, ZERO, nullptr,
-           nullptr, precision);
+      // X_ji = -(X_jj A_ji) x_i ; X_ij = -(x_i A_ij) X_jj
+      GemmGroup grp(s, precision);
+      grp.add(gemm_call(bj, bi, bj, ne, ONE, x.view(j), OP_N, a_ji, OP_N, tv(0, bi)));
+      grp.add(gemm_call(bi, bj, bi, ne, ONE, x.view(i), OP_N, a_ij, OP_N, tv(2, bj)));
+      grp.run();
+      grp.add(gemm_call(bj, bi, bi, ne, MONE, tv(0, bi), OP_N, x.view(i), OP_N, tv(1, bi)));
+      grp.add(gemm_call(bi, bj, bj, ne, MONE, tv(2, bj), OP_N, x.view(j), OP_N, tv(3, bj)));
+      grp.run();
       out_block(out, j, i, e0, ne, tv(1, bi), 0, ws);
-      // X_ij = -(x_i A_ij) X_jj
-      gemm(bi, bj, bi, ne, ONE, x.view(i), OP_N, a_ij, OP_N, tv(2, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           precision);
-      gemm(bi, bj, bj, ne, MONE, tv(2, bj), OP_N, x.view(j), OP_N, tv(3, bj), s, {}, ZERO, {}, ZERO, nullptr,
-           nullptr, precision);
       out_block(out, i, j, e0, ne, tv(3, bj), 0, ws);
       // X_ii = x_i - (x_i A_ij) X_ji
       gemm(bi, bi, bj, ne, MONE, tv(2, bj), OP_N, tv(1, bi), OP_N, tv(4, bi), s, x.view(i), ONE, {}, ZERO, nullptr,
@@ -616,7 +656,9 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
   for (size_t q = 0; q + 1 < offs.size(); ++q) ne_max = std::max(ne_max, offs[q + 1] - offs[q]);
   if (ne_max == 0) return;
 
-  const int NT = 12;
+  // Work matrices: 13, and 10 gather scratch ones when a block has a sparse pattern
+  const bool sparse = has_sparse_block(A.a) || has_sparse_block(A.sl) || has_sparse_block(A.sg);
+  const int NT = 13 + (sparse ? 10 : 0);
   const size_t tmp = (size_t)bmax * bmax * ne_max;
   std::vector<int> cur_sizes(sizes.begin() + 1, sizes.end());
   size_t total = 3 * stack_elems(sizes, ne_max) + NT * tmp + (size_t)bmax * bmax;
@@ -631,17 +673,23 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
     stl = carve(cur, cur_sizes, ne_max, bmax);
     stg = carve(cur, cur_sizes, ne_max, bmax);
   }
-  cplx* T[NT];
+  std::vector<cplx*> T(NT);
   for (int q = 0; q < NT; ++q) { T[q] = cur; cur += tmp; }
   Workspace ws{s, ne_max, bmax, cur};
   launch_fill_int(reinterpret_cast<int*>(ws.zero), (int64_t)4 * bmax * bmax, 0, s);
   cur += (size_t)bmax * bmax;
   int* info = reinterpret_cast<int*>(cur);
   launch_fill_int(info, ne_max * nb, 0, s);
+  // gather scratch: 0-2 and 3-5 A_ji, A_ij, A_jj of even and odd blocks, 6-7
+  // S_ij, 8-9 S_jj of the two components
+  auto gather = [&](int k) { return sparse ? T[13 + k] : nullptr; };
 
   const void* const* obc_r = A.obc ? A.obc->retarded : nullptr;
-  const void* const* obc_l = A.obc ? A.obc->lesser : nullptr;
-  const void* const* obc_g = A.obc ? A.obc->greater : nullptr;
+  const void* const* obc_c[2] = {A.obc ? A.obc->lesser : nullptr, A.obc ? A.obc->greater : nullptr};
+  const Btd* Sc[2] = {&A.sl, &A.sg};
+  const Btd* Oc[2] = {&A.xl, &A.xg};
+  BlockStack* Xc[2] = {&xl, &xg};
+  BlockStack* STc[2] = {&stl, &stg};
 
   // Which blocks of Sigma^< and Sigma^> hold a nonzero entry anywhere in the
   // stack.  ElectronSolver passes interior self-energies that are zero in the
@@ -654,11 +702,15 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
   for (size_t q = 0; q + 1 < offs.size(); ++q) {
     const int64_t e0 = offs[q], ne = offs[q + 1] - offs[q];
     auto tv = [&](int idx, int ld) { return MutView{T[idx], ld, (int64_t)bmax * bmax}; };
-    // G0..G3 (T[8..11]) are gather scratch for sparse input blocks
+    auto call = [&](int m, int n, int k, cplx f, MatView p, int op_p, MatView r, int op_r, MutView d,
+                    MatView c = MatView{}, cplx beta = ZERO, MatView c2 = MatView{}, cplx gamma = ZERO) {
+      return gemm_call(m, n, k, ne, f, p, op_p, r, op_r, d, c, beta, c2, gamma);
+    };
+    GemmGroup grp(s, prec);
     // ---- first block (rgf.py:207-231)
     {
       const int b0 = sizes[0];
-      MatView a00 = in_block(a, 0, 0, e0, ne, T[8], ws);
+      MatView a00 = in_block(a, 0, 0, e0, ne, gather(2), ws);
       MatView o = obc_view(obc_r, 0, b0, e0);
       if (o.ptr) {
         launch_axpby(b0, b0, ne, ONE, a00, MONE, o, tv(0, b0), s);
@@ -666,91 +718,126 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       } else {
         zinv(b0, ne, a00, xr.view(0), info, nullptr, s);
       }
-      for (int comp = 0; comp < 2; ++comp) {
-        const Btd& S = comp == 0 ? A.sl : A.sg;
-        const void* const* ob = comp == 0 ? obc_l : obc_g;
-        BlockStack& X = comp == 0 ? xl : xg;
-        MatView s00 = in_block(S, 0, 0, e0, ne, T[9], ws);
-        MatView o2 = obc_view(ob, 0, b0, e0);
-        MatView sv = s00;
+      for (int c = 0; c < 2; ++c) {
+        MatView sv = in_block(*Sc[c], 0, 0, e0, ne, gather(8 + c), ws);
+        MatView o2 = obc_view(obc_c[c], 0, b0, e0);
         if (o2.ptr) {
-          launch_axpby(b0, b0, ne, ONE, s00, ONE, o2, tv(1, b0), s);
-          sv = tv(1, b0);
+          launch_axpby(b0, b0, ne, ONE, sv, ONE, o2, tv(4 + 4 * c, b0), s);
+          sv = tv(4 + 4 * c, b0);
         }
-        gemm(b0, b0, b0, ne, ONE, xr.view(0), OP_N, sv, OP_N, tv(2, b0), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-             prec);
-        gemm(b0, b0, b0, ne, ONE, tv(2, b0), OP_N, xr.view(0), OP_C, X.view(0), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
+        grp.add(call(b0, b0, b0, ONE, xr.view(0), OP_N, sv, OP_N, tv(5 + 4 * c, b0)));
       }
+      grp.run();
+      for (int c = 0; c < 2; ++c)
+        grp.add(call(b0, b0, b0, ONE, tv(5 + 4 * c, b0), OP_N, xr.view(0), OP_C, Xc[c]->view(0)));
+      grp.run();
     }
-    // ---- forward sweep (rgf.py:233-295)
-    for (int i = 0; i + 1 < nb; ++i) {
-      const int j = i + 1, bi = sizes[i], bj = sizes[j];
-      MatView a_ji = in_block(a, j, i, e0, ne, T[8], ws);
-      MatView a_ij = in_block(a, i, j, e0, ne, T[9], ws);
-      {
-        MatView a_jj = in_block(a, j, j, e0, ne, T[10], ws);
-        // U = A_ji x_i ; M = A_jj - Sigma^R_j - U A_ij ; x_j = inv(M)
-        gemm(bj, bi, bi, ne, ONE, a_ji, OP_N, xr.view(i), OP_N, tv(0, bi), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-             prec);
-        gemm(bj, bj, bi, ne, MONE, tv(0, bi), OP_N, a_ij, OP_N, tv(1, bj), s, a_jj, ONE,
-             obc_view(obc_r, j, bj, e0), MONE, nullptr, nullptr, prec);
-        zinv(bj, ne, tv(1, bj), xr.view(j), info + (int64_t)j * ne_max, nullptr, s);
-      }
+    // ---- forward sweep (rgf.py:233-295).  Work matrices: U 0, M 1, of
+    // component c W_c, V_c, Q_c, x_j Q_c from 2 + 4 c on, the second W 10.
+    // U = A_ji x_i and M = A_jj - Sigma^R_j - U A_ij of the next step ride with
+    // the products of this one; X_c,j of a step without injection (pend) with
+    // the first launch of the next.
+    struct Couplings {
+      MatView ji, ij, jj;
+    };
+    auto couplings = [&](int j) {
+      const int i = j - 1, k = 3 * (j & 1);
+      return Couplings{in_block(a, j, i, e0, ne, gather(k), ws), in_block(a, i, j, e0, ne, gather(k + 1), ws),
+                       in_block(a, j, j, e0, ne, gather(k + 2), ws)};
+    };
+    auto add_u = [&](int j, const Couplings& k) {
+      grp.add(call(sizes[j], sizes[j - 1], sizes[j - 1], ONE, k.ji, OP_N, xr.view(j - 1), OP_N, tv(0, sizes[j - 1])));
+    };
+    auto add_m = [&](int j, const Couplings& k) {
+      grp.add(call(sizes[j], sizes[j], sizes[j - 1], MONE, tv(0, sizes[j - 1]), OP_N, k.ij, OP_N, tv(1, sizes[j]),
+                   k.jj, ONE, obc_view(obc_r, j, sizes[j], e0), MONE));
+    };
+    std::vector<GemmCall> pend;
+    Couplings now;
+    if (nb > 1) {
+      now = couplings(1);
+      add_u(1, now);
+      grp.run();
+      add_m(1, now);
+      grp.run();
+    }
+    int w_at = 2;
+    for (int j = 1; j < nb; ++j) {
+      const int i = j - 1, bi = sizes[i], bj = sizes[j];
+      const bool more = j + 1 < nb;
+      zinv(bj, ne, tv(1, bj), xr.view(j), info + (int64_t)j * ne_max, nullptr, s);
+      Couplings next;
+      if (more) next = couplings(j + 1);
+      for (const GemmCall& g : pend) grp.add(g);
+      pend.clear();
       // W = x_j A_ji, shared by both components when neither injects at
       // (i, j) or (j, j): X_j = W X_i W^H (3 products for two components
       // instead of 8)
       bool shared_w = !want_cur;
-      for (int comp = 0; comp < 2; ++comp)
-        shared_w = shared_w && !nz(comp, i, j) && !nz(comp, j, j) && !obc_view(comp == 0 ? obc_l : obc_g, j, bj, e0).ptr;
+      for (int c = 0; c < 2; ++c)
+        shared_w = shared_w && !nz(c, i, j) && !nz(c, j, j) && !obc_view(obc_c[c], j, bj, e0).ptr;
       if (shared_w) {
-        gemm(bj, bi, bj, ne, ONE, xr.view(j), OP_N, a_ji, OP_N, tv(2, bi), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-             prec);
-        for (int comp = 0; comp < 2; ++comp) {
-          BlockStack& X = comp == 0 ? xl : xg;
-          gemm(bj, bi, bi, ne, ONE, tv(2, bi), OP_N, X.view(i), OP_N, tv(5, bi), s, {}, ZERO, {}, ZERO, nullptr,
-               nullptr, prec);
-          gemm(bj, bj, bi, ne, ONE, tv(5, bi), OP_N, tv(2, bi), OP_C, X.view(j), s, {}, ZERO, {}, ZERO, nullptr,
-               nullptr, prec);
-        }
+        const MutView w = tv(w_at, bi);
+        grp.add(call(bj, bi, bj, ONE, xr.view(j), OP_N, now.ji, OP_N, w));
+        if (more) add_u(j + 1, next);
+        grp.run();
+        for (int c = 0; c < 2; ++c)
+          grp.add(call(bj, bi, bi, ONE, w, OP_N, Xc[c]->view(i), OP_N, tv(5 + 4 * c, bi)));
+        if (more) add_m(j + 1, next);
+        grp.run();
+        for (int c = 0; c < 2; ++c)
+          pend.push_back(call(bj, bj, bi, ONE, tv(5 + 4 * c, bi), OP_N, w, OP_C, Xc[c]->view(j)));
+        w_at = w_at == 2 ? 10 : 2;
+        now = next;
         continue;
       }
-      for (int comp = 0; comp < 2; ++comp) {
-        const Btd& S = comp == 0 ? A.sl : A.sg;
-        const void* const* ob = comp == 0 ? obc_l : obc_g;
-        BlockStack& X = comp == 0 ? xl : xg;
-        const bool inj_ij = nz(comp, i, j);
-        MatView s_ij = inj_ij ? in_block(S, i, j, e0, ne, T[10], ws) : MatView{};
-        MatView s_jj = nz(comp, j, j) ? in_block(S, j, j, e0, ne, T[11], ws) : MatView{};
-        // W = U S_ij (zero when S_ij is)
-        if (inj_ij)
-          gemm(bj, bj, bi, ne, ONE, tv(0, bi), OP_N, s_ij, OP_N, tv(2, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-               prec);
-        // V = X_i A_ji^H
-        gemm(bi, bj, bi, ne, ONE, X.view(i), OP_N, a_ji, OP_C, tv(3, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-             prec);
+      grp.run();  // X_c,i complete
+      for (int c = 0; c < 2; ++c) {
+        // W = U S_ij (zero when S_ij is) ; V = X_i A_ji^H
+        if (nz(c, i, j))
+          grp.add(call(bj, bj, bi, ONE, tv(0, bi), OP_N, in_block(*Sc[c], i, j, e0, ne, gather(6 + c), ws), OP_N,
+                       tv(2 + 4 * c, bj)));
+        grp.add(call(bi, bj, bi, ONE, Xc[c]->view(i), OP_N, now.ji, OP_C, tv(3 + 4 * c, bj)));
+      }
+      grp.run();
+      for (int c = 0; c < 2; ++c) {
+        // Q = A_ji V + W^H - W + S_jj + Sigma^<_obc,j ; the layer current keeps
+        // Sigma~ = A_ji V + W^H - W
         if (want_cur) {
-          BlockStack& ST = comp == 0 ? stl : stg;
-          // Sigma~ = A_ji V + W^H - W  (kept for the layer current)
-          gemm(bj, bj, bi, ne, ONE, a_ji, OP_N, tv(3, bj), OP_N, ST.view(i), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-               prec);
-          if (inj_ij) launch_skew_combine(bj, ne, ST.view(i), tv(2, bj), ST.view(i), s);
-          launch_axpby(bj, bj, ne, ONE, ST.view(i), ONE, s_jj.ptr ? s_jj : MatView{ws.zero, bj, 0}, tv(4, bj), s);
-          MatView o2 = obc_view(ob, j, bj, e0);
-          if (o2.ptr) launch_axpby(bj, bj, ne, ONE, tv(4, bj), ONE, o2, tv(4, bj), s);
+          grp.add(call(bj, bj, bi, ONE, now.ji, OP_N, tv(3 + 4 * c, bj), OP_N, STc[c]->view(i)));
         } else {
-          // Q = A_ji V + S_jj + Sigma^<_obc,j ; Q += W^H - W
-          gemm(bj, bj, bi, ne, ONE, a_ji, OP_N, tv(3, bj), OP_N, tv(4, bj), s, s_jj, ONE, obc_view(ob, j, bj, e0),
-               ONE, nullptr, nullptr, prec);
-          if (inj_ij) launch_skew_combine(bj, ne, tv(4, bj), tv(2, bj), tv(4, bj), s);
+          const MatView s_jj = nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, gather(8 + c), ws) : MatView{};
+          grp.add(call(bj, bj, bi, ONE, now.ji, OP_N, tv(3 + 4 * c, bj), OP_N, tv(4 + 4 * c, bj), s_jj, ONE,
+                       obc_view(obc_c[c], j, bj, e0), ONE));
+        }
+      }
+      if (more) add_u(j + 1, next);  // (U of this step is in W already)
+      grp.run();
+      for (int c = 0; c < 2; ++c) {
+        const MutView w = tv(2 + 4 * c, bj), qv = tv(4 + 4 * c, bj);
+        if (want_cur) {
+          const MutView st = STc[c]->view(i);
+          if (nz(c, i, j)) launch_skew_combine(bj, ne, st, w, st, s);
+          const MatView s_jj =
+              nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, gather(8 + c), ws) : MatView{ws.zero, bj, 0};
+          launch_axpby(bj, bj, ne, ONE, st, ONE, s_jj, qv, s);
+          const MatView o2 = obc_view(obc_c[c], j, bj, e0);
+          if (o2.ptr) launch_axpby(bj, bj, ne, ONE, qv, ONE, o2, qv, s);
+        } else if (nz(c, i, j)) {
+          launch_skew_combine(bj, ne, qv, w, qv, s);
         }
         // X_j = x_j Q x_j^H
-        gemm(bj, bj, bj, ne, ONE, xr.view(j), OP_N, tv(4, bj), OP_N, tv(5, bj), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
-        gemm(bj, bj, bj, ne, ONE, tv(5, bj), OP_N, xr.view(j), OP_C, X.view(j), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
+        grp.add(call(bj, bj, bj, ONE, xr.view(j), OP_N, qv, OP_N, tv(5 + 4 * c, bj)));
       }
+      if (more) add_m(j + 1, next);
+      grp.run();
+      for (int c = 0; c < 2; ++c)
+        grp.add(call(bj, bj, bj, ONE, tv(5 + 4 * c, bj), OP_N, xr.view(j), OP_C, Xc[c]->view(j)));
+      grp.run();
+      now = next;
     }
+    for (const GemmCall& g : pend) grp.add(g);
+    grp.run();
     // ---- last diagonal blocks (rgf.py:297-305)
     {
       const int n = nb - 1;
@@ -758,65 +845,62 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       out_block(A.xg, n, n, e0, ne, xg.view(n), 1, ws);
       if (want_r) out_block(A.xr, n, n, e0, ne, xr.view(n), 0, ws);
     }
-    // ---- backward sweep (rgf.py:307-404)
+    // ---- backward sweep (rgf.py:307-404).  Work matrices: P1 0, P2 1, P3 10,
+    // P4 11, the new x_i 12, of component c Y, t1, t2, X_ij from 2 + 4 c on.
     for (int i = nb - 2; i >= 0; --i) {
       const int j = i + 1, bi = sizes[i], bj = sizes[j];
-      MatView a_ij = in_block(a, i, j, e0, ne, T[8], ws);
-      MatView a_ji = in_block(a, j, i, e0, ne, T[9], ws);
-      // P1 = x_i A_ij (bi x bj), P2 = X_jj A_ji (bj x bi), P3 = P1 X_jj, P4 = P1 P2
-      gemm(bi, bj, bi, ne, ONE, xr.view(i), OP_N, a_ij, OP_N, tv(0, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           prec);
-      gemm(bj, bi, bj, ne, ONE, xr.view(j), OP_N, a_ji, OP_N, tv(1, bi), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           prec);
-      gemm(bi, bj, bj, ne, ONE, tv(0, bj), OP_N, xr.view(j), OP_N, tv(2, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           prec);
-      gemm(bi, bi, bj, ne, ONE, tv(0, bj), OP_N, tv(1, bi), OP_N, tv(3, bi), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           prec);
+      MatView a_ij = in_block(a, i, j, e0, ne, gather(1), ws);
+      MatView a_ji = in_block(a, j, i, e0, ne, gather(0), ws);
+      const MutView p1 = tv(0, bj), p2 = tv(1, bi), p3 = tv(10, bj), p4 = tv(11, bi), gii = tv(12, bi);
+      auto y = [&](int c) { return tv(2 + 4 * c, bj); };
+      auto t1 = [&](int c) { return tv(3 + 4 * c, bi); };
+      auto t2 = [&](int c) { return tv(4 + 4 * c, bj); };
+      auto xij = [&](int c) { return tv(5 + 4 * c, bj); };
+      const bool inj[2] = {nz(0, i, j), nz(1, i, j)};
+      // P1 = x_i A_ij (bi x bj), P2 = X_jj A_ji (bj x bi), Y = x_i S_ij (zero when S_ij is)
+      grp.add(call(bi, bj, bi, ONE, xr.view(i), OP_N, a_ij, OP_N, p1));
+      grp.add(call(bj, bi, bj, ONE, xr.view(j), OP_N, a_ji, OP_N, p2));
+      for (int c = 0; c < 2; ++c)
+        if (inj[c])
+          grp.add(call(bi, bj, bi, ONE, xr.view(i), OP_N, in_block(*Sc[c], i, j, e0, ne, gather(6 + c), ws), OP_N,
+                       y(c)));
+      grp.run();
+      // P3 = P1 X_jj (only injection and the off-diagonal X^R use it), P4 = P1 P2, t2 = P1 X_j
+      if (want_r_off || inj[0] || inj[1]) grp.add(call(bi, bj, bj, ONE, p1, OP_N, xr.view(j), OP_N, p3));
+      grp.add(call(bi, bi, bj, ONE, p1, OP_N, p2, OP_N, p4));
+      for (int c = 0; c < 2; ++c) grp.add(call(bi, bj, bj, ONE, p1, OP_N, Xc[c]->view(j), OP_N, t2(c)));
+      grp.run();
       if (want_r_off) {
         // X^R_ij = -P3 ; X^R_ji = -P2 x_i
-        launch_axpby(bi, bj, ne, MONE, tv(2, bj), ZERO, {}, tv(4, bj), s);
-        out_block(A.xr, i, j, e0, ne, tv(4, bj), 0, ws);
-        gemm(bj, bi, bi, ne, MONE, tv(1, bi), OP_N, xr.view(i), OP_N, tv(4, bi), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
-        out_block(A.xr, j, i, e0, ne, tv(4, bi), 0, ws);
+        launch_axpby(bi, bj, ne, MONE, p3, ZERO, {}, tv(12, bj), s);
+        out_block(A.xr, i, j, e0, ne, tv(12, bj), 0, ws);
+        grp.add(call(bj, bi, bi, MONE, p2, OP_N, xr.view(i), OP_N, tv(12, bi)));
+        grp.run();
+        out_block(A.xr, j, i, e0, ne, tv(12, bi), 0, ws);
       }
-      for (int comp = 0; comp < 2; ++comp) {
-        const Btd& S = comp == 0 ? A.sl : A.sg;
-        const Btd& OUT = comp == 0 ? A.xl : A.xg;
-        BlockStack& X = comp == 0 ? xl : xg;
-        const bool inj_ij = nz(comp, i, j);
-        MatView s_ij = inj_ij ? in_block(S, i, j, e0, ne, T[10], ws) : MatView{};
-        // Y = x_i S_ij (zero when S_ij is)
-        if (inj_ij)
-          gemm(bi, bj, bi, ne, ONE, xr.view(i), OP_N, s_ij, OP_N, tv(4, bj), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-               prec);
-        // t1 = P4 X_i - Y P3^H ; t1 -= t1^H
-        gemm(bi, bi, bi, ne, ONE, tv(3, bi), OP_N, X.view(i), OP_N, tv(5, bi), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
-        if (inj_ij)
-          gemm(bi, bi, bj, ne, MONE, tv(4, bj), OP_N, tv(2, bj), OP_C, tv(5, bi), s, tv(5, bi), ONE, {}, ZERO,
-               nullptr, nullptr, prec);
-        launch_sub_herm_inplace(bi, ne, tv(5, bi), s);
-        // t2 = P1 X_j
-        gemm(bi, bj, bj, ne, ONE, tv(0, bj), OP_N, X.view(j), OP_N, tv(6, bj), s, {}, ZERO, {}, ZERO, nullptr,
-             nullptr, prec);
-        // X_ij = Y X_jj^H - t2 - X_i P2^H
-        if (inj_ij) {
-          gemm(bi, bj, bj, ne, ONE, tv(4, bj), OP_N, xr.view(j), OP_C, tv(7, bj), s, tv(6, bj), MONE, {}, ZERO,
-               nullptr, nullptr, prec);
-          gemm(bi, bj, bi, ne, MONE, X.view(i), OP_N, tv(1, bi), OP_C, tv(7, bj), s, tv(7, bj), ONE, {}, ZERO,
-               nullptr, nullptr, prec);
-        } else {
-          gemm(bi, bj, bi, ne, MONE, X.view(i), OP_N, tv(1, bi), OP_C, tv(7, bj), s, tv(6, bj), MONE, {}, ZERO,
-               nullptr, nullptr, prec);
-        }
-        out_block(OUT, i, j, e0, ne, tv(7, bj), 0, ws);
-        if (!symmetric) out_block(OUT, j, i, e0, ne, tv(7, bj), 2, ws);
+      // t1 = P4 X_i - Y P3^H ; X_ij = Y X_jj^H - t2 - X_i P2^H ; G_ii = x_i + P4 x_i
+      for (int c = 0; c < 2; ++c) {
+        grp.add(call(bi, bi, bi, ONE, p4, OP_N, Xc[c]->view(i), OP_N, t1(c)));
+        if (inj[c]) grp.add(call(bi, bj, bj, ONE, y(c), OP_N, xr.view(j), OP_C, xij(c), t2(c), MONE));
+        else grp.add(call(bi, bj, bi, MONE, Xc[c]->view(i), OP_N, p2, OP_C, xij(c), t2(c), MONE));
+      }
+      grp.add(call(bi, bi, bi, ONE, p4, OP_N, xr.view(i), OP_N, gii, xr.view(i), ONE));
+      grp.run();
+      for (int c = 0; c < 2; ++c) {
+        if (!inj[c]) continue;
+        grp.add(call(bi, bi, bj, MONE, y(c), OP_N, p3, OP_C, t1(c), t1(c), ONE));
+        grp.add(call(bi, bj, bi, MONE, Xc[c]->view(i), OP_N, p2, OP_C, xij(c), xij(c), ONE));
+      }
+      grp.run();
+      for (int c = 0; c < 2; ++c) {
+        launch_sub_herm_inplace(bi, ne, t1(c), s);
+        out_block(*Oc[c], i, j, e0, ne, xij(c), 0, ws);
+        if (!symmetric) out_block(*Oc[c], j, i, e0, ne, xij(c), 2, ws);
         // X_i += t2 P1^H + t1
-        gemm(bi, bi, bj, ne, ONE, tv(6, bj), OP_N, tv(0, bj), OP_C, X.view(i), s, X.view(i), ONE, tv(5, bi), ONE,
-             nullptr, nullptr, prec);
-        out_block(OUT, i, i, e0, ne, X.view(i), 1, ws);
+        grp.add(call(bi, bi, bj, ONE, t2(c), OP_N, p1, OP_C, Xc[c]->view(i), Xc[c]->view(i), ONE, t1(c), ONE));
       }
+      grp.run();
+      for (int c = 0; c < 2; ++c) out_block(*Oc[c], i, i, e0, ne, Xc[c]->view(i), 1, ws);
       if (want_cur) {
         // current_i = Tr[Sigma~^>_i X^<_j - X^>_j Sigma~^<_i]
         cplx* cur_out = T[11];
@@ -826,10 +910,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         launch_axpby(1, 1, ne, ONE, MatView{cur_out, 1, 1}, ZERO, {}, MutView{A.current + e0 * (nb - 1) + i, 1, nb - 1},
                      s);
       }
-      // x_i <- x_i + P4 x_i  (full G^R_ii)
-      gemm(bi, bi, bi, ne, ONE, tv(3, bi), OP_N, xr.view(i), OP_N, tv(4, bi), s, xr.view(i), ONE, {}, ZERO, nullptr,
-           nullptr, prec);
-      std::swap(xr.ptr[i], T[4]);
+      std::swap(xr.ptr[i], T[12]);
       if (want_r) out_block(A.xr, i, i, e0, ne, xr.view(i), 0, ws);
     }
   }
@@ -840,16 +921,17 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Sancho-Rubio (src/qttools/boundary_conditions/obc/sancho_rubio.py:33-86)
 // ---------------------------------------------------------------------------
+constexpr int SR_TEMPS = 10;  // n x n work matrices per batch entry
 // Returns true when every entry converged.
 bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView a_ij, MatView a_ji, double tol,
                        int max_iter, MutView x, int* iterations, cudaStream_t s) {
   const size_t mat = (size_t)n * n * batch;
-  DevBuf buf(sizeof(cplx) * 9 * mat + sizeof(int) * (3 * batch + 2), s);
+  DevBuf buf(sizeof(cplx) * SR_TEMPS * mat + sizeof(int) * (3 * batch + 2), s);
   cplx* p = buf.as<cplx>();
   auto slot = [&](int q) { return MutView{p + q * mat, n, (int64_t)n * n}; };
   MutView eps = slot(0), eps_s = slot(1), alpha = slot(2), beta = slot(3), inv = slot(4), t0 = slot(5),
-          t1 = slot(6), t2 = slot(7), t3 = slot(8);
-  int* active = reinterpret_cast<int*>(p + 9 * mat);
+          t1 = slot(6), t2 = slot(7), t3 = slot(8), t4 = slot(9);
+  int* active = reinterpret_cast<int*>(p + SR_TEMPS * mat);
   int* its = active + batch;
   int* num_active = its + batch;
   int* info = num_active + 2;  // zero pivots of the decimation inverses (sticky over the iterations)
@@ -863,16 +945,22 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView
   bool converged = false;
   for (int it = 0; it < max_iter; ++it) {
     zinv(n, batch, eps, inv, info, active, s);
-    gemm(n, n, n, batch, ONE, alpha, OP_N, inv, OP_N, t0, s, {}, ZERO, {}, ZERO, active);   // a inv
-    gemm(n, n, n, batch, ONE, beta, OP_N, inv, OP_N, t1, s, {}, ZERO, {}, ZERO, active);    // b inv
-    gemm(n, n, n, batch, ONE, t0, OP_N, beta, OP_N, t2, s, {}, ZERO, {}, ZERO, active);     // a inv b
-    launch_axpby(n, n, batch, ONE, eps_s, MONE, t2, eps_s, s, active);                      // eps_s -= a inv b
-    // eps = eps - a inv b - b inv a
-    gemm(n, n, n, batch, MONE, t1, OP_N, alpha, OP_N, eps, s, eps, ONE, t2, MONE, active);
-    gemm(n, n, n, batch, ONE, t0, OP_N, alpha, OP_N, t3, s, {}, ZERO, {}, ZERO, active);    // a inv a
-    gemm(n, n, n, batch, ONE, t1, OP_N, beta, OP_N, t2, s, {}, ZERO, {}, ZERO, active);     // b inv b
+    GemmGroup grp(s);
+    auto prod = [&](cplx f, MatView x1, MatView x2, MutView d, MatView c = MatView{}) {
+      grp.add(gemm_call(n, n, n, batch, f, x1, OP_N, x2, OP_N, d, c, ONE, {}, ZERO, active));
+    };
+    prod(ONE, alpha, inv, t0);  // a inv
+    prod(ONE, beta, inv, t1);   // b inv
+    grp.run();
+    prod(ONE, t0, beta, t2);          // a inv b
+    prod(ONE, t0, alpha, t3);         // a inv a
+    prod(ONE, t1, beta, t4);          // b inv b
+    prod(MONE, t1, alpha, eps, eps);  // eps -= b inv a
+    grp.run();
+    launch_axpby(n, n, batch, ONE, eps_s, MONE, t2, eps_s, s, active);  // eps_s -= a inv b
+    launch_axpby(n, n, batch, ONE, eps, MONE, t2, eps, s, active);      // eps -= a inv b
     std::swap(alpha.ptr, t3.ptr);
-    std::swap(beta.ptr, t2.ptr);
+    std::swap(beta.ptr, t4.ptr);
     launch_fill_int(num_active, 1, 0, s);
     launch_sr_norm_update(n, batch, alpha, beta, tol, active, its, num_active, s);
     if (read_status(ctx, num_active, 1, s).head == 0) {
@@ -1044,23 +1132,37 @@ void transport_sweep(TransportWS w, const qtx_transport_problem& P, const qtx_tr
   zinv(b, ne, tv(1), xr.view(0), info, nullptr, s);
   gemm(b, b, b, ne, I1, xr.view(0), OP_N, V(C[8]), OP_N, tv(2), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
   gemm(b, b, b, ne, ONE, tv(2), OP_N, xr.view(0), OP_C, yl.view(0), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-  // ---- forward sweep
-  for (int i = 0; i + 1 < nb; ++i) {
-    const int j = i + 1;
-    gemm(b, b, b, ne, ONE, lo(i), OP_N, xr.view(i), OP_N, tv(0), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    // M = (E + i eta) I - H_jj - Sigma^R_j - U A_ij
-    gemm(b, b, b, ne, MONE, tv(0), OP_N, up(i), OP_N, tv(1), s, hd(j), MONE, obc_r(j), MONE, nullptr, shift, prec);
-    zinv(b, ne, tv(1), xr.view(j), info + (int64_t)j * ne_max, nullptr, s);
-    // X_L,j = x_j A_ji X_L,i A_ji^H x_j^H = W X_L,i W^H with W = x_j A_ji
-    // (no source past block 0)
-    gemm(b, b, b, ne, ONE, xr.view(j), OP_N, lo(i), OP_N, tv(3), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, tv(3), OP_N, yl.view(i), OP_N, tv(4), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, tv(4), OP_N, tv(3), OP_C, yl.view(j), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
+  // ---- forward sweep.  X_L,j = x_j A_ji X_L,i A_ji^H x_j^H = W_j X_L,i W_j^H with W_j = x_j A_ji (no
+  // source past block 0) does not hold up the chain of the x_j, so its three
+  // products ride with the next steps' U and M, one behind the other:
+  //   { U_j+1, W_j, X_L,j-1 } { M_j+1, W_j X_L,j-1 } inverse ...
+  auto sq = [&](cplx f, MatView p, int op_p, MatView q, int op_q, MutView d, MatView c = MatView{}, cplx beta = ZERO,
+                MatView c2 = MatView{}, cplx gamma = ZERO, const cplx* dshift = nullptr) {
+    return gemm_call(b, b, b, ne, f, p, op_p, q, op_q, d, c, beta, c2, gamma, nullptr, dshift);
+  };
+  GemmGroup grp(s, prec);
+  MutView w_now = tv(3), w_old = tv(5);  // W_j, W_j-1
+  for (int j = 0; j < nb; ++j) {
+    // on entry x_j is known, X_L up to block j - 2 and W_{j-1} X_L,{j-2} (in tv(4))
+    if (j + 1 < nb) grp.add(sq(ONE, lo(j), OP_N, xr.view(j), OP_N, tv(0)));  // U = A_{j+1,j} x_j
+    if (j >= 1) grp.add(sq(ONE, xr.view(j), OP_N, lo(j - 1), OP_N, w_now));
+    if (j >= 2) grp.add(sq(ONE, tv(4), OP_N, w_old, OP_C, yl.view(j - 1)));
+    grp.run();
+    // M = (E + i eta) I - H_kk - Sigma^R_k - U A_jk, k = j + 1
+    if (j + 1 < nb)
+      grp.add(sq(MONE, tv(0), OP_N, up(j), OP_N, tv(1), hd(j + 1), MONE, obc_r(j + 1), MONE, shift));
+    if (j >= 1) grp.add(sq(ONE, w_now, OP_N, yl.view(j - 1), OP_N, tv(4)));
+    grp.run();
+    if (j + 1 < nb) zinv(b, ne, tv(1), xr.view(j + 1), info + (int64_t)(j + 1) * ne_max, nullptr, s);
+    std::swap(w_now, w_old);
   }
   // ---- last block: X_R,n = x_n (i Gamma_R) x_n^H, outputs, corner chain start
   const int n = nb - 1;
-  gemm(b, b, b, ne, I1, xr.view(n), OP_N, V(C[9]), OP_N, tv(2), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-  gemm(b, b, b, ne, ONE, tv(2), OP_N, xr.view(n), OP_C, yr.view(n), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
+  if (n > 0) grp.add(sq(ONE, tv(4), OP_N, w_old, OP_C, yl.view(n)));
+  grp.add(sq(I1, xr.view(n), OP_N, V(C[9]), OP_N, tv(2)));
+  grp.run();
+  grp.add(sq(ONE, tv(2), OP_N, xr.view(n), OP_C, yr.view(n)));
+  grp.run();
   launch_keldysh_combine(b, ne, yl.view(n), yr.view(n), fl, fr, 1.0, true, out_ptr(O.gl_diag, nb, n), nb * bb,
                          out_ptr(O.gg_diag, nb, n), nb * bb, s);
   if (O.gr_diag) launch_axpby(b, b, ne, ONE, xr.view(n), ZERO, {}, out_at(O.gr_diag, nb, n), s);
@@ -1078,48 +1180,54 @@ void transport_sweep(TransportWS w, const qtx_transport_problem& P, const qtx_tr
   cplx* corner = T[8];
   cplx* corner2 = T[9];
   if (O.transmission) launch_axpby(b, b, ne, ONE, xr.view(n), ZERO, {}, V(corner), s);
-  // ---- backward sweep
+  // ---- backward sweep: three launches of independent products per block
+  //   { P4 = P1 P2, G_ij, G_ji, corner, t2 = P1 X_L,j, t2R = P1 X_R,j }
+  //   { t1 = P4 X_L,i, X_ij, X_R,i, G_ii }
+  //   { X_L,i += t2 P1^H + t1 - t1^H, P1 = x_i A_ij and P2 = G_jj A_ji of the next block }
+  // (P1 alternates between two buffers; g_L is not needed any more).
+  MutView p1 = tv(0), p1_next = V(C[0]);
+  auto add_p = [&](int i, MutView p) {
+    grp.add(sq(ONE, xr.view(i), OP_N, up(i), OP_N, p));
+    grp.add(sq(ONE, xr.view(i + 1), OP_N, lo(i), OP_N, tv(1)));
+  };
+  if (nb > 1) add_p(nb - 2, p1);
+  grp.run();
   for (int i = nb - 2; i >= 0; --i) {
     const int j = i + 1;
-    gemm(b, b, b, ne, ONE, xr.view(i), OP_N, up(i), OP_N, tv(0), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, xr.view(j), OP_N, lo(i), OP_N, tv(1), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
     // G^R_ij = -P1 G_jj: only an output, so written there directly (and
     // skipped when it is not asked for)
-    if (O.gr_upper)
-      gemm(b, b, b, ne, MONE, tv(0), OP_N, xr.view(j), OP_N, out_at(O.gr_upper, nb - 1, i), s, {}, ZERO, {}, ZERO,
-           nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, tv(0), OP_N, tv(1), OP_N, tv(3), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    if (O.gr_lower)
-      gemm(b, b, b, ne, MONE, tv(1), OP_N, xr.view(i), OP_N, out_at(O.gr_lower, nb - 1, i), s, {}, ZERO, {}, ZERO,
-           nullptr, nullptr, prec);
+    if (O.gr_upper) grp.add(sq(MONE, p1, OP_N, xr.view(j), OP_N, out_at(O.gr_upper, nb - 1, i)));
+    grp.add(sq(ONE, p1, OP_N, tv(1), OP_N, tv(3)));
+    if (O.gr_lower) grp.add(sq(MONE, tv(1), OP_N, xr.view(i), OP_N, out_at(O.gr_lower, nb - 1, i)));
     if (O.transmission) {
       // G_{i,N-1} = -(x_i A_ij) G_{j,N-1}
-      gemm(b, b, b, ne, MONE, tv(0), OP_N, V(corner), OP_N, V(corner2), s, {}, ZERO, {}, ZERO, nullptr, nullptr,
-           prec);
+      grp.add(sq(MONE, p1, OP_N, V(corner), OP_N, V(corner2)));
       std::swap(corner, corner2);
     }
+    grp.add(sq(ONE, p1, OP_N, yl.view(j), OP_N, tv(6)));
+    grp.add(sq(ONE, p1, OP_N, yr.view(j), OP_N, tv(2)));
+    grp.run();
     // X_L: t1 = P4 X_i - (P4 X_i)^H ; t2 = P1 X_j ; X_ij = -t2 - X_i P2^H ; X_i += t2 P1^H + t1
-    gemm(b, b, b, ne, ONE, tv(3), OP_N, yl.view(i), OP_N, tv(5), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
+    // X_R (zero in the forward sweep): t2R = P1 X_j ; X_ij = -t2R ; X_i = t2R P1^H
+    grp.add(sq(ONE, tv(3), OP_N, yl.view(i), OP_N, tv(5)));
+    if (uppers) grp.add(sq(MONE, yl.view(i), OP_N, tv(1), OP_C, tv(7), tv(6), MONE));
+    grp.add(sq(ONE, tv(2), OP_N, p1, OP_C, yr.view(i)));
+    grp.add(sq(ONE, tv(3), OP_N, xr.view(i), OP_N, tv(4), xr.view(i), ONE));  // G_ii = x_i + P4 x_i
+    grp.run();
+    std::swap(xr.ptr[i], T[4]);
     launch_sub_herm_inplace(b, ne, tv(5), s);
-    gemm(b, b, b, ne, ONE, tv(0), OP_N, yl.view(j), OP_N, tv(6), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
+    grp.add(sq(ONE, tv(6), OP_N, p1, OP_C, yl.view(i), yl.view(i), ONE, tv(5), ONE));
+    if (i > 0) add_p(i - 1, p1_next);
+    grp.run();
+    std::swap(p1, p1_next);
     if (uppers)
-      gemm(b, b, b, ne, MONE, yl.view(i), OP_N, tv(1), OP_C, tv(7), s, tv(6), MONE, {}, ZERO, nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, tv(6), OP_N, tv(0), OP_C, yl.view(i), s, yl.view(i), ONE, tv(5), ONE, nullptr, nullptr,
-         prec);
-    // X_R (zero in the forward sweep): t2 = P1 X_j ; X_ij = -t2 ; X_i = t2 P1^H
-    gemm(b, b, b, ne, ONE, tv(0), OP_N, yr.view(j), OP_N, tv(5), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    gemm(b, b, b, ne, ONE, tv(5), OP_N, tv(0), OP_C, yr.view(i), s, {}, ZERO, {}, ZERO, nullptr, nullptr, prec);
-    if (uppers)
-      launch_keldysh_combine(b, ne, tv(7), tv(5), fl, fr, -1.0, false, out_ptr(O.gl_upper, nb - 1, i),
+      launch_keldysh_combine(b, ne, tv(7), tv(2), fl, fr, -1.0, false, out_ptr(O.gl_upper, nb - 1, i),
                              (nb - 1) * bb, out_ptr(O.gg_upper, nb - 1, i), (nb - 1) * bb, s);
-    launch_layer_current(b, ne, tv(7), tv(5), fl, fr, -1.0, h_up + i * bb, lcur, nb - 1, i, s);
+    launch_layer_current(b, ne, tv(7), tv(2), fl, fr, -1.0, h_up + i * bb, lcur, nb - 1, i, s);
     launch_keldysh_combine(b, ne, yl.view(i), yr.view(i), fl, fr, 1.0, true, out_ptr(O.gl_diag, nb, i), nb * bb,
                            out_ptr(O.gg_diag, nb, i), nb * bb, s);
     launch_keldysh_density(b, ne, yl.view(i), yr.view(i), fl, fr, O.density ? O.density + e0 * nb : nullptr,
                            O.hole_density ? O.hole_density + e0 * nb : nullptr, nb, i, s);
-    gemm(b, b, b, ne, ONE, tv(3), OP_N, xr.view(i), OP_N, tv(4), s, xr.view(i), ONE, {}, ZERO, nullptr, nullptr,
-         prec);
-    std::swap(xr.ptr[i], T[4]);
     if (O.gr_diag) launch_axpby(b, b, ne, ONE, xr.view(i), ZERO, {}, out_at(O.gr_diag, nb, i), s);
     launch_block_dos(b, ne, xr.view(i), dos, nb, i, s);
   }
@@ -1368,11 +1476,11 @@ struct HostArr {
 };
 
 // Energies per streamed batch: two staging sets plus the solver's work space
-// (about (3 nb + 20) bmax^2 complex per energy) in 70 % of the free memory.
+// (about (3 nb + 32) bmax^2 complex per energy) in 70 % of the free memory.
 int64_t host_batch(int64_t max_batch, int64_t NE, size_t staging_per_energy, int nb, int bmax) {
   size_t free_b = 0, total_b = 0;
   QTX_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-  const size_t ws = sizeof(cplx) * (size_t)(3 * nb + 20) * bmax * bmax;
+  const size_t ws = sizeof(cplx) * (size_t)(3 * nb + 32) * bmax * bmax;
   const size_t per = 2 * staging_per_energy + ws;
   int64_t ne = (int64_t)((double)free_b * 0.7 / (double)std::max<size_t>(per, 1));
   ne = std::max<int64_t>(1, std::min<int64_t>({ne, max_batch, NE}));
@@ -1740,9 +1848,9 @@ int64_t qtx_graph_replays(const qtx_ctx* ctx) { return ctx ? ctx->graph_replays 
 
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call, int32_t precision) {
   if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
-  const size_t b = (size_t)block_size, ne = (size_t)energies_per_call;
   size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
-  bytes += sizeof(cplx) * 9 * b * b * ne + sizeof(int) * (2 * ne + 2);  // Sancho-Rubio
+  bytes += sizeof(cplx) * SR_TEMPS * (size_t)block_size * block_size * energies_per_call +
+           sizeof(int) * (3 * (size_t)energies_per_call + 2);  // Sancho-Rubio
   if (precision == QTX_PREC_MIXED)
     bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
   bytes += zinv_workspace_bytes(block_size, energies_per_call);

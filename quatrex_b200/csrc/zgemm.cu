@@ -68,6 +68,12 @@ struct Params {
   cplx* d; int64_t ldd, sd; cplx alpha;
   const int* active;
   const cplx* diag_shift;
+  int op_a, op_b;
+};
+
+// Products of one launch (grid.y picks one).
+struct Group {
+  Params p[ZGEMM_GROUP_MAX];
 };
 
 // Load one K-slice of op(A) (TILE x BK) into shared memory.
@@ -161,8 +167,7 @@ __device__ __forceinline__ void mma_step(const cplx* sa, const cplx* sb, int m, 
 }
 
 template <int TILE, int OPA, int OPB>
-__global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_kernel(Params p) {
-  qtx_grid_dependency();
+__device__ __forceinline__ void gemm_tile(const Params& p, int m0, int n0) {
   using C = Cfg<TILE>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* smem = reinterpret_cast<cplx*>(smem_raw);
@@ -171,7 +176,6 @@ __global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_ke
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int wm0 = (warp >> 1) * C::W, wn0 = (warp & 1) * C::W;
-  const int m0 = blockIdx.y * TILE, n0 = blockIdx.x * TILE;
   const int ktiles = (p.k + BK - 1) / BK;
   // a warp tile outside the matrix only copies (small tile: the wide one is
   // taken where the tiles are full)
@@ -255,12 +259,48 @@ __global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_ke
 }
 
 template <int TILE, int OPA, int OPB>
+__global__ void __launch_bounds__(THREADS, Cfg<TILE>::CTAS_PER_SM) zgemm_dmma_kernel(Params p) {
+  qtx_grid_dependency();
+  gemm_tile<TILE, OPA, OPB>(p, blockIdx.y * TILE, blockIdx.x * TILE);
+}
+
+// Several products, grid.y picks one (32x32 tiles in row order along grid.x).
+__global__ void __launch_bounds__(THREADS, Cfg<32>::CTAS_PER_SM) zgemm_group_kernel(const __grid_constant__ Group g) {
+  qtx_grid_dependency();
+  const Params& p = g.p[blockIdx.y];
+  const int ntiles_n = (p.n + 31) / 32;
+  const int m0 = (int)(blockIdx.x / ntiles_n) * 32, n0 = (int)(blockIdx.x % ntiles_n) * 32;
+  if (m0 >= p.m) return;  // fewer tiles than the largest product
+  if (p.op_a == OP_N) {
+    if (p.op_b == OP_N) gemm_tile<32, OP_N, OP_N>(p, m0, n0);
+    else gemm_tile<32, OP_N, OP_C>(p, m0, n0);
+  } else {
+    if (p.op_b == OP_N) gemm_tile<32, OP_C, OP_N>(p, m0, n0);
+    else gemm_tile<32, OP_C, OP_C>(p, m0, n0);
+  }
+}
+
+template <int TILE, int OPA, int OPB>
 void launch_t(const Params& p, cudaStream_t stream) {
   constexpr int smem = Cfg<TILE>::SMEM_BYTES;
   // opt-in to the large shared-memory carve-out (per device)
   qtx_opt_in_smem((const void*)zgemm_dmma_kernel<TILE, OPA, OPB>, smem);
-  dim3 grid(ceil_div_u(p.n, TILE), ceil_div_u(p.m, TILE), (unsigned)(p.batch < 65535 ? p.batch : 65535));
+  const dim3 grid(ceil_div_u(p.n, TILE), ceil_div_u(p.m, TILE), (unsigned)(p.batch < 65535 ? p.batch : 65535));
   qtx_launch(zgemm_dmma_kernel<TILE, OPA, OPB>, grid, THREADS, smem, stream, p);
+}
+
+// Waves of the resident CTAs that `tiles` take.
+template <int TILE>
+int64_t waves(int64_t tiles) {
+  int dev = 0, sms = 0;
+  QTX_CUDA_TRY(cudaGetDevice(&dev));
+  QTX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t resident = (int64_t)Cfg<TILE>::CTAS_PER_SM * sms;
+  return (tiles + resident - 1) / resident;
+}
+template <int TILE>
+int64_t tiles_of(const Params& p) {
+  return (int64_t)((p.m + TILE - 1) / TILE) * ((p.n + TILE - 1) / TILE) * p.batch;
 }
 
 // The tile whose waves finish first.  A full wave of 64x64 tiles covers twice
@@ -272,14 +312,7 @@ void launch_t(const Params& p, cudaStream_t stream) {
 // us for 16 of b = 256 (two waves against one).
 bool wide_tile(const Params& p) {
   if (p.m > 32 * 65535) return true;  // grid.y
-  int dev = 0, sms = 0;
-  QTX_CUDA_TRY(cudaGetDevice(&dev));
-  QTX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  auto waves = [&](int64_t tile, int64_t resident) {
-    const int64_t tiles = ((p.m + tile - 1) / tile) * ((p.n + tile - 1) / tile) * p.batch;
-    return (tiles + resident * sms - 1) / (resident * sms);
-  };
-  return 0.985 * 2.0 * (double)waves(64, Cfg<64>::CTAS_PER_SM) <= (double)waves(32, Cfg<32>::CTAS_PER_SM);
+  return 0.985 * 2.0 * (double)waves<64>(tiles_of<64>(p)) <= (double)waves<32>(tiles_of<32>(p));
 }
 
 template <int OPA, int OPB>
@@ -288,10 +321,28 @@ void launch_op(const Params& p, cudaStream_t stream) {
   else launch_t<32, OPA, OPB>(p, stream);
 }
 
-}  // namespace
+void launch_one(const Params& p, cudaStream_t stream) {
+  if (p.op_a == OP_N && p.op_b == OP_N) launch_op<OP_N, OP_N>(p, stream);
+  else if (p.op_a == OP_N && p.op_b == OP_C) launch_op<OP_N, OP_C>(p, stream);
+  else if (p.op_a == OP_C && p.op_b == OP_N) launch_op<OP_C, OP_N>(p, stream);
+  else launch_op<OP_C, OP_C>(p, stream);
+  qtx_check_launch("zgemm_dmma_kernel");
+}
 
-void launch_zgemm(const GemmCall& g, cudaStream_t stream) {
-  if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return;
+void launch_several(const Group& g, int count, cudaStream_t stream) {
+  constexpr int smem = Cfg<32>::SMEM_BYTES;
+  qtx_opt_in_smem((const void*)zgemm_group_kernel, smem);
+  int64_t tiles = 0, batch = 0;
+  for (int q = 0; q < count; ++q) {
+    tiles = std::max(tiles, tiles_of<32>(g.p[q]) / g.p[q].batch);
+    batch = std::max(batch, g.p[q].batch);
+  }
+  qtx_launch(zgemm_group_kernel, dim3((unsigned)tiles, count, (unsigned)std::min<int64_t>(batch, 65535)), THREADS,
+             smem, stream, g);
+  qtx_check_launch("zgemm_group_kernel");
+}
+
+Params params_of(const GemmCall& g) {
   Params p;
   p.m = g.m; p.n = g.n; p.k = g.k; p.batch = g.batch;
   p.a = g.a.ptr; p.lda = g.a.ld; p.sa = g.a.stride;
@@ -301,9 +352,42 @@ void launch_zgemm(const GemmCall& g, cudaStream_t stream) {
   p.d = g.d.ptr; p.ldd = g.d.ld; p.sd = g.d.stride; p.alpha = g.alpha;
   p.active = g.active;
   p.diag_shift = g.diag_shift;
-  if (g.op_a == OP_N && g.op_b == OP_N) launch_op<OP_N, OP_N>(p, stream);
-  else if (g.op_a == OP_N && g.op_b == OP_C) launch_op<OP_N, OP_C>(p, stream);
-  else if (g.op_a == OP_C && g.op_b == OP_N) launch_op<OP_C, OP_N>(p, stream);
-  else launch_op<OP_C, OP_C>(p, stream);
-  qtx_check_launch("zgemm_dmma_kernel");
+  p.op_a = g.op_a;
+  p.op_b = g.op_b;
+  return p;
+}
+
+}  // namespace
+
+// Products of up to GROUP_WAVES waves of 32x32 tiles share a launch.  A product
+// of less than one wave costs its latency whatever runs beside it; the group
+// kernel itself is about 2 us slower than the one-product kernel (it looks its
+// operands up in the parameter array), so products that fill the GPU for many
+// waves keep their own launches.
+constexpr int GROUP_WAVES = 4;
+
+void launch_zgemm_group(const GemmCall* calls, int count, cudaStream_t stream) {
+  Group g;
+  int n = 0;
+  auto flush = [&]() {
+    if (n == 1) launch_one(g.p[0], stream);
+    else if (n > 1) launch_several(g, n, stream);
+    n = 0;
+  };
+  for (int q = 0; q < count; ++q) {
+    if (calls[q].m <= 0 || calls[q].n <= 0 || calls[q].batch <= 0) continue;
+    const Params p = params_of(calls[q]);
+    if (waves<32>(tiles_of<32>(p)) > GROUP_WAVES) {
+      launch_one(p, stream);
+      continue;
+    }
+    g.p[n++] = p;
+    if (n == ZGEMM_GROUP_MAX) flush();
+  }
+  flush();
+}
+
+void launch_zgemm(const GemmCall& g, cudaStream_t stream) {
+  if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return;
+  launch_one(params_of(g), stream);
 }

@@ -267,6 +267,44 @@ def test_host_buffer_streaming_equals_device_path(max_batch_size):
     assert isinstance(x_h.data, np.ndarray)
     assert np.array_equal(x_h.data, x_d.data.cpu().numpy())
 
+@pytest.mark.parametrize("scatter", [False, True], ids=["ballistic", "scattering"])
+@pytest.mark.parametrize("sizes", [[48] * 4, [33, 65, 40, 64], [100] * 3])
+def test_selected_solve_does_not_depend_on_the_batch(sizes, scatter):
+    """A few energies run their products grouped in one launch, many run each
+    on its own (and on the wide tile): every energy of a large stack equals its
+    own single-energy call bit for bit, retarded off-diagonals aside."""
+    rng = np.random.default_rng(sum(sizes))
+    ne, nb = 160, len(sizes)
+
+    def cr(*shape):
+        return rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+
+    d = [cr(ne, b, b) + 4 * np.sqrt(b) * np.eye(b) for b in sizes]
+    u = [cr(ne, p, q) for p, q in zip(sizes, sizes[1:])]
+    lo = [cr(ne, q, p) for p, q in zip(sizes, sizes[1:])]
+    s = [1j * (x @ x.conj().swapaxes(-1, -2)) for x in d]
+    su = [cr(ne, p, q) for p, q in zip(sizes, sizes[1:])]
+    if not scatter:
+        s = [s[0]] + [np.zeros_like(x) for x in s[1:]]
+        su = [np.zeros_like(x) for x in su]
+    sl = [-x.conj().swapaxes(-1, -2) for x in su]
+
+    def solve(sel, current):
+        cut = [[x[sel] for x in part] for part in (d, u, lo)]
+        a = DSDBCOO.from_blocks(*cut, device="cuda")
+        sig = DSDBCOO.from_blocks([x[sel] for x in s], [x[sel] for x in su], [x[sel] for x in sl], device="cuda")
+        return RGF(max_batch_size=1000).selected_solve(a, sig, sig, return_retarded=True, return_current=current)
+
+    for current in (False, True):
+        big = solve(slice(0, ne), current)
+        for e in (0, ne - 1):
+            one = solve(slice(e, e + 1), current)
+            for q in range(3):
+                assert torch.equal(one[q].data[0], big[q].data[e]), q
+            if current:
+                # (the trace over a block is one CTA per energy in either case)
+                assert torch.equal(one[3][0], big[3][e])
+
 
 def test_coulomb_screening_call_pattern():
     """The second upstream caller of the same solver, CoulombScreeningSolver.solve
