@@ -567,6 +567,91 @@ void launch_trace_product_h(int rows, int cols, int64_t batch, MatView x, MatVie
 }
 
 
+namespace {
+
+// The elementwise end of one decimation step of the unconverged entries:
+// eps -= t, eps_s -= t (t = a inv b), the convergence measure
+// delta = || |alpha| + |beta| ||_F / 2 of the new alpha and beta, and from it
+// the entry's flags; the last entry to finish stores the number still active
+// in mapped host memory.  grid.x CTAs share a matrix: their partial sums are
+// added in a fixed order by the one that finishes last, so delta does not
+// depend on the schedule.  `count` (batch + 2 words: CTAs done per entry,
+// entries done, entries active) and every flag are left as the next step
+// needs them.  Bound by HBM (7 passes over n^2 elements); with one CTA per
+// matrix the norm alone took 243 us at b = 512, 24 matrices, where the data
+// streams in 0.1 ms.
+constexpr int SRS_THREADS = 256, SRS_ELEMS = 2048, SRS_MAX_CHUNKS = 64;
+__global__ void __launch_bounds__(SRS_THREADS)
+    sr_step_kernel(int nn, int64_t batch, const cplx* alpha, const cplx* beta, const cplx* t, cplx* eps, cplx* eps_s,
+                   double tol, int* active, int* iterations, double* part, unsigned* count, int* mapped_out) {
+  qtx_grid_dependency();
+  const int chunks = gridDim.x;
+  const int per = (nn + chunks - 1) / chunks;
+  const int q0 = blockIdx.x * per, q1 = min(nn, q0 + per);
+  for (int64_t e = blockIdx.y; e < batch; e += gridDim.y) {
+    bool last = false;  // thread 0: this CTA finished entry e
+    if (active[e]) {
+      const int64_t o = e * nn;
+      double acc = 0.0;
+      for (int q = q0 + threadIdx.x; q < q1; q += SRS_THREADS) {
+        const cplx v = t[o + q];
+        eps[o + q] = csub(eps[o + q], v);
+        eps_s[o + q] = csub(eps_s[o + q], v);
+        acc += sr_norm_term(alpha[o + q], beta[o + q]);
+      }
+      const cplx s = block_sum(cmk(acc, 0));
+      if (threadIdx.x == 0) {
+        part[e * chunks + blockIdx.x] = s.x;
+        __threadfence();
+        if (atomicAdd(&count[e], 1u) == (unsigned)chunks - 1) {
+          __threadfence();
+          double total = 0.0;
+          for (int c = 0; c < chunks; ++c) total += ((volatile double*)part)[e * chunks + c];
+          count[e] = 0;
+          iterations[e] += 1;
+          if (sqrt(total) / 2.0 < tol) active[e] = 0;
+          else atomicAdd(&count[batch + 1], 1u);
+          last = true;
+        }
+      }
+    } else if (threadIdx.x == 0 && blockIdx.x == 0) {
+      last = true;
+    }
+    if (last) {
+      __threadfence();
+      if (atomicAdd(&count[batch], 1u) == (unsigned)batch - 1) {
+        __threadfence();
+        *(volatile int*)(mapped_out + 2) = (int)((volatile unsigned*)count)[batch + 1];
+        count[batch] = 0;
+        count[batch + 1] = 0;
+        __threadfence_system();
+      }
+    }
+    __syncthreads();
+  }
+}
+
+int sr_step_chunks(int n) {
+  return std::max(1, std::min(SRS_MAX_CHUNKS, (n * n + SRS_ELEMS - 1) / SRS_ELEMS));
+}
+
+}  // namespace
+
+size_t sr_step_scratch_bytes(int n, int64_t batch) {
+  return sizeof(double) * (size_t)batch * sr_step_chunks(n) + sizeof(unsigned) * (size_t)(batch + 2);
+}
+
+void launch_sr_step(int n, int64_t batch, const cplx* alpha, const cplx* beta, const cplx* t, cplx* eps, cplx* eps_s,
+                    double tol, int* active, int* iterations, void* scratch, int* mapped_out, cudaStream_t stream) {
+  const int chunks = sr_step_chunks(n);
+  double* part = static_cast<double*>(scratch);
+  unsigned* count = reinterpret_cast<unsigned*>(part + (size_t)batch * chunks);
+  const dim3 grid(chunks, (unsigned)std::min<int64_t>(batch, 65535));
+  qtx_launch(sr_step_kernel, grid, SRS_THREADS, 0, stream, n * n, batch, alpha, beta, t, eps, eps_s, tol, active,
+             iterations, part, count, mapped_out);
+  qtx_check_launch("sr_step_kernel");
+}
+
 void launch_sr_norm_update(int n, int64_t batch, MatView alpha, MatView beta, double tol, int* active,
                            int* iterations, int* num_active, cudaStream_t stream) {
   unsigned g = (unsigned)(batch < 65535 ? batch : 65535);

@@ -94,6 +94,14 @@ void launch_trace_product_h(int rows, int cols, int64_t batch, MatView x, MatVie
 // active[e] = active[e] && delta >= tol; iterations[e] += active-before.
 void launch_sr_norm_update(int n, int64_t batch, MatView alpha, MatView beta, double tol, int* active,
                            int* iterations, int* num_active, cudaStream_t stream);
+// End of a decimation step on contiguous n x n matrices, for entries with
+// active[e]: eps -= t, eps_s -= t, iterations[e] += 1, delta as above of the new
+// alpha and beta, active[e] = delta >= tol.  mapped_out[2] (device alias of
+// mapped host memory) receives the number still active.  scratch:
+// sr_step_scratch_bytes, its words zeroed once before the first step.
+size_t sr_step_scratch_bytes(int n, int64_t batch);
+void launch_sr_step(int n, int64_t batch, const cplx* alpha, const cplx* beta, const cplx* t, cplx* eps, cplx* eps_s,
+                    double tol, int* active, int* iterations, void* scratch, int* mapped_out, cudaStream_t stream);
 // A_ii(E) = (E + i eta) I - H  for energies[batch]; out (batch, n, n).
 void launch_assemble_diag(int n, int64_t batch, const cplx* h, const double* energies, double eta, MutView out,
                           cudaStream_t stream);

@@ -200,6 +200,7 @@ struct qtx_ctx {
   size_t mem_limit = 0;
   int* h_pinned = nullptr;     // pinned host words (process-wide pool)
   int* d_pinned = nullptr;     // their device alias: status words are stored there by a kernel
+  cudaEvent_t step_event[2] = {nullptr, nullptr};  // status words of the last two decimation steps stored
   PinRing* ring = nullptr;     // page-locked staging of the host-buffer mode (process-wide pool)
   bool timing = false;
   std::vector<TimedLaunch> timed;
@@ -922,19 +923,25 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
 // Sancho-Rubio (src/qttools/boundary_conditions/obc/sancho_rubio.py:33-86)
 // ---------------------------------------------------------------------------
 constexpr int SR_TEMPS = 10;  // n x n work matrices per batch entry
+size_t sancho_rubio_bytes(int n, int64_t batch) {
+  return sizeof(cplx) * SR_TEMPS * (size_t)n * n * batch + sr_step_scratch_bytes(n, batch) +
+         sizeof(int) * (3 * (size_t)batch);
+}
 // Returns true when every entry converged.
 bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView a_ij, MatView a_ji, double tol,
                        int max_iter, MutView x, int* iterations, cudaStream_t s) {
   const size_t mat = (size_t)n * n * batch;
-  DevBuf buf(sizeof(cplx) * SR_TEMPS * mat + sizeof(int) * (3 * batch + 2), s);
+  DevBuf buf(sancho_rubio_bytes(n, batch), s);
   cplx* p = buf.as<cplx>();
   auto slot = [&](int q) { return MutView{p + q * mat, n, (int64_t)n * n}; };
   MutView eps = slot(0), eps_s = slot(1), alpha = slot(2), beta = slot(3), inv = slot(4), t0 = slot(5),
           t1 = slot(6), t2 = slot(7), t3 = slot(8), t4 = slot(9);
-  int* active = reinterpret_cast<int*>(p + SR_TEMPS * mat);
+  double* step_scratch = reinterpret_cast<double*>(p + SR_TEMPS * mat);
+  const size_t scratch_words = sr_step_scratch_bytes(n, batch) / sizeof(int);
+  int* active = reinterpret_cast<int*>(step_scratch) + scratch_words;
   int* its = active + batch;
-  int* num_active = its + batch;
-  int* info = num_active + 2;  // zero pivots of the decimation inverses (sticky over the iterations)
+  int* info = its + batch;  // zero pivots of the decimation inverses (sticky over the iterations)
+  launch_fill_int(reinterpret_cast<int*>(step_scratch), (int64_t)scratch_words, 0, s);
   launch_fill_int(info, batch, 0, s);
   launch_axpby(n, n, batch, ONE, a_ii, ZERO, {}, eps, s);
   launch_axpby(n, n, batch, ONE, a_ii, ZERO, {}, eps_s, s);
@@ -942,6 +949,19 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView
   launch_axpby(n, n, batch, ONE, a_ij, ZERO, {}, beta, s);
   launch_fill_int(active, batch, 1, s);
   launch_fill_int(its, batch, 0, s);
+  // The count of unconverged entries of step `it` is read while step it + 1 is
+  // already queued (a round trip to the host between two steps left the GPU
+  // idle for about 10 us; a step of 40 leads of b = 64 takes 60 us).  Entries
+  // that have converged are masked, so the one step queued past the end
+  // changes nothing.
+  for (cudaEvent_t& e : ctx->step_event)
+    if (!e) QTX_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  constexpr int SLOT = 16;  // words between the two status slots
+  auto all_done = [&](int it) {
+    QTX_CUDA_TRY(cudaEventSynchronize(ctx->step_event[it & 1]));
+    volatile int* h = ctx->h_pinned + SLOT * (it & 1);
+    return h[2] == 0;
+  };
   bool converged = false;
   for (int it = 0; it < max_iter; ++it) {
     zinv(n, batch, eps, inv, info, active, s);
@@ -957,17 +977,18 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView
     prod(ONE, t1, beta, t4);          // b inv b
     prod(MONE, t1, alpha, eps, eps);  // eps -= b inv a
     grp.run();
-    launch_axpby(n, n, batch, ONE, eps_s, MONE, t2, eps_s, s, active);  // eps_s -= a inv b
-    launch_axpby(n, n, batch, ONE, eps, MONE, t2, eps, s, active);      // eps -= a inv b
     std::swap(alpha.ptr, t3.ptr);
     std::swap(beta.ptr, t4.ptr);
-    launch_fill_int(num_active, 1, 0, s);
-    launch_sr_norm_update(n, batch, alpha, beta, tol, active, its, num_active, s);
-    if (read_status(ctx, num_active, 1, s).head == 0) {
+    // eps -= a inv b, eps_s -= a inv b, convergence of the new alpha, beta
+    launch_sr_step(n, batch, alpha.ptr, beta.ptr, t2.ptr, eps.ptr, eps_s.ptr, tol, active, its, step_scratch,
+                   ctx->d_pinned + SLOT * (it & 1), s);
+    QTX_CUDA_TRY(cudaEventRecord(ctx->step_event[it & 1], s));
+    if (it > 0 && all_done(it - 1)) {
       converged = true;
       break;
     }
   }
+  if (!converged && max_iter > 0) converged = all_done(max_iter - 1);
   zinv(n, batch, eps_s, x, info, nullptr, s);
   if (iterations) launch_copy_int(iterations, 1, its, 1, batch, s);
   read_info_or_throw(ctx, info, batch, s, "sancho_rubio (decimation block)");
@@ -1816,6 +1837,8 @@ qtx_status qtx_ctx_destroy(qtx_ctx* ctx) {
   }
   if (ctx->capture_stream) cudaStreamDestroy(ctx->capture_stream);
   for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
+  for (cudaEvent_t e : ctx->step_event)
+    if (e) cudaEventDestroy(e);
   pinned_give(ctx->h_pinned);
   ring_give(ctx->ring);
   delete ctx;
@@ -1849,8 +1872,7 @@ int64_t qtx_graph_replays(const qtx_ctx* ctx) { return ctx ? ctx->graph_replays 
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call, int32_t precision) {
   if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
   size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
-  bytes += sizeof(cplx) * SR_TEMPS * (size_t)block_size * block_size * energies_per_call +
-           sizeof(int) * (3 * (size_t)energies_per_call + 2);  // Sancho-Rubio
+  bytes += sancho_rubio_bytes(block_size, energies_per_call);
   if (precision == QTX_PREC_MIXED)
     bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
   bytes += zinv_workspace_bytes(block_size, energies_per_call);

@@ -75,3 +75,28 @@ def test_memoizer_device_tensors():
     x, rel, ab = memo((a_ii, a_ij, a_ji), "left")
     assert isinstance(x, torch.Tensor) and x.is_cuda
     assert float(rel.max()) < 1e-6
+
+
+@pytest.mark.parametrize("b,ne", [(3, 2), (45, 3), (46, 3), (64, 70), (150, 5), (400, 2)])
+def test_sancho_rubio_step_sizes(b, ne):
+    """The decimation with one and with several CTAs per matrix in its
+    elementwise step (2048 elements each, 64 at most): result and iteration
+    counts of every energy against the oracle run energy by energy."""
+    dev = make_device(num_blocks=2, block_size=b, num_energies=ne, seed=b, eta=1e-3)
+    d, u, lo = dev.system_blocks()
+    sr = SanchoRubio(max_iterations=100, convergence_tol=1e-10)
+    x = sr(d[0], u[0], lo[0])
+    for e in range(ne):
+        want, its = orc.sancho_rubio(d[0][e:e + 1], u[0][e:e + 1], lo[0][e:e + 1], 100, 1e-10)
+        # eta = 1e-3 bounds the condition of the decimation blocks by about 1e4
+        assert np.linalg.norm(x[e] - want[0]) / np.linalg.norm(want[0]) < 1e-9
+        assert int(np.max(its)) == int(sr.last_iterations[e])
+
+
+@pytest.mark.parametrize("limit", [1, 2, 5])
+def test_sancho_rubio_stops_at_the_iteration_limit(limit):
+    a_ii, a_ij, a_ji = _lead()
+    sr = SanchoRubio(max_iterations=limit, convergence_tol=1e-12)
+    with pytest.warns(RuntimeWarning):
+        sr(a_ii, a_ij, a_ji)
+    assert (sr.last_iterations == limit).all()
