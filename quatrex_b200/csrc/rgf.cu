@@ -1493,8 +1493,39 @@ struct HostArr {
   char* hw = nullptr;       // writable host base (outputs)
   size_t row_bytes = 0;
   bool in = false, out = false;
+  // The parts of a row that the call writes (byte offset, length), ascending.
+  // Only these come back, so the rest of the caller's array keeps its values
+  // and the output need not be uploaded first.  Many or small parts come back
+  // as whole rows instead, which are then uploaded too (`whole`).
+  std::vector<std::pair<size_t, size_t>> parts;
+  bool whole = false;
   char* dev[2] = {nullptr, nullptr};
+  bool uploads() const { return in || (out && whole); }
+  const char* src() const { return out ? hw : h; }
 };
+
+// Parts of an output row of layout d: the diagonal, upper and lower blocks that
+// are written.  A copy of one part per row chunk pays from about 16 KB on.
+void set_parts(HostArr& a, const qtx_btd_desc* d, bool diag, bool upper, bool lower) {
+  const int nb = d->num_blocks;
+  std::vector<std::pair<size_t, size_t>> p;
+  for (int i = 0; i < nb; ++i)
+    for (int j = std::max(0, i - 1); j <= std::min(nb - 1, i + 1); ++j) {
+      const int k = bidx(i, j);
+      if (!(i == j ? diag : (j > i ? upper : lower)) || d->block_offset[k] < 0 || d->block_nnz[k] == 0) continue;
+      p.push_back({sizeof(cplx) * (size_t)d->block_offset[k], sizeof(cplx) * (size_t)d->block_nnz[k]});
+    }
+  std::sort(p.begin(), p.end());
+  size_t bytes = 0;
+  for (const auto& x : p) {
+    bytes += x.second;
+    if (!a.parts.empty() && a.parts.back().first + a.parts.back().second == x.first) a.parts.back().second += x.second;
+    else a.parts.push_back(x);
+  }
+  constexpr size_t MIN_PART = 16u << 10;
+  a.whole = a.parts.size() > 1 && bytes < MIN_PART * a.parts.size();
+  if (a.whole) a.parts.assign(1, {0, a.row_bytes});
+}
 
 // Energies per streamed batch: two staging sets plus the solver's work space
 // (about (3 nb + 32) bmax^2 complex per energy) in 70 % of the free memory.
@@ -1516,29 +1547,33 @@ struct RingCopier {
   PinRing& R;
   cudaStream_t cs;
   int next = 0;
-  struct Pending {
+  struct Pending {  // rows of len bytes, packed in the slot, pitch apart in host memory
     int slot;
     char* host;
-    size_t len;
+    size_t len, pitch;
+    int64_t rows;
   };
   std::deque<Pending> pending;
 
-  static void memcpy_mt(char* dst, const char* src, size_t n) {
+  // n bytes over a few host threads: fn(offset, length) of each one's share, cut at multiples of `unit`
+  template <typename F>
+  static void split_mt(size_t n, size_t unit, F fn) {
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const size_t nt = std::min<size_t>({8, (size_t)std::max(1u, hw / 2), n / (4u << 20) + 1});
     if (nt <= 1) {
-      memcpy(dst, src, n);
+      fn((size_t)0, n);
       return;
     }
     std::vector<std::thread> th;
-    const size_t part = (n + nt - 1) / nt;
-    for (size_t t = 0; t < nt; ++t) {
-      const size_t off = t * part;
-      if (off >= n) break;
+    const size_t part = ((n + nt - 1) / nt + unit - 1) / unit * unit;
+    for (size_t off = 0; off < n; off += part) {
       const size_t len = std::min(part, n - off);
-      th.emplace_back([=] { memcpy(dst + off, src + off, len); });
+      th.emplace_back([=] { fn(off, len); });
     }
     for (auto& x : th) x.join();
+  }
+  static void memcpy_mt(char* dst, const char* src, size_t n) {
+    split_mt(n, 1, [=](size_t off, size_t len) { memcpy(dst + off, src + off, len); });
   }
   int take_slot() {
     const int sl = next;
@@ -1561,18 +1596,43 @@ struct RingCopier {
   void download(char* host, const char* dev, size_t n) {
     for (size_t off = 0; off < n; off += PinRing::kSlotBytes) {
       const size_t len = std::min(PinRing::kSlotBytes, n - off);
-      if ((int)pending.size() >= PinRing::kSlots - 1) drain_one();
-      const int sl = take_slot();
+      const int sl = next_download_slot();
       QTX_CUDA_TRY(cudaMemcpyAsync(R.slot(sl), dev + off, len, cudaMemcpyDeviceToHost, cs));
       QTX_CUDA_TRY(cudaEventRecord(R.ev[sl], cs));
-      pending.push_back({sl, host + off, len});
+      pending.push_back({sl, host + off, len, len, 1});
     }
+  }
+  // `len` bytes of each of `rows` rows, pitch bytes apart on both sides
+  void download_rows(char* host, const char* dev, size_t pitch, size_t len, int64_t rows) {
+    if (len > PinRing::kSlotBytes) {
+      for (int64_t r = 0; r < rows; ++r) download(host + r * pitch, dev + r * pitch, len);
+      return;
+    }
+    const int64_t per = std::max<int64_t>(1, PinRing::kSlotBytes / len);
+    for (int64_t r = 0; r < rows; r += per) {
+      const int64_t nr = std::min(per, rows - r);
+      const int sl = next_download_slot();
+      QTX_CUDA_TRY(cudaMemcpy2DAsync(R.slot(sl), len, dev + r * pitch, pitch, len, nr, cudaMemcpyDeviceToHost, cs));
+      QTX_CUDA_TRY(cudaEventRecord(R.ev[sl], cs));
+      pending.push_back({sl, host + r * pitch, len, pitch, nr});
+    }
+  }
+  int next_download_slot() {
+    if ((int)pending.size() >= PinRing::kSlots - 1) drain_one();
+    return take_slot();
   }
   void drain_one() {
     Pending p = pending.front();
     pending.pop_front();
     QTX_CUDA_TRY(cudaEventSynchronize(R.ev[p.slot]));
-    memcpy_mt(p.host, R.slot(p.slot), p.len);
+    const char* from = R.slot(p.slot);
+    if (p.rows == 1) {
+      memcpy_mt(p.host, from, p.len);
+      return;
+    }
+    split_mt(p.len * p.rows, p.len, [=](size_t off, size_t len) {
+      for (size_t o = off; o < off + len; o += p.len) memcpy(p.host + o / p.len * p.pitch, from + o, p.len);
+    });
   }
   void drain_all() {
     while (!pending.empty()) drain_one();
@@ -1636,8 +1696,7 @@ struct CopyWorker {
 };
 
 // Streams `solve(e0, ne, set)` over the stack.  `arrs` are the per-energy
-// arrays (inputs copied up, outputs copied down; outputs are also copied up so
-// that entries the solver does not write keep their values).  With the
+// arrays (inputs copied up, the written parts of the outputs copied down).  With the
 // context's PinRing, a copy thread uploads batch q + 1 and downloads batch
 // q - 1 through page-locked slots while the solver runs batch q; without one
 // (page-locked memory refused) the copies go straight from the pageable arrays.
@@ -1682,14 +1741,18 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
       auto upload = [&](int64_t e0, int64_t ne, int set) {
         return w.post([&, e0, ne, set] {
           for (auto& a : arrs)
-            if (a.in || a.out) rc.upload(a.dev[set], (a.out ? a.hw : a.h) + e0 * a.row_bytes, ne * a.row_bytes);
+            if (a.uploads()) rc.upload(a.dev[set], a.src() + e0 * a.row_bytes, ne * a.row_bytes);
           QTX_CUDA_TRY(cudaEventRecord(up[set], cs));
         });
       };
       auto download = [&](int64_t e0, int64_t ne, int set) {
         return w.post([&, e0, ne, set] {
           for (auto& a : arrs)
-            if (a.out) rc.download(a.hw + e0 * a.row_bytes, a.dev[set], ne * a.row_bytes);
+            for (const auto& part : a.parts) {
+              char* host = a.hw + e0 * a.row_bytes + part.first;
+              if (part.second == a.row_bytes) rc.download(host, a.dev[set], ne * a.row_bytes);
+              else rc.download_rows(host, a.dev[set] + part.first, a.row_bytes, part.second, ne);
+            }
           rc.drain_all();
         });
       };
@@ -1710,8 +1773,8 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
     } else {
       auto upload = [&](int64_t e0, int64_t ne, int set) {
         for (auto& a : arrs)
-          if (a.in || a.out)
-            QTX_CUDA_TRY(cudaMemcpyAsync(a.dev[set], (a.out ? a.hw : a.h) + e0 * a.row_bytes, ne * a.row_bytes,
+          if (a.uploads())
+            QTX_CUDA_TRY(cudaMemcpyAsync(a.dev[set], a.src() + e0 * a.row_bytes, ne * a.row_bytes,
                                          cudaMemcpyHostToDevice, cs));
         QTX_CUDA_TRY(cudaEventRecord(up[set], cs));
       };
@@ -1725,9 +1788,9 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
         QTX_CUDA_TRY(cudaEventRecord(solved, s));
         QTX_CUDA_TRY(cudaStreamWaitEvent(cs, solved, 0));
         for (auto& a : arrs)
-          if (a.out)
-            QTX_CUDA_TRY(cudaMemcpyAsync(a.hw + e0 * a.row_bytes, a.dev[set], ne * a.row_bytes,
-                                         cudaMemcpyDeviceToHost, cs));
+          for (const auto& part : a.parts)
+            QTX_CUDA_TRY(cudaMemcpy2DAsync(a.hw + e0 * a.row_bytes + part.first, a.row_bytes, a.dev[set] + part.first,
+                                           a.row_bytes, part.second, ne, cudaMemcpyDeviceToHost, cs));
       }
     }
     QTX_CUDA_TRY(cudaStreamSynchronize(cs));
@@ -1958,6 +2021,7 @@ qtx_status qtx_selected_inv(qtx_ctx* ctx, const qtx_btd_desc* a_desc, const void
       arrs[1].hw = reinterpret_cast<char*>(out);
       arrs[1].row_bytes = desc_row_bytes(out_desc);
       arrs[1].out = true;
+      set_parts(arrs[1], out_desc, true, true, true);
       std::vector<int> obc_i;
       add_obc_arrays(arrs, obc_retarded, a_desc, obc_i);
       size_t per_e = 0;
@@ -2029,14 +2093,22 @@ qtx_status qtx_selected_solve(qtx_ctx* ctx, const qtx_btd_desc* a_desc, const vo
       add(a_desc, a, false);
       add(sl_desc, sigma_lesser, false);
       add(sg_desc, sigma_greater, false);
+      const bool lower = (flags & QTX_FLAG_SYMMETRIC_OUT) == 0;
       add(xl_desc, xl, true);
+      set_parts(arrs.back(), xl_desc, true, true, lower);
       add(xg_desc, xg, true);
-      if (want_xr) add(xr_desc, xr, true);
+      set_parts(arrs.back(), xg_desc, true, true, lower);
+      if (want_xr) {
+        const bool off = (flags & QTX_FLAG_RETARDED_OFFDIAG) != 0;
+        add(xr_desc, xr, true);
+        set_parts(arrs.back(), xr_desc, (flags & QTX_FLAG_RETURN_RETARDED) != 0, off, off);
+      }
       if (want_cur) {
         HostArr h;
         h.hw = reinterpret_cast<char*>(current);
         h.row_bytes = sizeof(cplx) * (size_t)(nb - 1);
         h.out = true;
+        if (nb > 1) h.parts.push_back({0, h.row_bytes});
         arrs.push_back(h);
       }
       const size_t first_obc = arrs.size();

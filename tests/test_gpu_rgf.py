@@ -306,6 +306,26 @@ def test_selected_solve_does_not_depend_on_the_batch(sizes, scatter):
                 assert torch.equal(one[3][0], big[3][e])
 
 
+@pytest.mark.parametrize("b", [4, 40])
+def test_host_outputs_come_back_in_the_written_parts(b):
+    """Host outputs are not uploaded: the written blocks come back by parts
+    (blocks of at least 16 KB) or by whole rows (smaller ones), and what the
+    call does not write keeps its values."""
+    dev = make_device(num_blocks=6, block_size=b, num_energies=5, seed=3)
+    _, _, _, _, Ah, Zh, ob = _transport_inputs(dev, device=None)
+    _, _, _, _, Ad, Zd, _ = _transport_inputs(dev, device="cuda")
+    outs_h = [DSDBCOO.zeros_like(Ah) for _ in range(3)]
+    outs_d = [DSDBCOO.zeros_like(Ad) for _ in range(3)]
+    for x in outs_h + outs_d:
+        x.data[...] = -2.0 + 5.0j
+    solver = RGF(max_batch_size=2)
+    solver.selected_solve(Ah, Zh, Zh, obc_blocks=ob, out=outs_h, return_retarded=True)
+    solver.selected_solve(Ad, Zd, Zd, obc_blocks=ob, out=outs_d, return_retarded=True)
+    for h, x in zip(outs_h, outs_d):
+        assert np.array_equal(h.data, x.data.cpu().numpy())
+    assert np.all(outs_h[2].blocks[2, 3] == -2.0 + 5.0j)
+
+
 def test_coulomb_screening_call_pattern():
     """The second upstream caller of the same solver, CoulombScreeningSolver.solve
     (src/quatrex/coulomb_screening/solver.py:466-489): out=(W^<, W^>) of length
