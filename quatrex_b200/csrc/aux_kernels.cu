@@ -136,31 +136,37 @@ __global__ void axpby_kernel(int rows, int cols, int64_t batch, cplx alpha, cons
   }
 }
 
-// scatter dense block -> data slice; mode 0 copy, 1 0.5(X - X^H), 2 -X^H
-// (mode 2: the stored block is cols_out x rows_out = the transpose shape of x;
-// `rows`/`cols` are the shape of the STORED block)
-__global__ void block_scatter_kernel(int rows, int cols, int64_t batch, const cplx* x, int64_t ldx, int64_t sx,
-                                     int mode, cplx* data, int64_t stride, int64_t nnz, const int32_t* index) {
+// The blocks one step of a recursion stores, grid.y picks the block, grid.z the
+// batch entry (see launch_block_scatter for the modes; `rows` / `cols` are the
+// shape of the STORED block).  A block of a small batch is a few microseconds of
+// latency, so the blocks of a step share a launch; 32-bit index arithmetic
+// within a block.
+struct ScatterGroup {
+  ScatterCall c[SCATTER_GROUP_MAX];
+};
+__global__ void __launch_bounds__(TB) block_scatter_kernel(const __grid_constant__ ScatterGroup g, int64_t batch) {
   qtx_grid_dependency();
-  const int64_t total = batch * nnz;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t e = t / nnz;
-    int64_t q = t % nnz;
-    int lin = index ? index[q] : (int)q;
-    int r = lin / cols, c = lin % cols;
-    const cplx* xb = x + e * sx;
-    cplx v;
-    if (mode == 0) {
-      v = xb[(int64_t)r * ldx + c];
-    } else if (mode == 1) {
-      cplx a = xb[(int64_t)r * ldx + c];
-      cplx b = xb[(int64_t)c * ldx + r];
-      v = cmk(0.5 * (a.x - b.x), 0.5 * (a.y + b.y));
-    } else {
-      cplx b = xb[(int64_t)c * ldx + r];
-      v = cmk(-b.x, b.y);
+  const ScatterCall& s = g.c[blockIdx.y];
+  const int nnz = (int)s.nnz, cols = s.cols, mode = s.mode;
+  const int64_t ldx = s.x.ld;
+  for (int64_t e = blockIdx.z; e < batch; e += gridDim.z) {
+    const cplx* xb = s.x.ptr + e * s.x.stride;
+    cplx* out = s.data + e * s.stride;
+    for (int q = blockIdx.x * TB + threadIdx.x; q < nnz; q += gridDim.x * TB) {
+      const int lin = s.index ? s.index[q] : q;
+      const int r = lin / cols, c = lin % cols;
+      cplx v;
+      if (mode == 0) {
+        v = xb[r * ldx + c];
+      } else if (mode == 1) {
+        const cplx a = xb[r * ldx + c], b = xb[c * ldx + r];
+        v = cmk(0.5 * (a.x - b.x), 0.5 * (a.y + b.y));
+      } else {
+        const cplx b = xb[c * ldx + r];
+        v = cmk(-b.x, b.y);
+      }
+      out[q] = v;
     }
-    data[e * stride + q] = v;
   }
 }
 
@@ -532,14 +538,21 @@ void launch_energy_shift(int64_t batch, const double* energies, double eta, cplx
   qtx_check_launch("energy_shift_kernel");
 }
 
-void launch_block_scatter(int rows, int cols, int64_t batch, MatView x, int mode, cplx* data, int64_t stride,
-                          int64_t nnz, const int32_t* index, cudaStream_t stream) {
-  if (nnz <= 0) return;
-  qtx_launch(block_scatter_kernel, grid_for(batch * nnz), TB, 0, stream, rows, cols, batch, x.ptr, x.ld, x.stride,
-             mode, data, stride, nnz, index);
-  qtx_check_launch("block_scatter_kernel");
+void launch_block_scatter_group(const ScatterCall* calls, int count, int64_t batch, cudaStream_t stream) {
+  ScatterGroup g;
+  for (int q0 = 0; q0 < count; q0 += SCATTER_GROUP_MAX) {
+    const int n = std::min(SCATTER_GROUP_MAX, count - q0);
+    int64_t nnz = 0;
+    for (int q = 0; q < n; ++q) {
+      g.c[q] = calls[q0 + q];
+      nnz = std::max(nnz, g.c[q].nnz);
+    }
+    if (nnz <= 0 || batch <= 0) continue;
+    const dim3 grid(ceil_div_u(nnz, TB), n, (unsigned)std::min<int64_t>(batch, 65535));
+    qtx_launch(block_scatter_kernel, grid, TB, 0, stream, g, batch);
+    qtx_check_launch("block_scatter_kernel");
+  }
 }
-
 void launch_block_gather(int rows, int cols, int64_t batch, const cplx* data, int64_t stride, int64_t nnz,
                          const int32_t* index, MutView out, cudaStream_t stream) {
   qtx_launch(block_gather_kernel, grid_for(batch * (int64_t)rows * cols), TB, 0, stream, rows, cols, batch, data,

@@ -78,8 +78,17 @@ void launch_energy_shift(int64_t batch, const double* energies, double eta, cplx
 // data slice (entry q of the block at data[e * stride + q], local index
 // index[q] = r * cols + c, or row-major dense when index == nullptr).
 // mode: 0 = copy, 1 = 0.5 (X - X^H) (square), 2 = -X^H (out is cols x rows of x^H)
-void launch_block_scatter(int rows, int cols, int64_t batch, MatView x, int mode, cplx* data, int64_t stride,
-                          int64_t nnz, const int32_t* index, cudaStream_t stream);
+struct ScatterCall {
+  int rows = 0, cols = 0, mode = 0;
+  MatView x;
+  cplx* data = nullptr;
+  int64_t stride = 0, nnz = 0;
+  const int32_t* index = nullptr;
+};
+constexpr int SCATTER_GROUP_MAX = 8;
+// Several blocks of one batch (SCATTER_GROUP_MAX per launch); no block may be
+// another one's source.
+void launch_block_scatter_group(const ScatterCall* calls, int count, int64_t batch, cudaStream_t stream);
 void launch_block_gather(int rows, int cols, int64_t batch, const cplx* data, int64_t stride, int64_t nnz,
                          const int32_t* index, MutView out, cudaStream_t stream);
 

@@ -388,14 +388,32 @@ MatView in_block(const Btd& m, int i, int j, int64_t e0, int64_t ne, cplx* scrat
   return out;
 }
 
-// Store x (rows x cols of block (i, j), or its source for modes 1/2) into block (i, j).
-void out_block(const Btd& m, int i, int j, int64_t e0, int64_t ne, MatView x, int mode, const Workspace& ws) {
-  if (!m.data) return;
-  int k = bidx(i, j);
-  if (m.empty(k)) return;
-  cplx* base = m.data + e0 * m.d->stack_stride + m.off(k);
-  launch_block_scatter(m.size(i), m.size(j), ne, x, mode, base, m.d->stack_stride, m.nnz(k), m.index(k), ws.s);
-}
+// Blocks to store, in one launch.
+struct ScatterList {
+  const Workspace& ws;
+  int64_t e0, ne;
+  std::vector<ScatterCall> calls;
+  // x (rows x cols of block (i, j), or its source for modes 1/2) into block (i, j)
+  void add(const Btd& m, int i, int j, MatView x, int mode) {
+    if (!m.data) return;
+    const int k = bidx(i, j);
+    if (m.empty(k)) return;
+    ScatterCall c;
+    c.rows = m.size(i);
+    c.cols = m.size(j);
+    c.mode = mode;
+    c.x = x;
+    c.data = m.data + e0 * m.d->stack_stride + m.off(k);
+    c.stride = m.d->stack_stride;
+    c.nnz = m.nnz(k);
+    c.index = m.index(k);
+    calls.push_back(c);
+  }
+  void run() {
+    launch_block_scatter_group(calls.data(), (int)calls.size(), ne, ws.s);
+    calls.clear();
+  }
+};
 
 // OBC block view (contiguous (stack, b, b)), or null view
 MatView obc_view(const void* const* arr, int i, int b, int64_t e0) {
@@ -574,7 +592,9 @@ void selected_inv_impl(qtx_ctx* ctx, const Btd& a, const void* const* obc_r, con
            precision);
       zinv(bj, ne, tv(1, bj), x.view(j), info + (int64_t)j * ne_max, nullptr, s);
     }
-    out_block(out, nb - 1, nb - 1, e0, ne, x.view(nb - 1), 0, ws);
+    ScatterList store{ws, e0, ne, {}};
+    store.add(out, nb - 1, nb - 1, x.view(nb - 1), 0);
+    store.run();
     // backward
     for (int i = nb - 2; i >= 0; --i) {
       const int j = i + 1, bi = sizes[i], bj = sizes[j];
@@ -588,13 +608,14 @@ void selected_inv_impl(qtx_ctx* ctx, const Btd& a, const void* const* obc_r, con
       grp.add(gemm_call(bj, bi, bi, ne, MONE, tv(0, bi), OP_N, x.view(i), OP_N, tv(1, bi)));
       grp.add(gemm_call(bi, bj, bj, ne, MONE, tv(2, bj), OP_N, x.view(j), OP_N, tv(3, bj)));
       grp.run();
-      out_block(out, j, i, e0, ne, tv(1, bi), 0, ws);
-      out_block(out, i, j, e0, ne, tv(3, bj), 0, ws);
+      store.add(out, j, i, tv(1, bi), 0);
+      store.add(out, i, j, tv(3, bj), 0);
       // X_ii = x_i - (x_i A_ij) X_ji
       gemm(bi, bi, bj, ne, MONE, tv(2, bj), OP_N, tv(1, bi), OP_N, tv(4, bi), s, x.view(i), ONE, {}, ZERO, nullptr,
            nullptr, precision);
       std::swap(x.ptr[i], T[4]);
-      out_block(out, i, i, e0, ne, x.view(i), 0, ws);
+      store.add(out, i, i, x.view(i), 0);
+      store.run();
     }
   }
   read_info_or_throw(ctx, info, ne_max * nb, s, "selected_inv");
@@ -840,11 +861,13 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
     for (const GemmCall& g : pend) grp.add(g);
     grp.run();
     // ---- last diagonal blocks (rgf.py:297-305)
+    ScatterList store{ws, e0, ne, {}};
     {
       const int n = nb - 1;
-      out_block(A.xl, n, n, e0, ne, xl.view(n), 1, ws);
-      out_block(A.xg, n, n, e0, ne, xg.view(n), 1, ws);
-      if (want_r) out_block(A.xr, n, n, e0, ne, xr.view(n), 0, ws);
+      store.add(A.xl, n, n, xl.view(n), 1);
+      store.add(A.xg, n, n, xg.view(n), 1);
+      if (want_r) store.add(A.xr, n, n, xr.view(n), 0);
+      store.run();
     }
     // ---- backward sweep (rgf.py:307-404).  Work matrices: P1 0, P2 1, P3 10,
     // P4 11, the new x_i 12, of component c Y, t1, t2, X_ij from 2 + 4 c on.
@@ -874,10 +897,12 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       if (want_r_off) {
         // X^R_ij = -P3 ; X^R_ji = -P2 x_i
         launch_axpby(bi, bj, ne, MONE, p3, ZERO, {}, tv(12, bj), s);
-        out_block(A.xr, i, j, e0, ne, tv(12, bj), 0, ws);
+        store.add(A.xr, i, j, tv(12, bj), 0);
+        store.run();
         grp.add(call(bj, bi, bi, MONE, p2, OP_N, xr.view(i), OP_N, tv(12, bi)));
         grp.run();
-        out_block(A.xr, j, i, e0, ne, tv(12, bi), 0, ws);
+        store.add(A.xr, j, i, tv(12, bi), 0);
+        store.run();
       }
       // t1 = P4 X_i - Y P3^H ; X_ij = Y X_jj^H - t2 - X_i P2^H ; G_ii = x_i + P4 x_i
       for (int c = 0; c < 2; ++c) {
@@ -895,13 +920,15 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       grp.run();
       for (int c = 0; c < 2; ++c) {
         launch_sub_herm_inplace(bi, ne, t1(c), s);
-        out_block(*Oc[c], i, j, e0, ne, xij(c), 0, ws);
-        if (!symmetric) out_block(*Oc[c], j, i, e0, ne, xij(c), 2, ws);
         // X_i += t2 P1^H + t1
         grp.add(call(bi, bi, bj, ONE, t2(c), OP_N, p1, OP_C, Xc[c]->view(i), Xc[c]->view(i), ONE, t1(c), ONE));
       }
       grp.run();
-      for (int c = 0; c < 2; ++c) out_block(*Oc[c], i, i, e0, ne, Xc[c]->view(i), 1, ws);
+      for (int c = 0; c < 2; ++c) {
+        store.add(*Oc[c], i, j, xij(c), 0);
+        if (!symmetric) store.add(*Oc[c], j, i, xij(c), 2);
+        store.add(*Oc[c], i, i, Xc[c]->view(i), 1);
+      }
       if (want_cur) {
         // current_i = Tr[Sigma~^>_i X^<_j - X^>_j Sigma~^<_i]
         cplx* cur_out = T[11];
@@ -912,7 +939,8 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
                      s);
       }
       std::swap(xr.ptr[i], T[12]);
-      if (want_r) out_block(A.xr, i, i, e0, ne, xr.view(i), 0, ws);
+      if (want_r) store.add(A.xr, i, i, xr.view(i), 0);
+      store.run();
     }
   }
   read_info_or_throw(ctx, info, ne_max * nb, s, "selected_solve");
