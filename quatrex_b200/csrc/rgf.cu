@@ -530,11 +530,14 @@ StatusRead read_status(qtx_ctx* ctx, const int* d, int64_t n, cudaStream_t s) {
   return StatusRead{h[0], h[1], h[2]};
 }
 
+[[noreturn]] void throw_singular(const char* what, int64_t entry, int pivot) {
+  throw QtxError(QTX_E_SINGULAR, std::string(what) + ": exactly singular diagonal block (stack entry " +
+                                     std::to_string(entry) + ", pivot " + std::to_string(pivot) + ")");
+}
+
 void read_info_or_throw(qtx_ctx* ctx, const int* d_info, int64_t n, cudaStream_t s, const char* what) {
   const StatusRead r = read_status(ctx, d_info, n, s);
-  if (r.first)
-    throw QtxError(QTX_E_SINGULAR, std::string(what) + ": exactly singular diagonal block (stack entry " +
-                                       std::to_string(r.first - 1) + ", pivot " + std::to_string(r.value) + ")");
+  if (r.first) throw_singular(what, r.first - 1, r.value);
 }
 
 // ---------------------------------------------------------------------------
@@ -955,13 +958,27 @@ size_t sancho_rubio_bytes(int n, int64_t batch) {
   return sizeof(cplx) * SR_TEMPS * (size_t)n * n * batch + sr_step_scratch_bytes(n, batch) +
          sizeof(int) * (3 * (size_t)batch);
 }
-// Returns true when every entry converged.
-bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView a_ij, MatView a_ji, double tol,
-                       int max_iter, MutView x, int* iterations, cudaStream_t s) {
-  const size_t mat = (size_t)n * n * batch;
+// One lead of a decimation call: `batch` energies, the surface function into x
+// (contiguous matrices), the iteration counts into iterations (optional).
+struct Lead {
+  MatView a_ii, a_ij, a_ji;
+  int64_t batch = 0;
+  MutView x;
+  int* iterations = nullptr;
+  int64_t iterations_stride = 1;
+};
+
+// Decimates all leads together, as one batch.  Returns true when every entry
+// converged.
+bool sancho_rubio_impl(qtx_ctx* ctx, int n, const std::vector<Lead>& leads, double tol, int max_iter,
+                       cudaStream_t s) {
+  int64_t batch = 0;
+  for (const Lead& l : leads) batch += l.batch;
+  const int64_t nn = (int64_t)n * n;
+  const size_t mat = (size_t)nn * batch;
   DevBuf buf(sancho_rubio_bytes(n, batch), s);
   cplx* p = buf.as<cplx>();
-  auto slot = [&](int q) { return MutView{p + q * mat, n, (int64_t)n * n}; };
+  auto slot = [&](int q) { return MutView{p + q * mat, n, nn}; };
   MutView eps = slot(0), eps_s = slot(1), alpha = slot(2), beta = slot(3), inv = slot(4), t0 = slot(5),
           t1 = slot(6), t2 = slot(7), t3 = slot(8), t4 = slot(9);
   double* step_scratch = reinterpret_cast<double*>(p + SR_TEMPS * mat);
@@ -971,10 +988,15 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView
   int* info = its + batch;  // zero pivots of the decimation inverses (sticky over the iterations)
   launch_fill_int(reinterpret_cast<int*>(step_scratch), (int64_t)scratch_words, 0, s);
   launch_fill_int(info, batch, 0, s);
-  launch_axpby(n, n, batch, ONE, a_ii, ZERO, {}, eps, s);
-  launch_axpby(n, n, batch, ONE, a_ii, ZERO, {}, eps_s, s);
-  launch_axpby(n, n, batch, ONE, a_ji, ZERO, {}, alpha, s);
-  launch_axpby(n, n, batch, ONE, a_ij, ZERO, {}, beta, s);
+  int64_t at = 0;
+  for (const Lead& l : leads) {
+    auto part = [&](MutView v) { return MutView{v.ptr + at * nn, n, nn}; };
+    launch_axpby(n, n, l.batch, ONE, l.a_ii, ZERO, {}, part(eps), s);
+    launch_axpby(n, n, l.batch, ONE, l.a_ii, ZERO, {}, part(eps_s), s);
+    launch_axpby(n, n, l.batch, ONE, l.a_ji, ZERO, {}, part(alpha), s);
+    launch_axpby(n, n, l.batch, ONE, l.a_ij, ZERO, {}, part(beta), s);
+    at += l.batch;
+  }
   launch_fill_int(active, batch, 1, s);
   launch_fill_int(its, batch, 0, s);
   // The count of unconverged entries of step `it` is read while step it + 1 is
@@ -1017,9 +1039,30 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, int64_t batch, MatView a_ii, MatView
     }
   }
   if (!converged && max_iter > 0) converged = all_done(max_iter - 1);
-  zinv(n, batch, eps_s, x, info, nullptr, s);
-  if (iterations) launch_copy_int(iterations, 1, its, 1, batch, s);
-  read_info_or_throw(ctx, info, batch, s, "sancho_rubio (decimation block)");
+  at = 0;
+  for (size_t q = 0; q < leads.size();) {
+    // one call for the leads whose results follow one another in memory
+    int64_t count = leads[q].batch;
+    size_t next = q + 1;
+    while (next < leads.size() && leads[next].x.ptr == leads[q].x.ptr + count * nn) count += leads[next++].batch;
+    zinv(n, count, MutView{eps_s.ptr + at * nn, n, nn}, leads[q].x, info + at, nullptr, s);
+    at += count;
+    q = next;
+  }
+  at = 0;
+  for (const Lead& l : leads) {
+    if (l.iterations) launch_copy_int(l.iterations, l.iterations_stride, its + at, 1, l.batch, s);
+    at += l.batch;
+  }
+  const StatusRead st = read_status(ctx, info, batch, s);
+  if (st.first) {
+    int64_t e = st.first - 1;
+    for (const Lead& l : leads) {
+      if (e < l.batch) break;
+      e -= l.batch;
+    }
+    throw_singular("sancho_rubio (decimation block)", e, st.value);
+  }
   return converged;
 }
 
@@ -1087,6 +1130,13 @@ void transport_couplings(const TransportWS& w, const cplx* h_upper, cudaStream_t
   }
 }
 
+// Both leads of a batch decimate as one where a single lead leaves SMs idle:
+// the elimination of a panel takes one CTA, so one SM, per matrix (b > 64), the
+// register inverse two CTAs per SM (b <= 64).  Above that the two in turn need
+// half the work space.  Transport on B200, together / in turn: nb = 16, b = 64,
+// 32 energies 4.70 / 6.23 ms; nb = 8, b = 512, 24 energies 333 / 354 ms.
+bool leads_together(int b, int64_t ne) { return ne <= (b <= 64 ? 148 : 74); }
+
 // Contacts of energies [e0, e0 + ne) (src/quatrex/electron/solver.py:305-386):
 // Sancho-Rubio on both leads (host-synchronising convergence checks), then
 // Sigma^R, Gamma, Sigma^<, Sigma^> and the (E + i eta) shifts, all into `w`.
@@ -1100,26 +1150,40 @@ bool transport_contacts(qtx_ctx* ctx, const TransportWS& w, const qtx_transport_
   auto V = [&](cplx* p) { return MutView{p, b, bb}; };
   const double* en = P.energies + e0;
   launch_energy_shift(ne, en, P.eta, w.shift, s);
-  // left: g_L = SR(A_00, A_01, A_10)
-  launch_assemble_diag(b, ne, h_diag, en, P.eta, V(w.T[0]), s);
-  bool okl = sancho_rubio_impl(ctx, b, ne, V(w.T[0]), up(0), lo(0), P.sr_tol, P.sr_max_iterations, V(w.C[0]), w.its,
-                               s);
-  if (O.sr_iterations) launch_copy_int(O.sr_iterations + 2 * e0, 2, w.its, 1, ne, s);
-  // right: g_R = SR(A_nn, A_nm, A_mn)
-  launch_assemble_diag(b, ne, h_diag + (int64_t)(nb - 1) * bb, en, P.eta, V(w.T[0]), s);
-  bool okr = sancho_rubio_impl(ctx, b, ne, V(w.T[0]), lo(nb - 2), up(nb - 2), P.sr_tol, P.sr_max_iterations,
-                               V(w.C[1]), w.its, s);
-  if (O.sr_iterations) launch_copy_int(O.sr_iterations + 2 * e0 + 1, 2, w.its, 1, ne, s);
+  // left: g_L = SR(A_00, A_01, A_10), right: g_R = SR(A_nn, A_nm, A_mn)
+  Lead lead[2];
+  for (int c = 0; c < 2; ++c) {
+    const MutView a_ii = V(w.T[c]);
+    launch_assemble_diag(b, ne, h_diag + (c == 0 ? 0 : (int64_t)(nb - 1) * bb), en, P.eta, a_ii, s);
+    lead[c].a_ii = a_ii;
+    lead[c].a_ij = c == 0 ? up(0) : lo(nb - 2);
+    lead[c].a_ji = c == 0 ? lo(0) : up(nb - 2);
+    lead[c].batch = ne;
+    lead[c].x = V(w.C[c]);
+    if (O.sr_iterations) {
+      lead[c].iterations = O.sr_iterations + 2 * e0 + c;
+      lead[c].iterations_stride = 2;
+    }
+  }
+  bool ok = true;
+  if (leads_together(b, ne)) {
+    ok = sancho_rubio_impl(ctx, b, {lead[0], lead[1]}, P.sr_tol, P.sr_max_iterations, s);
+  } else {
+    for (const Lead& l : lead) ok = sancho_rubio_impl(ctx, b, {l}, P.sr_tol, P.sr_max_iterations, s) && ok;
+  }
   // Sigma^R_L = A_10 g_L A_01 ; Sigma^R_R = A_mn g_R A_nm
-  gemm(b, b, b, ne, ONE, lo(0), OP_N, V(w.C[0]), OP_N, V(w.T[1]), s);
-  gemm(b, b, b, ne, ONE, V(w.T[1]), OP_N, up(0), OP_N, V(w.C[2]), s);
-  gemm(b, b, b, ne, ONE, up(nb - 2), OP_N, V(w.C[1]), OP_N, V(w.T[1]), s);
-  gemm(b, b, b, ne, ONE, V(w.T[1]), OP_N, lo(nb - 2), OP_N, V(w.C[3]), s);
+  GemmGroup grp(s);
+  for (int c = 0; c < 2; ++c)
+    grp.add(gemm_call(b, b, b, ne, ONE, lead[c].a_ji, OP_N, V(w.C[c]), OP_N, V(w.T[2 + c])));
+  grp.run();
+  for (int c = 0; c < 2; ++c)
+    grp.add(gemm_call(b, b, b, ne, ONE, V(w.T[2 + c]), OP_N, lead[c].a_ij, OP_N, V(w.C[2 + c])));
+  grp.run();
   launch_fermi(ne, en, P.mu_left, P.kt, w.occ_l, s);
   launch_fermi(ne, en, P.mu_right, P.kt, w.occ_r, s);
   launch_obc_lesser_greater(b, ne, V(w.C[2]), w.occ_l, V(w.C[4]), V(w.C[6]), V(w.C[8]), s);
   launch_obc_lesser_greater(b, ne, V(w.C[3]), w.occ_r, V(w.C[5]), V(w.C[7]), V(w.C[9]), s);
-  return okl && okr;
+  return ok;
 }
 
 // Selected solve and observables of energies [e0, e0 + ne) once the contacts
@@ -1963,7 +2027,7 @@ int64_t qtx_graph_replays(const qtx_ctx* ctx) { return ctx ? ctx->graph_replays 
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call, int32_t precision) {
   if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
   size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
-  bytes += sancho_rubio_bytes(block_size, energies_per_call);
+  bytes += sancho_rubio_bytes(block_size, (leads_together(block_size, energies_per_call) ? 2 : 1) * energies_per_call);
   if (precision == QTX_PREC_MIXED)
     bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
   bytes += zinv_workspace_bytes(block_size, energies_per_call);
@@ -2201,10 +2265,14 @@ qtx_status qtx_sancho_rubio(qtx_ctx* ctx, int32_t n, int64_t batch, const void* 
       throw QtxError(QTX_E_INVAL, "qtx_sancho_rubio: bad arguments");
     if (batch == 0) return;  // an empty energy batch: nothing to decimate
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    ok = sancho_rubio_impl(ctx, n, batch, MatView{reinterpret_cast<const cplx*>(a_ii), n, stride_ii},
-                           MatView{reinterpret_cast<const cplx*>(a_ij), n, stride_ij},
-                           MatView{reinterpret_cast<const cplx*>(a_ji), n, stride_ji}, convergence_tol,
-                           max_iterations, MutView{reinterpret_cast<cplx*>(x), n, (int64_t)n * n}, iterations, s);
+    Lead lead;
+    lead.a_ii = MatView{reinterpret_cast<const cplx*>(a_ii), n, stride_ii};
+    lead.a_ij = MatView{reinterpret_cast<const cplx*>(a_ij), n, stride_ij};
+    lead.a_ji = MatView{reinterpret_cast<const cplx*>(a_ji), n, stride_ji};
+    lead.batch = batch;
+    lead.x = MutView{reinterpret_cast<cplx*>(x), n, (int64_t)n * n};
+    lead.iterations = iterations;
+    ok = sancho_rubio_impl(ctx, n, {lead}, convergence_tol, max_iterations, s);
     QTX_CUDA_TRY(cudaStreamSynchronize(s));
   });
   if (st == QTX_OK && !ok) {

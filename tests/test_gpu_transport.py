@@ -147,3 +147,15 @@ def test_transport_ballistic_transmission_matches_current():
     # interface currents of the selected solve in tests/test_oracle.py)
     lay = out["layer_current"].cpu().numpy()
     assert np.allclose(lay, lay[:, :1], rtol=1e-2, atol=1e-9 * np.abs(lay).max())
+
+
+@pytest.mark.parametrize("b,ne,batch", [(24, 160, 40), (96, 80, 20)])
+def test_leads_decimated_together_or_in_turn(b, ne, batch):
+    """Both leads of a small energy batch decimate as one batch, those of a
+    large one in turn; energies are independent, so every output of every
+    energy is the same bit for bit, iteration counts included."""
+    dev = make_device(num_blocks=3, block_size=b, num_energies=ne, seed=b, eta=1e-4)
+    in_turn = TransportSolver(dev, max_batch_size=ne).solve(dev.energies)
+    together = TransportSolver(dev, max_batch_size=batch).solve(dev.energies)
+    for k in in_turn:
+        assert torch.equal(in_turn[k], together[k]), k
