@@ -4,6 +4,10 @@ against the oracle.  Tolerances: relative Frobenius error 1e-12 for a single
 GEMM, 1e-10 for inverses of well-conditioned blocks."""
 
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -150,6 +154,32 @@ def test_inverse_of_tied_pivots(n):
     want = np.stack([h.T / n, h.T / (n * scale[None, :])])
     # orthogonal up to scale (condition number 1), growth factor n
     assert _rel(x, want) < 4 * n * 2.0**-53
+
+
+_ONE_LAUNCH = """
+import numpy as np, torch
+from quatrex_b200 import _lib
+lib, ctx = _lib.load(), _lib.context(0)
+for n, batch in ((65, 3), (100, 3), (128, 3), (129, 3), (256, 150), (257, 2), (512, 2)):
+    assert lib.qtx_transport_footprint(4, n, 4, 0) > 0
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
+    a[:, np.arange(n), np.arange(n)] += np.sqrt(n)
+    t = torch.from_numpy(a[:, np.roll(np.arange(n), n // 3)].copy()).cuda()
+    x = torch.empty_like(t)
+    _lib.check(lib.qtx_inv(ctx, n, batch, t.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
+    want = torch.linalg.inv(t)
+    err = float(torch.linalg.vector_norm(x - want) / torch.linalg.vector_norm(want))
+    assert err < 4 * n * 2.0**-53 * float(torch.linalg.cond(t).max()), (n, err)
+"""
+
+
+def test_one_launch_inverse_without_scratch():
+    """The form that takes no scratch (QTX_INV_SPLIT_BELOW=0, read once per
+    process): every shape of its panel elimination."""
+    env = dict(os.environ, QTX_INV_SPLIT_BELOW="0")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", _ONE_LAUNCH], check=True, env=env, cwd=root, timeout=300)
 
 
 @pytest.mark.parametrize("n", [96, 200, 256, 300])
