@@ -521,13 +521,12 @@ BlockStack carve(cplx*& cursor, const std::vector<int>& sizes, int64_t ne, int b
 struct StatusRead {
   int first;  // 1 + index of the first nonzero entry, 0 if none
   int value;  // that entry
-  int head;   // entry 0
 };
 StatusRead read_status(qtx_ctx* ctx, const int* d, int64_t n, cudaStream_t s) {
   launch_flag_reduce(d, n, ctx->d_pinned, s);
   QTX_CUDA_TRY(cudaStreamSynchronize(s));
   volatile int* h = ctx->h_pinned;
-  return StatusRead{h[0], h[1], h[2]};
+  return StatusRead{h[0], h[1]};
 }
 
 [[noreturn]] void throw_singular(const char* what, int64_t entry, int pivot) {
@@ -1132,9 +1131,11 @@ void transport_couplings(const TransportWS& w, const cplx* h_upper, cudaStream_t
 
 // Both leads of a batch decimate as one where a single lead leaves SMs idle:
 // the elimination of a panel takes one CTA, so one SM, per matrix (b > 64), the
-// register inverse two CTAs per SM (b <= 64).  Above that the two in turn need
-// half the work space.  Transport on B200, together / in turn: nb = 16, b = 64,
-// 32 energies 4.70 / 6.23 ms; nb = 8, b = 512, 24 energies 333 / 354 ms.
+// register inverse two CTAs per SM (b <= 64).  Above that the gain shrinks and
+// the two in turn need half the work space.  Two-block transport on B200,
+// together / in turn, ms: b = 64, 74 energies 3.29 / 4.70, 148 5.10 / 6.24, 296
+// 9.66 / 10.01; b = 128, 74 15.3 / 18.7, 148 29.98 / 30.12; b = 256, 37 50.8 /
+// 57.8, 74 92.6 / 100.2, 148 181.7 / 182.9.
 bool leads_together(int b, int64_t ne) { return ne <= (b <= 64 ? 148 : 74); }
 
 // Contacts of energies [e0, e0 + ne) (src/quatrex/electron/solver.py:305-386):
@@ -2027,7 +2028,8 @@ int64_t qtx_graph_replays(const qtx_ctx* ctx) { return ctx ? ctx->graph_replays 
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call, int32_t precision) {
   if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
   size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
-  bytes += sancho_rubio_bytes(block_size, (leads_together(block_size, energies_per_call) ? 2 : 1) * energies_per_call);
+  const int leads = leads_together(block_size, energies_per_call) ? 2 : 1;
+  bytes += sancho_rubio_bytes(block_size, leads * energies_per_call);
   if (precision == QTX_PREC_MIXED)
     bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
   bytes += zinv_workspace_bytes(block_size, energies_per_call);

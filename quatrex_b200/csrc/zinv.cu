@@ -1050,8 +1050,9 @@ void launch_regs(int n, int64_t batch, MatView a, MutView x, int* info, const in
 
 // QTX_INV_SPLIT_BELOW sends batches of that many matrices or more of n > 64 to
 // the one-launch kernel (0: all of them), which takes no scratch.  The two-launch
-// panels are the faster form at every batch measured (b = 256: 1.31 against 1.65 ms for 148 matrices, 0.54 against 1.72 for 16), so by default
-// all batches take them.
+// panels are the faster form at every batch measured (b = 256: 1.31 against 1.65
+// ms for 148 matrices, 0.54 against 1.72 for 16), so by default all batches take
+// them.
 int64_t split_below() {
   static const int64_t v = [] {
     const char* e = getenv("QTX_INV_SPLIT_BELOW");
