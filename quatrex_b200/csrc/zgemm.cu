@@ -11,7 +11,7 @@
 //   32x32, warp tile 16x16, four CTAs per SM (40 KB each)
 // Bound by the DMMA pipe (87-90 % active in either form where the tiles fill
 // whole waves), so the choice is the one with the shorter last wave: see
-// launch_zgemm.  Per output element both run the same DMMA sequence, so the
+// wide_tile().  Per output element both run the same DMMA sequence, so the
 // result does not depend on the tile.
 //
 // Tried and not kept: three real products instead of four (Gauss's identity,

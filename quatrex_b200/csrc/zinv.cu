@@ -663,9 +663,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 
 // ---------------------------------------------------------------------------
 // Blocks of up to 64: the whole matrix in registers (gj_regs.cuh), one CTA per
-// matrix, four threads per row (four warps up to 32 rows, eight up to 64).  The row and column permutations are applied on the store:
-// the row-swapping elimination would hold row p_k at position k, so with pos(r)
-// the step at which row r was the pivot, X[pos(r)][p_c] = M[r][c].
+// matrix, four threads per row (four warps up to 32 rows, eight up to 64).  The
+// row and column permutations are applied on the store: the row-swapping
+// elimination would hold row p_k at position k, so with pos(r) the step at which
+// row r was the pivot, X[pos(r)][p_c] = M[r][c].
 // Bound by the chain of n dependent steps: about 1100 cycles each at 32 rows,
 // 1700 at 64.  Measured on B200, us per call with its status read: b = 32, 8
 // matrices 44 (66 with the blocked kernel), b = 64, 32 matrices 89 (147).
@@ -1082,8 +1083,8 @@ void launch_split(int n, int64_t batch, MatView a, MutView x, void* scratch, int
 
   for (int k0 = 0; k0 < n; k0 += W) {
     const int w = std::min(W, n - k0);
-    qtx_launch(zinv_panel_kernel<TPR, CPT, NW>, gb, 32 * NW, psmem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr, x.ld,
-               x.stride, k0, sc, info, active);
+    qtx_launch(zinv_panel_kernel<TPR, CPT, NW>, gb, 32 * NW, psmem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr,
+               x.ld, x.stride, k0, sc, info, active);
     // the first update reads A itself, so an out-of-place call needs no copy
     const MatView from = k0 == 0 ? a : MatView(x);
     qtx_launch(zinv_update_kernel, dim3(nslab, gb), UPD_THREADS, usmem, stream, n, batch, from.ptr, from.ld,
