@@ -156,28 +156,121 @@ __device__ inline GjSmem gj_smem_layout(unsigned char* base, int n, int wp, int 
   return s;
 }
 
+// Eliminates a panel of at most CPT columns and of up to RPT * THREADS rows
+// that the threads of the CTA hold RPT rows each (row r0 + q * THREADS in
+// reg[q]): the steps of gj_eliminate for more rows than threads.  Column kk of the
+// register rows is picked by selects.  24 matrices of n = 512 take 11.3 ms; 12.0
+// with all columns unrolled and static, 12.8 with one update formula for the
+// pivot row and the others on top, as in gj_eliminate (registers).
+template <int RPT, int CPT>
+__device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, int k0, int w, int WP,
+                                                  const GjSmem& sm, int& zero_pivot) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  bool used[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) used[q] = tid + q * THREADS < k0;  // the pivots of earlier panels
+  // One barrier per column: every warp publishes the panel row of its own
+  // best candidate before the barrier, so afterwards the winner's row is read
+  // directly.
+#pragma unroll 32
+  for (int kk = 0; kk < w; ++kk) {
+    // each row reads and clears its column-kk entry: the staged pivot row
+    // carries 1 there, so the update below is one x - fd p for every entry
+    // (-fd at column kk) and p d for the pivot row (d at kk)
+    cplx colv[RPT];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      cplx v = cmk(0, 0);
+#pragma unroll
+      for (int j = 0; j < CPT; ++j)
+        if (j == kk) {
+          v = reg[q][j];
+          reg[q][j] = cmk(0, 0);
+        }
+      colv[q] = v;
+    }
+    // A NaN entry counts as infinite: every candidate is then above the -1 of
+    // the rows that are none, and the same row is found by all lanes.
+    double bv = -1.0;
+    int bi = n;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int r = tid + q * THREADS;
+      if (r < n && !used[q]) argmax_combine(bv, bi, fmin(cabs1(colv[q]), (double)INFINITY), r);
+    }
+    // butterfly: every lane ends with the warp's best candidate
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
+      const int i2 = __shfl_xor_sync(0xffffffffu, bi, off);
+      argmax_combine(bv, bi, v2, i2);
+    }
+    const int slot = (kk & 1) * NWARPS;
+    cplx* my_cand = sm.cand + (size_t)(slot + warp) * WP;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+      if (tid + q * THREADS == bi) {
+#pragma unroll
+        for (int j = 0; j < CPT; ++j)
+          if (j < w) my_cand[j] = reg[q][j];
+        my_cand[kk] = cmk(1, 0);
+        sm.red_piv[slot + warp] = colv[q];
+      }
+    if (lane == 0) {
+      sm.red_v[slot + warp] = bv;
+      sm.red_i[slot + warp] = bi;
+    }
+    __syncthreads();  // candidates of every warp visible
+    // best over the warps: every group of NWARPS lanes holds all candidates
+    double v = sm.red_v[slot + lane % NWARPS];
+    int p = sm.red_i[slot + lane % NWARPS];
+#pragma unroll
+    for (int off = NWARPS / 2; off > 0; off >>= 1) {
+      const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
+      const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
+      argmax_combine(v, p, v2, i2);
+    }
+    const int pw = (p % THREADS) >> 5;  // the warp that holds row p published it
+    const cplx* prow = sm.cand + (size_t)(slot + pw) * WP;
+    const cplx piv = sm.red_piv[slot + pw];
+    if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k0 + kk + 1;
+    const cplx d = crecip_pivot(piv);
+    if (tid == 0) sm.pivs[kk] = p;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int r = tid + q * THREADS;
+      if (r >= n) continue;
+      if (r == p) {
+        used[q] = true;
+#pragma unroll
+        for (int j = 0; j < CPT; ++j)
+          if (j < w) reg[q][j] = cmul(prow[j], d);
+      } else {
+        const cplx fd = cmul(colv[q], d);
+#pragma unroll
+        for (int j = 0; j < CPT; ++j)
+          if (j < w) reg[q][j] = cfms(fd, prow[j], reg[q][j]);
+      }
+    }
+  }
+}
+
 // Steps 1 and 2 for the panel [k0, k0 + w) of X (rows in the current order):
-// eliminate it in shared memory / registers, turn its pivots into the row
-// permutation sigma (pos2row / row2pos, relative to the current order) and
-// the swaps perm[k0 .. k0 + w), and leave the eliminated panel in P (rows in
-// the current order).  Ends with a CTA barrier.
+// eliminate it in registers, turn its pivots into the row permutation sigma
+// (pos2row / row2pos, relative to the current order) and the swaps
+// perm[k0 .. k0 + w), and leave the eliminated panel in P (rows in the current
+// order).  TPR threads a row of CPT columns each, or (TPR = 1) RPT rows a
+// thread.  Ends with a CTA barrier.
 template <int TPR, int RPT, int CPT>
 __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cplx* X, int64_t ldx, const GjSmem& sm,
                                          int& zero_pivot) {
+  static_assert(TPR == 1 || RPT == 1, "several rows a thread: whole rows");
   cplx* P = sm.P;
   int* pos2row = sm.pos2row;
   int* row2pos = sm.row2pos;
   int* perm = sm.perm;
   int* pivs = sm.pivs;
-  double* red_v = sm.red_v;
-  cplx* red_piv = sm.red_piv;
-  int* red_i = sm.red_i;
-  cplx* cand = sm.cand;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // elimination ownership: thread -> (rows r0 + q * rstride, columns cl + j * TPR)
-  const int rstride = THREADS / TPR;
-  const int r_own = tid / TPR;
-  const int c_own = tid % TPR;
+  const int tid = threadIdx.x;
     // ---- 1. stage the panel (rows in the current order of X), every
     // element in flight at once (asynchronous copies)
     for (int idx = tid; idx < n * w; idx += THREADS) {
@@ -193,9 +286,8 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
     __syncthreads();
 
     // The thread's panel entries live in registers during the elimination:
-    // reg[q][j] = P[r_own + q * rstride][c_own + j * TPR].  The column factor
-    // of a row comes from the lane of the row's group that holds column kk;
-    // the pivot row is broadcast through shared memory.
+    // reg[q][j] = P[r_own + q * rstride][c_own + j * TPR].
+    const int rstride = THREADS / TPR, r_own = tid / TPR, c_own = tid % TPR;
     cplx reg[RPT][CPT];
 #pragma unroll
     for (int q = 0; q < RPT; ++q)
@@ -204,197 +296,15 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
         const int r = r_own + q * rstride, c = c_own + j * TPR;
         reg[q][j] = (r < n && c < w) ? P[pidx(r, c, WP)] : cmk(0, 0);
       }
-    const int grp0 = lane - c_own;  // first lane of this row's group (groups never straddle warps)
     // rows before k0 are the pivots of earlier panels (rows are in the new order now)
-    if constexpr (TPR == 1 && RPT == 1 && CPT == 32) {
-      // Register rotation: at step kk, reg[0][j] holds panel column
-      // (kk + j) mod 32, so the step's column is always reg[0][0] (no
-      // selects over the row) and every update is unpredicated (columns
-      // at or beyond w stay zero: the published pivot rows carry zeros
-      // there).  The same pivots and the same update of every non-pivot
-      // row as the generic loop.
-      bool used = r_own < k0;
-      auto rotate = [&]() {
-        const cplx t0 = reg[0][0];
-#pragma unroll
-        for (int j = 0; j < 31; ++j) reg[0][j] = reg[0][j + 1];
-        reg[0][31] = t0;
-      };
-#pragma unroll 1
-      for (int kk = 0; kk < w; ++kk) {
-        const int k = k0 + kk;
-        const cplx colv = reg[0][0];
-        reg[0][0] = cmk(0, 0);
-        double bv = -1.0;
-        int bi = n;
-        if (r_own < n && !used) {
-          bv = cabs1(colv);
-          bi = r_own;
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-          int i2 = __shfl_xor_sync(0xffffffffu, bi, off);
-          argmax_combine(bv, bi, v2, i2);
-        }
-        const int par = kk & 1;
-        cplx* my_cand = cand + (size_t)(par * NWARPS + warp) * WP;
-        const int slot = par * NWARPS;
-        if (r_own == bi) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) my_cand[j] = reg[0][j];
-          my_cand[0] = cmk(1, 0);
-          red_piv[slot + warp] = colv;
-        }
-        if (lane == 0) {
-          red_v[slot + warp] = bv;
-          red_i[slot + warp] = bi;
-        }
-        __syncthreads();  // candidates of every warp visible
-        double v = red_v[slot + lane % NWARPS];
-        int p = red_i[slot + lane % NWARPS];
-#pragma unroll
-        for (int off = NWARPS / 2; off > 0; off >>= 1) {
-          const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
-          const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
-          argmax_combine(v, p, v2, i2);
-        }
-        const int pw = p >> 5;  // one row per thread: row p lives in warp p / 32
-        const cplx* prow = cand + (size_t)(par * NWARPS + pw) * WP;
-        const cplx piv = red_piv[slot + pw];
-        if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k + 1;
-        const cplx d = crecip_pivot(piv);
-        if (tid == 0) pivs[kk] = p;
-        if (r_own < n) {
-          // the pivot row as 0 - (-d) p: one update formula for every
-          // row, so the warp holding the pivot row does not run two
-          // branches while the others wait at the next barrier
-          const bool is_p = r_own == p;
-          used = used || is_p;
-          const cplx fd = is_p ? cmk(-d.x, -d.y) : cmul(colv, d);
-          if (is_p) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) reg[0][j] = cmk(0, 0);
-          }
-#pragma unroll
-          for (int j = 0; j < 32; ++j) reg[0][j] = cfms(fd, prow[j], reg[0][j]);
-        }
-        rotate();
-      }
-      for (int extra = w; extra < 32; ++extra) rotate();  // natural column order again
+    int turned = 0;
+    if constexpr (RPT == 1) {
+      __shared__ GjRegs<TPR, CPT, NWARPS> regs;
+      const int zero = gj_eliminate<TPR, CPT, NWARPS>(reg[0], w, r_own, c_own, r_own < k0 || r_own >= n, regs, pivs);
+      if (zero && !zero_pivot) zero_pivot = k0 + zero;
+      turned = w / TPR;
     } else {
-      bool used[RPT];
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) used[q] = r_own + q * rstride < k0;
-      // One barrier per column: every warp publishes the panel row of its own
-      // best candidate before the barrier, so afterwards the winner's row is
-      // read directly.  Column kk of the register rows is picked by static
-      // selects; with 32 register columns the loop stays rolled (one copy of
-      // its body fits the instruction cache), narrower rows unroll it.
-      constexpr int kKUnroll = (CPT >= 2 && CPT <= 16) ? 32 : 1;
-#pragma unroll kKUnroll
-      for (int kk = 0; kk < w; ++kk) {
-        const int k = k0 + kk;
-        // each row reads and clears its column-kk entry: the staged pivot
-        // row carries 1 there, so the update below is one x - fd p for
-        // every entry (-fd at column kk) and p d for the pivot row (d at kk)
-        cplx colv[RPT];
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          cplx v = cmk(0, 0);
-#pragma unroll
-          for (int j = 0; j < CPT; ++j)
-            if (c_own + j * TPR == kk) {
-              v = reg[q][j];
-              reg[q][j] = cmk(0, 0);
-            }
-          colv[q] = v;
-        }
-        // pivot search: the owner of (r, kk) looks at row r if it is not a pivot yet
-        double bv = -1.0;
-        int bi = n;
-        if (c_own == kk % TPR) {
-#pragma unroll
-          for (int q = 0; q < RPT; ++q) {
-            const int r = r_own + q * rstride;
-            if (r < n && !used[q]) argmax_combine(bv, bi, cabs1(colv[q]), r);
-          }
-        }
-        // butterfly: every lane ends with the warp's best candidate
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          double v2 = __shfl_xor_sync(0xffffffffu, bv, off);
-          int i2 = __shfl_xor_sync(0xffffffffu, bi, off);
-          argmax_combine(bv, bi, v2, i2);
-        }
-        // factors of this thread's rows (column kk, from the group's owner lane)
-        cplx f[RPT];
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          const double fx = __shfl_sync(0xffffffffu, colv[q].x, grp0 + kk % TPR);
-          const double fy = __shfl_sync(0xffffffffu, colv[q].y, grp0 + kk % TPR);
-          f[q] = cmk(fx, fy);
-        }
-        const int par = kk & 1;
-        cplx* my_cand = cand + (size_t)(par * NWARPS + warp) * WP;
-        const int slot = par * NWARPS;
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          if (r_own + q * rstride == bi) {
-#pragma unroll
-            for (int j = 0; j < CPT; ++j) {
-              const int c = c_own + j * TPR;
-              if (c < w) my_cand[c] = reg[q][j];
-            }
-            if (c_own == kk % TPR) {
-              my_cand[kk] = cmk(1, 0);
-              red_piv[slot + warp] = colv[q];
-            }
-          }
-        }
-        if (lane == 0) {
-          red_v[slot + warp] = bv;
-          red_i[slot + warp] = bi;
-        }
-        __syncthreads();  // S: candidates of every warp visible
-        // best over the warps, lane-parallel: every group of NWARPS lanes
-        // holds all candidates (same choice as a scan in warp order)
-        double v = red_v[slot + lane % NWARPS];
-        int p = red_i[slot + lane % NWARPS];
-#pragma unroll
-        for (int off = NWARPS / 2; off > 0; off >>= 1) {
-          const double v2 = __shfl_xor_sync(0xffffffffu, v, off);
-          const int i2 = __shfl_xor_sync(0xffffffffu, p, off);
-          argmax_combine(v, p, v2, i2);
-        }
-        // the global best is the best of the warp that owns row p
-        const int pw = ((p % rstride) * TPR) >> 5;
-        const cplx* prow = cand + (size_t)(par * NWARPS + pw) * WP;
-        const cplx piv = red_piv[slot + pw];
-        if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k + 1;
-        const cplx d = crecip_pivot(piv);
-        if (tid == 0) pivs[kk] = p;
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          const int r = r_own + q * rstride;
-          if (r >= n) continue;
-          if (r == p) {
-            used[q] = true;
-#pragma unroll
-            for (int j = 0; j < CPT; ++j) {
-              const int c = c_own + j * TPR;
-              if (c < w) reg[q][j] = cmul(prow[c], d);
-            }
-          } else {
-            const cplx fd = cmul(f[q], d);
-#pragma unroll
-            for (int j = 0; j < CPT; ++j) {
-              const int c = c_own + j * TPR;
-              if (c < w) reg[q][j] = cfms(fd, prow[c], reg[q][j]);
-            }
-          }
-        }
-      }
+      gj_eliminate_rows<RPT, CPT>(reg, n, k0, w, WP, sm, zero_pivot);
     }
     // classic row-swap semantics of the panel's pivots: position k0 + kk
     // receives row pivs[kk], the displaced row goes to the pivot's position
@@ -415,7 +325,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
     for (int q = 0; q < RPT; ++q)
 #pragma unroll
       for (int j = 0; j < CPT; ++j) {
-        const int r = r_own + q * rstride, c = c_own + j * TPR;
+        const int r = r_own + q * rstride, c = ((j + turned) % CPT) * TPR + c_own;
         if (r < n && c < w) P[pidx(r, c, WP)] = reg[q][j];
       }
     __syncthreads();
@@ -1051,8 +961,8 @@ void launch_regs(int n, int64_t batch, MatView a, MutView x, int* info, const in
 
 // QTX_INV_SPLIT_BELOW sends batches of that many matrices or more of n > 64 to
 // the one-launch kernel (0: all of them), which takes no scratch.  The two-launch
-// panels are the faster form at every batch measured (b = 256: 1.31 against 1.65
-// ms for 148 matrices, 0.54 against 1.72 for 16), so by default all batches take
+// panels are the faster form at every batch measured (b = 256: 1.31 against 1.50
+// ms for 148 matrices, 0.54 against 1.26 for 16), so by default all batches take
 // them.
 int64_t split_below() {
   static const int64_t v = [] {
@@ -1132,6 +1042,7 @@ void launch_zinv(int n, int64_t batch, MatView a, MutView x, int* info, const in
   const int cpt = (s.w + s.tpr - 1) / s.tpr;
   if (s.tpr == 1 && rpt == 1 && cpt <= 32) launch_inv_r<1, 1, 32>(n, batch, a, x, info, active, stream);
   else if (s.tpr == 1 && rpt == 2 && cpt <= 16) launch_inv_r<1, 2, 16>(n, batch, a, x, info, active, stream);
+  else if (s.tpr == 2 && rpt == 1 && cpt <= 8) launch_inv_r<2, 1, 8>(n, batch, a, x, info, active, stream);
   else if (s.tpr == 2 && rpt == 1 && cpt <= 16) launch_inv_r<2, 1, 16>(n, batch, a, x, info, active, stream);
   else throw QtxError(QTX_E_UNSUPPORTED, "qtx inverse: block size outside the supported shapes");
   qtx_check_launch("zinv_gj_kernel");

@@ -156,30 +156,68 @@ def test_inverse_of_tied_pivots(n):
     assert _rel(x, want) < 4 * n * 2.0**-53
 
 
-_ONE_LAUNCH = """
-import numpy as np, torch
-from quatrex_b200 import _lib
-lib, ctx = _lib.load(), _lib.context(0)
-for n, batch in ((65, 3), (100, 3), (128, 3), (129, 3), (256, 150), (257, 2), (512, 2)):
-    assert lib.qtx_transport_footprint(4, n, 4, 0) > 0
-    rng = np.random.default_rng(n)
-    a = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
-    a[:, np.arange(n), np.arange(n)] += np.sqrt(n)
-    t = torch.from_numpy(a[:, np.roll(np.arange(n), n // 3)].copy()).cuda()
-    x = torch.empty_like(t)
-    _lib.check(lib.qtx_inv(ctx, n, batch, t.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
-    want = torch.linalg.inv(t)
-    err = float(torch.linalg.vector_norm(x - want) / torch.linalg.vector_norm(want))
-    assert err < 4 * n * 2.0**-53 * float(torch.linalg.cond(t).max()), (n, err)
-"""
+def _one_launch(check):
+    """Run `check` (t is this module) in a process whose inverses take no scratch
+    (QTX_INV_SPLIT_BELOW=0, read once per process)."""
+    env = dict(os.environ, QTX_INV_SPLIT_BELOW="0")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = f"import sys; sys.path[:0] = ['.', 'tests']; import test_gpu_kernels as t; {check}"
+    subprocess.run([sys.executable, "-c", code], check=True, env=env, cwd=root, timeout=300)
+
+
+def _check_one_launch():
+    lib, ctx = _lib.load(), _lib.context(0)
+    for n, batch in ((65, 3), (100, 3), (128, 3), (129, 3), (256, 150), (257, 2), (512, 2)):
+        rng = np.random.default_rng(n)
+        a = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
+        a[:, np.arange(n), np.arange(n)] += np.sqrt(n)
+        t = torch.from_numpy(a[:, np.roll(np.arange(n), n // 3)].copy()).cuda()
+        x = torch.empty_like(t)
+        _lib.check(lib.qtx_inv(ctx, n, batch, t.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
+        want = torch.linalg.inv(t)
+        err = float(torch.linalg.vector_norm(x - want) / torch.linalg.vector_norm(want))
+        assert err < 4 * n * 2.0**-53 * float(torch.linalg.cond(t).max()), (n, err)
 
 
 def test_one_launch_inverse_without_scratch():
-    """The form that takes no scratch (QTX_INV_SPLIT_BELOW=0, read once per
-    process): every shape of its panel elimination."""
-    env = dict(os.environ, QTX_INV_SPLIT_BELOW="0")
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    subprocess.run([sys.executable, "-c", _ONE_LAUNCH], check=True, env=env, cwd=root, timeout=300)
+    """The form that takes no scratch: every shape of its panel elimination."""
+    _one_launch("t._check_one_launch()")
+
+
+def _check_non_finite(n):
+    """A matrix with a column of NaN (every bit set, the sign included), one
+    with a single NaN and one with an infinity between finite ones: the finite
+    ones come out as without them, nothing outside the output is written, and
+    the NaN ones do not come out finite.  A pivot search that lost a NaN row
+    named no row, or a used one, and the permutation then pointed anywhere."""
+    lib, ctx = _lib.load(), _lib.context(0)
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((5, n, n)) + 1j * rng.standard_normal((5, n, n))
+    a[:, np.arange(n), np.arange(n)] += np.sqrt(n)
+    a.view(np.uint64)[1, :, 2 * (n // 2):2 * (n // 2) + 2] = 0xFFFFFFFFFFFFFFFF
+    a[2, n // 3, 0] = complex(np.nan, 1.0)
+    a[3, n - 1, n // 2] = complex(0.0, -np.inf)
+    buf = torch.full((7, n, n), 7.0, dtype=torch.complex128, device="cuda")
+    x = buf[1:6]
+    ta = torch.from_numpy(a).cuda()
+    st = lib.qtx_inv(ctx, n, 5, ta.data_ptr(), n * n, x.data_ptr(), n * n, 0)
+    assert st in (_lib.QTX_OK, _lib.QTX_E_SINGULAR)
+    good = ta[[0, 4]].contiguous()
+    want = torch.empty_like(good)
+    _lib.check(lib.qtx_inv(ctx, n, 2, good.data_ptr(), n * n, want.data_ptr(), n * n, 0), ctx, "inv")
+    assert torch.equal(x[[0, 4]], want)
+    assert bool((buf[[0, 6]] == 7.0).all())
+    for e in (1, 2):  # (an infinity may have a finite inverse: 1 / inf = 0)
+        assert not bool(torch.isfinite(torch.view_as_real(x[e])).all())
+
+
+@pytest.mark.parametrize("n", [1, 5, 32, 33, 64, 65, 97, 128, 129, 256, 257, 384, 385, 512])
+def test_inverse_with_nan_and_inf(n):
+    _check_non_finite(n)
+
+
+def test_one_launch_inverse_with_nan_and_inf():
+    _one_launch("[t._check_non_finite(n) for n in (65, 97, 128, 129, 256, 257, 512)]")
 
 
 @pytest.mark.parametrize("n", [96, 200, 256, 300])
