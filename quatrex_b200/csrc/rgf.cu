@@ -952,7 +952,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Sancho-Rubio (src/qttools/boundary_conditions/obc/sancho_rubio.py:33-86)
 // ---------------------------------------------------------------------------
-constexpr int SR_TEMPS = 10;  // n x n work matrices per batch entry
+constexpr int SR_TEMPS = 9;  // n x n work matrices per batch entry
 size_t sancho_rubio_bytes(int n, int64_t batch) {
   return sizeof(cplx) * SR_TEMPS * (size_t)n * n * batch + sr_step_scratch_bytes(n, batch) +
          sizeof(int) * (3 * (size_t)batch);
@@ -979,7 +979,8 @@ bool sancho_rubio_impl(qtx_ctx* ctx, int n, const std::vector<Lead>& leads, doub
   cplx* p = buf.as<cplx>();
   auto slot = [&](int q) { return MutView{p + q * mat, n, nn}; };
   MutView eps = slot(0), eps_s = slot(1), alpha = slot(2), beta = slot(3), inv = slot(4), t0 = slot(5),
-          t1 = slot(6), t2 = slot(7), t3 = slot(8), t4 = slot(9);
+          t1 = slot(6), t3 = slot(7), t4 = slot(8);
+  const MutView t2 = inv;  // a inv b: the inverse has been used by then, and t2 by the next step's inverse
   double* step_scratch = reinterpret_cast<double*>(p + SR_TEMPS * mat);
   const size_t scratch_words = sr_step_scratch_bytes(n, batch) / sizeof(int);
   int* active = reinterpret_cast<int*>(step_scratch) + scratch_words;

@@ -1,0 +1,59 @@
+"""Device memory that a call takes from the stream-ordered pool: its high-water
+mark against what the call is documented to hold."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from quatrex_b200 import _lib
+from quatrex_b200.workloads import make_device
+
+pytestmark = pytest.mark.gpu
+
+CPLX = 16
+SLACK = 1 << 20  # status words, small tables and the pool's rounding
+
+
+def _pool():
+    cu = ctypes.CDLL("libcuda.so.1")
+    dev = ctypes.c_int()
+    assert cu.cuDeviceGet(ctypes.byref(dev), torch.cuda.current_device()) == 0
+    pool = ctypes.c_void_p()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), dev) == 0
+    return cu, pool
+
+
+def _peak(call):
+    """Bytes of the device's default pool in use at the peak of call(), above
+    what was in use before."""
+    used, high = 7, 8  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT, CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    cu, pool = _pool()
+    torch.cuda.synchronize()
+    v = ctypes.c_uint64(0)
+    assert cu.cuMemPoolSetAttribute(pool, high, ctypes.byref(v)) == 0  # resets the mark
+    before = ctypes.c_uint64()
+    assert cu.cuMemPoolGetAttribute(pool, used, ctypes.byref(before)) == 0
+    call()
+    torch.cuda.synchronize()
+    assert cu.cuMemPoolGetAttribute(pool, high, ctypes.byref(v)) == 0
+    return v.value - before.value
+
+
+@pytest.mark.parametrize("n", [48, 256])
+def test_sancho_rubio_holds_nine_matrices(n):
+    """Nine work matrices per energy, and for n > 64 the inverse's panel scratch."""
+    ne = 24
+    d, u, lo = make_device(num_blocks=2, block_size=n, num_energies=ne, seed=5).system_blocks()
+    a_ii, a_ij, a_ji = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (d[0], u[0], lo[0]))
+    x = torch.empty_like(a_ii)
+    lib, ctx = _lib.load(), _lib.context(0)
+
+    def call():
+        st = lib.qtx_sancho_rubio(ctx, n, ne, a_ii.data_ptr(), n * n, a_ij.data_ptr(), n * n, a_ji.data_ptr(), n * n,
+                                  1e-12, 200, x.data_ptr(), None, 0)
+        _lib.check(st, ctx, "sancho_rubio")
+
+    panels = n * 32 * CPLX * ne if n > 64 else 0
+    assert _peak(call) <= 9 * n * n * CPLX * ne + panels + SLACK
