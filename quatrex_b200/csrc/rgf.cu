@@ -285,6 +285,15 @@ class DevBuf {
     ptr_ = qtx_malloc_async(bytes, s);
     if (!ptr_) throw QtxError(QTX_E_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed");
   }
+  // As above, empty (see operator bool) when the allocation fails.
+  static DevBuf attempt(size_t bytes, cudaStream_t s) {
+    DevBuf b;
+    b.stream_ = s;
+    b.bytes_ = bytes;
+    b.ptr_ = qtx_malloc_async(bytes, s);
+    return b;
+  }
+  explicit operator bool() const { return ptr_ != nullptr; }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   DevBuf(DevBuf&& o) noexcept { *this = std::move(o); }
@@ -967,15 +976,15 @@ struct Lead {
   int64_t iterations_stride = 1;
 };
 
-// Decimates all leads together, as one batch.  Returns true when every entry
+// Decimates all leads together, as one batch, in the work space `buf`
+// (sancho_rubio_bytes of all their entries).  Returns true when every entry
 // converged.
-bool sancho_rubio_impl(qtx_ctx* ctx, int n, const std::vector<Lead>& leads, double tol, int max_iter,
-                       cudaStream_t s) {
+bool sancho_rubio_impl(qtx_ctx* ctx, int n, const std::vector<Lead>& leads, const DevBuf& buf, double tol,
+                       int max_iter, cudaStream_t s) {
   int64_t batch = 0;
   for (const Lead& l : leads) batch += l.batch;
   const int64_t nn = (int64_t)n * n;
   const size_t mat = (size_t)nn * batch;
-  DevBuf buf(sancho_rubio_bytes(n, batch), s);
   cplx* p = buf.as<cplx>();
   auto slot = [&](int q) { return MutView{p + q * mat, n, nn}; };
   MutView eps = slot(0), eps_s = slot(1), alpha = slot(2), beta = slot(3), inv = slot(4), t0 = slot(5),
@@ -1168,10 +1177,14 @@ bool transport_contacts(qtx_ctx* ctx, const TransportWS& w, const qtx_transport_
     }
   }
   bool ok = true;
-  if (leads_together(b, ne)) {
-    ok = sancho_rubio_impl(ctx, b, {lead[0], lead[1]}, P.sr_tol, P.sr_max_iterations, s);
+  DevBuf both;  // where there is no room for both, one after the other
+  if (leads_together(b, ne)) both = DevBuf::attempt(sancho_rubio_bytes(b, 2 * ne), s);
+  if (both) {
+    ok = sancho_rubio_impl(ctx, b, {lead[0], lead[1]}, both, P.sr_tol, P.sr_max_iterations, s);
+    both.release();
   } else {
-    for (const Lead& l : lead) ok = sancho_rubio_impl(ctx, b, {l}, P.sr_tol, P.sr_max_iterations, s) && ok;
+    DevBuf one(sancho_rubio_bytes(b, ne), s);
+    for (const Lead& l : lead) ok = sancho_rubio_impl(ctx, b, {l}, one, P.sr_tol, P.sr_max_iterations, s) && ok;
   }
   // Sigma^R_L = A_10 g_L A_01 ; Sigma^R_R = A_mn g_R A_nm
   GemmGroup grp(s);
@@ -2275,7 +2288,8 @@ qtx_status qtx_sancho_rubio(qtx_ctx* ctx, int32_t n, int64_t batch, const void* 
     lead.batch = batch;
     lead.x = MutView{reinterpret_cast<cplx*>(x), n, (int64_t)n * n};
     lead.iterations = iterations;
-    ok = sancho_rubio_impl(ctx, n, {lead}, convergence_tol, max_iterations, s);
+    DevBuf buf(sancho_rubio_bytes(n, batch), s);
+    ok = sancho_rubio_impl(ctx, n, {lead}, buf, convergence_tol, max_iterations, s);
     QTX_CUDA_TRY(cudaStreamSynchronize(s));
   });
   if (st == QTX_OK && !ok) {

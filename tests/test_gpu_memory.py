@@ -8,11 +8,13 @@ import pytest
 import torch
 
 from quatrex_b200 import _lib
+from quatrex_b200.transport import TransportSolver
 from quatrex_b200.workloads import make_device
 
 pytestmark = pytest.mark.gpu
 
 CPLX = 16
+KEYS = ("density", "transmission", "current_left")
 SLACK = 1 << 20  # status words, small tables and the pool's rounding
 
 
@@ -41,10 +43,10 @@ def _peak(call):
     return v.value - before.value
 
 
-@pytest.mark.parametrize("n", [48, 256])
+@pytest.mark.parametrize("n", [64, 256])
 def test_sancho_rubio_holds_nine_matrices(n):
     """Nine work matrices per energy, and for n > 64 the inverse's panel scratch."""
-    ne = 24
+    ne = 40
     d, u, lo = make_device(num_blocks=2, block_size=n, num_energies=ne, seed=5).system_blocks()
     a_ii, a_ij, a_ji = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (d[0], u[0], lo[0]))
     x = torch.empty_like(a_ii)
@@ -57,3 +59,30 @@ def test_sancho_rubio_holds_nine_matrices(n):
 
     panels = n * 32 * CPLX * ne if n > 64 else 0
     assert _peak(call) <= 9 * n * n * CPLX * ne + panels + SLACK
+
+
+def test_leads_in_turn_where_there_is_no_room_for_both():
+    """A batch whose leads would decimate together (b = 256, 74 energies) with
+    the device filled up to about 1 GB more than the recursion's own work space:
+    both leads need 1.4 GB, one 0.7 GB.  The call goes through, with the result
+    of a call that has all the memory."""
+    nb, b, ne = 2, 256, 74
+    dev = make_device(num_blocks=nb, block_size=b, num_energies=ne, seed=6)
+    solver = TransportSolver(dev, max_batch_size=ne)
+    want = {k: v.clone() for k, v in solver.solve(dev.energies, keys=KEYS).items()}
+    out = solver.allocate_outputs(ne, KEYS)
+    lib, ctx = _lib.load(), _lib.context(0)
+    _lib.check(lib.qtx_ctx_trim(ctx), ctx, "trim")
+    torch.cuda.empty_cache()
+    sweep = (3 * nb + 20) * b * b * CPLX * ne
+    lead = 9 * b * b * CPLX * ne
+    free, _ = torch.cuda.mem_get_info()
+    ballast = torch.empty(free - sweep - lead - lead // 2, dtype=torch.uint8, device="cuda")
+    try:
+        got = solver.solve(dev.energies, out)
+        for k in KEYS:
+            assert torch.equal(got[k], want[k]), k
+    finally:
+        del ballast
+        _lib.check(lib.qtx_ctx_trim(ctx), ctx, "trim")
+        torch.cuda.empty_cache()
