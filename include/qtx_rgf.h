@@ -81,6 +81,9 @@ typedef int qtx_status;
 #define QTX_FLAG_RETARDED_OFFDIAG 0x10u /* also write X^R off-diagonal blocks into xr */
 #define QTX_FLAG_GRAPH 0x20u           /* qtx_transport_solve: capture the sweep of a single-batch call as a
                                           CUDA graph, cache it per (shapes, buffers, precision) and replay it */
+#define QTX_FLAG_LEADS_IN_TURN 0x40u   /* qtx_transport_solve: decimate the two leads one after the other at
+                                          every batch (half the work space, the same results; a small batch
+                                          otherwise takes both together) */
 
 typedef struct qtx_ctx qtx_ctx;
 typedef struct CUstream_st* qtx_stream; /* == cudaStream_t; NULL = legacy default stream */
@@ -342,9 +345,11 @@ qtx_status qtx_assemble_system(qtx_ctx* ctx, int64_t nnz, int64_t num_energies, 
                                int64_t stride_sigma, void* a, int64_t stride_a, qtx_stream stream);
 
 /* Device bytes one qtx_transport_solve call allocates for itself (recursion
- * state, couplings, Sancho-Rubio and, for QTX_PREC_MIXED, the slice buffers)
- * when it processes `energies_per_call` energies at a time; H and the outputs
- * are the caller's and not included.  Used for admission control. */
+ * state, couplings, Sancho-Rubio, the scratch of the block inverse and, for
+ * QTX_PREC_MIXED, the slice buffers) when it processes at most
+ * `energies_per_call` energies at a time; never less than for fewer energies.
+ * H and the outputs are the caller's and not included.  Used for admission
+ * control. */
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call,
                                int32_t precision);
 
@@ -361,7 +366,8 @@ size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t e
  * (<= 64) also takes every waiting FP64 request of the same b that fits the
  * budget, and solves them together in one qtx_transport_solve_grouped launch;
  * each still completes with its own status.  A request whose footprint
- * exceeds the whole budget is refused at submission (QTX_E_NOMEM).  The
+ * exceeds the whole budget runs with QTX_FLAG_LEADS_IN_TURN if it fits then,
+ * else it is refused at submission (QTX_E_NOMEM).  The
  * problem's device arrays (H, energies) and the outputs belong to the caller
  * and must stay valid until the request has completed.
  * ------------------------------------------------------------------------- */

@@ -35,6 +35,7 @@ QTX_FLAG_SYMMETRIC_OUT = 0x4
 QTX_FLAG_HOST_BUFFERS = 0x8
 QTX_FLAG_RETARDED_OFFDIAG = 0x10
 QTX_FLAG_GRAPH = 0x20
+QTX_FLAG_LEADS_IN_TURN = 0x40
 
 c_void_p = ctypes.c_void_p
 c_int32 = ctypes.c_int32

@@ -64,6 +64,11 @@ void launch_zinv(int n, int64_t batch, MatView a, MutView x, int* info, const in
 // Scratch that launch_zinv takes for one call.
 size_t zinv_workspace_bytes(int n, int64_t batch);
 
+// qtx_transport_footprint, of a call that decimates the leads together where
+// that is the faster form, or always in turn (QTX_FLAG_LEADS_IN_TURN).
+size_t transport_footprint(int num_blocks, int block_size, int64_t energies_per_call, int precision,
+                           bool leads_in_turn);
+
 // out = s + gamma_s * s2 + w^H - w  (n x n), in place allowed for out == s.
 void launch_skew_combine(int n, int64_t batch, MatView s, MatView w, MutView out, cudaStream_t stream);
 // x = x - x^H in place (n x n).

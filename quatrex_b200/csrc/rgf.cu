@@ -1146,13 +1146,13 @@ void transport_couplings(const TransportWS& w, const cplx* h_upper, cudaStream_t
 // together / in turn, ms: b = 64, 74 energies 3.29 / 4.70, 148 5.10 / 6.24, 296
 // 9.66 / 10.01; b = 128, 74 15.3 / 18.7, 148 29.98 / 30.12; b = 256, 37 50.8 /
 // 57.8, 74 92.6 / 100.2, 148 181.7 / 182.9.
-bool leads_together(int b, int64_t ne) { return ne <= (b <= 64 ? 148 : 74); }
+int64_t max_leads_together(int b) { return b <= 64 ? 148 : 74; }
 
 // Contacts of energies [e0, e0 + ne) (src/quatrex/electron/solver.py:305-386):
 // Sancho-Rubio on both leads (host-synchronising convergence checks), then
 // Sigma^R, Gamma, Sigma^<, Sigma^> and the (E + i eta) shifts, all into `w`.
 bool transport_contacts(qtx_ctx* ctx, const TransportWS& w, const qtx_transport_problem& P,
-                        const qtx_transport_outputs& O, int64_t e0, int64_t ne, cudaStream_t s) {
+                        const qtx_transport_outputs& O, int64_t e0, int64_t ne, bool in_turn, cudaStream_t s) {
   const int nb = w.nb, b = w.b;
   const int64_t bb = (int64_t)b * b;
   const cplx* h_diag = reinterpret_cast<const cplx*>(P.h_diag);
@@ -1178,7 +1178,7 @@ bool transport_contacts(qtx_ctx* ctx, const TransportWS& w, const qtx_transport_
   }
   bool ok = true;
   DevBuf both;  // where there is no room for both, one after the other
-  if (leads_together(b, ne)) both = DevBuf::attempt(sancho_rubio_bytes(b, 2 * ne), s);
+  if (!in_turn && ne <= max_leads_together(b)) both = DevBuf::attempt(sancho_rubio_bytes(b, 2 * ne), s);
   if (both) {
     ok = sancho_rubio_impl(ctx, b, {lead[0], lead[1]}, both, P.sr_tol, P.sr_max_iterations, s);
     both.release();
@@ -1376,7 +1376,7 @@ void transport_sweep(TransportWS w, const qtx_transport_problem& P, const qtx_tr
 }
 
 void transport_impl(qtx_ctx* ctx, const qtx_transport_problem& P, const qtx_transport_outputs& O, int prec,
-                    cudaStream_t s, bool& all_converged) {
+                    bool leads_in_turn, cudaStream_t s, bool& all_converged) {
   const int nb = P.num_blocks, b = P.block_size;
   const int64_t NE = P.num_energies;
   auto offs = batch_offsets(NE, P.max_batch_size > 0 ? P.max_batch_size : NE);
@@ -1389,7 +1389,7 @@ void transport_impl(qtx_ctx* ctx, const qtx_transport_problem& P, const qtx_tran
   launch_fill_int(w.info, (int64_t)nb * ne_max, 0, s);
   for (size_t q = 0; q + 1 < offs.size(); ++q) {
     const int64_t e0 = offs[q], ne = offs[q + 1] - offs[q];
-    all_converged = transport_contacts(ctx, w, P, O, e0, ne, s) && all_converged;
+    all_converged = transport_contacts(ctx, w, P, O, e0, ne, leads_in_turn, s) && all_converged;
     transport_sweep(w, P, O, e0, ne, prec, s);
   }
   read_info_or_throw(ctx, w.info, (int64_t)nb * ne_max, s, "transport_solve");
@@ -1400,7 +1400,7 @@ void transport_impl(qtx_ctx* ctx, const qtx_transport_problem& P, const qtx_tran
 // (shapes, buffers, precision) and replayed; the contacts run eagerly each call
 // (their convergence checks synchronise with the host).
 void transport_graph_impl(qtx_ctx* ctx, const qtx_transport_problem& P, const qtx_transport_outputs& O, int prec,
-                          cudaStream_t s, bool& all_converged) {
+                          bool leads_in_turn, cudaStream_t s, bool& all_converged) {
   const int nb = P.num_blocks, b = P.block_size;
   const int64_t ne = P.num_energies;
   if (ne == 0) return;
@@ -1433,7 +1433,7 @@ void transport_graph_impl(qtx_ctx* ctx, const qtx_transport_problem& P, const qt
   TransportWS w = carve_transport_ws(g->mem, nb, b, ne);
   transport_couplings(w, reinterpret_cast<const cplx*>(P.h_upper), s);
   launch_fill_int(w.info, (int64_t)nb * ne, 0, s);
-  all_converged = transport_contacts(ctx, w, P, O, 0, ne, s) && all_converged;
+  all_converged = transport_contacts(ctx, w, P, O, 0, ne, leads_in_turn, s) && all_converged;
   if (!g->exec) {
     std::lock_guard<std::mutex> capture_lock(g_capture_mutex);
     const int64_t before = ctx->launches;
@@ -1951,6 +1951,20 @@ qtx_status guarded(qtx_ctx* ctx, F&& f) {
 
 }  // namespace
 
+size_t transport_footprint(int num_blocks, int block_size, int64_t energies_per_call, int precision,
+                           bool leads_in_turn) {
+  if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
+  size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
+  // matrices of the largest decimation: of a batch of this size or of a smaller
+  // one (the last of a call) whose leads go together
+  int64_t mats = energies_per_call;
+  if (!leads_in_turn) mats = std::max(mats, 2 * std::min(energies_per_call, max_leads_together(block_size)));
+  bytes += sancho_rubio_bytes(block_size, mats) + zinv_workspace_bytes(block_size, mats);
+  if (precision == QTX_PREC_MIXED)
+    bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
+  return bytes + (4u << 20);  // allocator granularity
+}
+
 // ===========================================================================
 // C ABI
 // ===========================================================================
@@ -2040,14 +2054,7 @@ int64_t qtx_launch_count(const qtx_ctx* ctx) { return ctx ? ctx->launches : -1; 
 int64_t qtx_graph_replays(const qtx_ctx* ctx) { return ctx ? ctx->graph_replays : -1; }
 
 size_t qtx_transport_footprint(int32_t num_blocks, int32_t block_size, int64_t energies_per_call, int32_t precision) {
-  if (num_blocks < 2 || block_size < 1 || energies_per_call < 1) return 0;
-  size_t bytes = transport_ws_bytes(num_blocks, block_size, energies_per_call);
-  const int leads = leads_together(block_size, energies_per_call) ? 2 : 1;
-  bytes += sancho_rubio_bytes(block_size, leads * energies_per_call);
-  if (precision == QTX_PREC_MIXED)
-    bytes += mixed_workspace_bytes(block_size, block_size, block_size, energies_per_call, energies_per_call);
-  bytes += zinv_workspace_bytes(block_size, energies_per_call);
-  return bytes + (4u << 20);  // allocator granularity
+  return transport_footprint(num_blocks, block_size, energies_per_call, precision, false);
 }
 
 qtx_status qtx_ctx_release_graphs(qtx_ctx* ctx, qtx_stream stream) {
@@ -2533,8 +2540,9 @@ qtx_status qtx_transport_solve(qtx_ctx* ctx, const qtx_transport_problem* p, con
     if (p->num_energies == 0) return;  // an empty energy grid: nothing to solve
     const bool use_graph = (flags & QTX_FLAG_GRAPH) != 0 &&
                            (p->max_batch_size <= 0 || p->max_batch_size >= p->num_energies);
-    if (use_graph) transport_graph_impl(ctx, *p, *o, precision, reinterpret_cast<cudaStream_t>(stream), ok);
-    else transport_impl(ctx, *p, *o, precision, reinterpret_cast<cudaStream_t>(stream), ok);
+    const bool in_turn = (flags & QTX_FLAG_LEADS_IN_TURN) != 0;
+    if (use_graph) transport_graph_impl(ctx, *p, *o, precision, in_turn, reinterpret_cast<cudaStream_t>(stream), ok);
+    else transport_impl(ctx, *p, *o, precision, in_turn, reinterpret_cast<cudaStream_t>(stream), ok);
   });
   if (st == QTX_OK && !ok) {
     ctx->last_error = "Surface Green's function did not converge.";

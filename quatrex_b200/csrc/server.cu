@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/qtx_rgf.h"
+#include "kernels.h"
 
 namespace {
 
@@ -280,7 +281,12 @@ qtx_status qtx_server_submit(qtx_server* srv, const qtx_transport_problem* p, co
   // replayed and its work space would escape the admission budget
   req->flags = flags & ~QTX_FLAG_GRAPH;
   const int64_t ne_call = p->max_batch_size > 0 ? std::min(p->max_batch_size, p->num_energies) : p->num_energies;
-  req->footprint = qtx_transport_footprint(p->num_blocks, p->block_size, ne_call, precision);
+  const bool in_turn = (flags & QTX_FLAG_LEADS_IN_TURN) != 0;
+  req->footprint = transport_footprint(p->num_blocks, p->block_size, ne_call, precision, in_turn);
+  if (req->footprint > srv->budget && !in_turn) {
+    req->flags |= QTX_FLAG_LEADS_IN_TURN;
+    req->footprint = transport_footprint(p->num_blocks, p->block_size, ne_call, precision, true);
+  }
   if (groupable(srv, *req)) {
     // solved in a grouped launch: its work space when it runs alone
     const int32_t nb = p->num_blocks;

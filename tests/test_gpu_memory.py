@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+from oracle.rgf_oracle import get_batches
 from quatrex_b200 import _lib
 from quatrex_b200.transport import TransportSolver
 from quatrex_b200.workloads import make_device
@@ -86,3 +87,52 @@ def test_leads_in_turn_where_there_is_no_room_for_both():
         del ballast
         _lib.check(lib.qtx_ctx_trim(ctx), ctx, "trim")
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("b,ne,ne_call", [(64, 148, 148), (128, 74, 74), (256, 74, 74), (256, 149, 74), (300, 9, 9)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_transport_footprint_covers_the_call(b, ne, ne_call, precision):
+    """Both leads together, and (149 energies in batches of 75 and 74) a call
+    whose last batch decimates together after a larger one in turn."""
+    largest = max(get_batches(ne, ne_call)[0])
+    dev = make_device(num_blocks=2, block_size=b, num_energies=ne, seed=8)
+    solver = TransportSolver(dev, max_batch_size=ne_call, precision=precision)
+    out = solver.allocate_outputs(ne, KEYS)
+    prec = _lib.QTX_PREC_MIXED if precision == "mixed" else _lib.QTX_PREC_FP64
+    lib = _lib.load()
+    assert _peak(lambda: solver.solve(dev.energies, out)) <= lib.qtx_transport_footprint(2, b, largest, prec)
+
+
+def test_server_takes_the_leads_in_turn_to_fit_the_budget():
+    """A budget that holds one lead's decimation beside the sweep but not both:
+    the request is accepted, runs within the budget and returns the same bits."""
+    nb, b, ne = 2, 256, 40
+    dev = make_device(num_blocks=nb, block_size=b, num_energies=ne, seed=9)
+    solver = TransportSolver(dev, max_batch_size=ne)
+    want = solver.solve(dev.energies, keys=KEYS)
+    out = solver.allocate_outputs(ne, KEYS)
+    e = torch.from_numpy(dev.energies).cuda()
+    p = _lib.TransportProblem(
+        num_blocks=nb, block_size=b, num_energies=ne, h_diag=solver.h_diag.data_ptr(),
+        h_upper=solver.h_upper.data_ptr(), energies=e.data_ptr(), eta=dev.eta, mu_left=dev.mu_left,
+        mu_right=dev.mu_right, kt=dev.kt, sr_tol=dev.sr_tol, sr_max_iterations=dev.sr_max_iter, max_batch_size=ne)
+    o = _lib.TransportOutputs(**{k: out[k].data_ptr() for k in KEYS})
+    lib = _lib.load()
+    both = lib.qtx_transport_footprint(nb, b, ne, _lib.QTX_PREC_FP64)
+    budget = both - 9 * b * b * CPLX * ne
+    cfg = _lib.ServerConfig(device=torch.cuda.current_device(), slots=1, memory_budget=budget, group_max_block_size=0)
+    srv = ctypes.c_void_p()
+    assert lib.qtx_server_create(ctypes.byref(cfg), ctypes.byref(srv)) == _lib.QTX_OK
+    try:
+        def call():
+            rid, status, lat = ctypes.c_int64(), ctypes.c_int32(-1), ctypes.c_double()
+            assert lib.qtx_server_submit(srv, ctypes.byref(p), ctypes.byref(o), _lib.QTX_PREC_FP64, 0,
+                                         ctypes.byref(rid)) == _lib.QTX_OK
+            assert lib.qtx_server_wait(srv, rid, 60000, ctypes.byref(status), ctypes.byref(lat), None, 0) == 0
+            assert status.value == _lib.QTX_OK
+
+        assert _peak(call) <= budget
+    finally:
+        assert lib.qtx_server_destroy(srv) == 0
+    for k in KEYS:
+        assert torch.equal(out[k], want[k]), k

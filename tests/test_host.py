@@ -123,6 +123,22 @@ def test_transport_footprint_is_host_arithmetic():
     assert lib.qtx_transport_footprint(1, 64, 8, _lib.QTX_PREC_FP64) == 0
 
 
+@pytest.mark.parametrize("b", [64, 65, 256, 512])
+def test_transport_footprint_never_falls(b):
+    """A batch of up to 148 energies (b <= 64) or 74 decimates both leads at
+    once, a larger one in turn: the footprint of the larger batch still covers
+    the smaller one that the same call may end with.  At the switch it holds the
+    scratch of the block inverses of both leads (n > 64: 32 columns of panel per
+    matrix, 16 above 256)."""
+    lib = _lib.load()
+    fp = [lib.qtx_transport_footprint(4, b, ne, _lib.QTX_PREC_FP64) for ne in range(1, 320)]
+    assert all(x < y for x, y in zip(fp, fp[1:]))
+    ne = 148 if b <= 64 else 74
+    panel = 0 if b <= 64 else 16 * b * (32 if b <= 256 else 16)
+    sweep = 16 * (3 * 4 + 20) * b * b * ne
+    assert fp[ne - 1] >= sweep + 2 * ne * (9 * 16 * b * b + panel)
+
+
 def test_serving_call_size_fits_the_budget():
     """A request's energies per call: the tuned size capped by the request's
     energies, halved until one call's footprint fits the server budget; one
