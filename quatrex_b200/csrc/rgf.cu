@@ -335,13 +335,6 @@ struct Btd {
   bool dense(int k) const { return !index(k) && !empty(k); }
 };
 
-// A block of `m` is gathered from (or scattered to) a sparse pattern.
-bool has_sparse_block(const Btd& m) {
-  for (int k = 0; k < 3 * m.nb() - 2; ++k)
-    if (!m.empty(k) && !m.dense(k)) return true;
-  return false;
-}
-
 void validate_desc(const qtx_btd_desc* d, const char* name) {
   if (!d) throw QtxError(QTX_E_INVAL, std::string(name) + ": missing block descriptor");
   if (d->num_blocks < 1) throw QtxError(QTX_E_INVAL, std::string(name) + ": num_blocks < 1");
@@ -385,14 +378,15 @@ struct Workspace {
 };
 
 // Read view of block (i, j) for energies [e0, e0 + ne); sparse blocks are
-// gathered into `scratch` (ne * bmax^2 complex).
+// gathered into `scratch` (ne * bmax^2 complex, laid out as the work matrices
+// are, so a work matrix may be formed in place of the block it starts from).
 MatView in_block(const Btd& m, int i, int j, int64_t e0, int64_t ne, cplx* scratch, const Workspace& ws) {
   int k = bidx(i, j);
   int rows = m.size(i), cols = m.size(j);
   if (m.empty(k)) return MatView{ws.zero, cols, 0};
   cplx* base = m.data + e0 * m.d->stack_stride + m.off(k);
   if (m.dense(k)) return MatView{base, cols, m.d->stack_stride};
-  MutView out{scratch, cols, (int64_t)rows * cols};
+  MutView out{scratch, cols, (int64_t)ws.bmax * ws.bmax};
   launch_block_gather(rows, cols, ne, base, m.d->stack_stride, m.nnz(k), m.index(k), out, ws.s);
   return out;
 }
@@ -689,9 +683,9 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
   for (size_t q = 0; q + 1 < offs.size(); ++q) ne_max = std::max(ne_max, offs[q + 1] - offs[q]);
   if (ne_max == 0) return;
 
-  // Work matrices: 13, and 10 gather scratch ones when a block has a sparse pattern
-  const bool sparse = has_sparse_block(A.a) || has_sparse_block(A.sl) || has_sparse_block(A.sg);
-  const int NT = 13 + (sparse ? 10 : 0);
+  // Work matrices per energy.  A block with a sparse pattern is gathered into
+  // one that is free while the block is needed.
+  const int NT = 12;
   const size_t tmp = (size_t)bmax * bmax * ne_max;
   std::vector<int> cur_sizes(sizes.begin() + 1, sizes.end());
   size_t total = 3 * stack_elems(sizes, ne_max) + NT * tmp + (size_t)bmax * bmax;
@@ -706,16 +700,13 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
     stl = carve(cur, cur_sizes, ne_max, bmax);
     stg = carve(cur, cur_sizes, ne_max, bmax);
   }
-  std::vector<cplx*> T(NT);
+  cplx* T[NT];
   for (int q = 0; q < NT; ++q) { T[q] = cur; cur += tmp; }
   Workspace ws{s, ne_max, bmax, cur};
   launch_fill_int(reinterpret_cast<int*>(ws.zero), (int64_t)4 * bmax * bmax, 0, s);
   cur += (size_t)bmax * bmax;
   int* info = reinterpret_cast<int*>(cur);
   launch_fill_int(info, ne_max * nb, 0, s);
-  // gather scratch: 0-2 and 3-5 A_ji, A_ij, A_jj of even and odd blocks, 6-7
-  // S_ij, 8-9 S_jj of the two components
-  auto gather = [&](int k) { return sparse ? T[13 + k] : nullptr; };
 
   const void* const* obc_r = A.obc ? A.obc->retarded : nullptr;
   const void* const* obc_c[2] = {A.obc ? A.obc->lesser : nullptr, A.obc ? A.obc->greater : nullptr};
@@ -743,7 +734,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
     // ---- first block (rgf.py:207-231)
     {
       const int b0 = sizes[0];
-      MatView a00 = in_block(a, 0, 0, e0, ne, gather(2), ws);
+      MatView a00 = in_block(a, 0, 0, e0, ne, T[10], ws);
       MatView o = obc_view(obc_r, 0, b0, e0);
       if (o.ptr) {
         launch_axpby(b0, b0, ne, ONE, a00, MONE, o, tv(0, b0), s);
@@ -752,7 +743,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         zinv(b0, ne, a00, xr.view(0), info, nullptr, s);
       }
       for (int c = 0; c < 2; ++c) {
-        MatView sv = in_block(*Sc[c], 0, 0, e0, ne, gather(8 + c), ws);
+        MatView sv = in_block(*Sc[c], 0, 0, e0, ne, T[4 + 4 * c], ws);
         MatView o2 = obc_view(obc_c[c], 0, b0, e0);
         if (o2.ptr) {
           launch_axpby(b0, b0, ne, ONE, sv, ONE, o2, tv(4 + 4 * c, b0), s);
@@ -766,23 +757,25 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       grp.run();
     }
     // ---- forward sweep (rgf.py:233-295).  Work matrices: U 0, M 1, of
-    // component c W_c, V_c, Q_c, x_j Q_c from 2 + 4 c on, the second W 10.
+    // component c W_c, V_c, Q_c, x_j Q_c from 2 + 4 c on (a W that both share
+    // takes the places of W_0 and W_1 in turn); sparse blocks: A_ji 10 and 11 in
+    // turn, A_jj in M, A_ij 3 (no step holds V_0 when M is formed), S_ij and S_jj
+    // of component c in Q_c.
     // U = A_ji x_i and M = A_jj - Sigma^R_j - U A_ij of the next step ride with
     // the products of this one; X_c,j of a step without injection (pend) with
     // the first launch of the next.
     struct Couplings {
-      MatView ji, ij, jj;
+      MatView ji, jj;
     };
     auto couplings = [&](int j) {
-      const int i = j - 1, k = 3 * (j & 1);
-      return Couplings{in_block(a, j, i, e0, ne, gather(k), ws), in_block(a, i, j, e0, ne, gather(k + 1), ws),
-                       in_block(a, j, j, e0, ne, gather(k + 2), ws)};
+      return Couplings{in_block(a, j, j - 1, e0, ne, T[10 + (j & 1)], ws), in_block(a, j, j, e0, ne, T[1], ws)};
     };
     auto add_u = [&](int j, const Couplings& k) {
       grp.add(call(sizes[j], sizes[j - 1], sizes[j - 1], ONE, k.ji, OP_N, xr.view(j - 1), OP_N, tv(0, sizes[j - 1])));
     };
     auto add_m = [&](int j, const Couplings& k) {
-      grp.add(call(sizes[j], sizes[j], sizes[j - 1], MONE, tv(0, sizes[j - 1]), OP_N, k.ij, OP_N, tv(1, sizes[j]),
+      const MatView a_ij = in_block(a, j - 1, j, e0, ne, T[3], ws);
+      grp.add(call(sizes[j], sizes[j], sizes[j - 1], MONE, tv(0, sizes[j - 1]), OP_N, a_ij, OP_N, tv(1, sizes[j]),
                    k.jj, ONE, obc_view(obc_r, j, sizes[j], e0), MONE));
     };
     std::vector<GemmCall> pend;
@@ -820,7 +813,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         grp.run();
         for (int c = 0; c < 2; ++c)
           pend.push_back(call(bj, bj, bi, ONE, tv(5 + 4 * c, bi), OP_N, w, OP_C, Xc[c]->view(j)));
-        w_at = w_at == 2 ? 10 : 2;
+        w_at = w_at == 2 ? 6 : 2;
         now = next;
         continue;
       }
@@ -828,7 +821,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       for (int c = 0; c < 2; ++c) {
         // W = U S_ij (zero when S_ij is) ; V = X_i A_ji^H
         if (nz(c, i, j))
-          grp.add(call(bj, bj, bi, ONE, tv(0, bi), OP_N, in_block(*Sc[c], i, j, e0, ne, gather(6 + c), ws), OP_N,
+          grp.add(call(bj, bj, bi, ONE, tv(0, bi), OP_N, in_block(*Sc[c], i, j, e0, ne, T[4 + 4 * c], ws), OP_N,
                        tv(2 + 4 * c, bj)));
         grp.add(call(bi, bj, bi, ONE, Xc[c]->view(i), OP_N, now.ji, OP_C, tv(3 + 4 * c, bj)));
       }
@@ -839,7 +832,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         if (want_cur) {
           grp.add(call(bj, bj, bi, ONE, now.ji, OP_N, tv(3 + 4 * c, bj), OP_N, STc[c]->view(i)));
         } else {
-          const MatView s_jj = nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, gather(8 + c), ws) : MatView{};
+          const MatView s_jj = nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, T[4 + 4 * c], ws) : MatView{};
           grp.add(call(bj, bj, bi, ONE, now.ji, OP_N, tv(3 + 4 * c, bj), OP_N, tv(4 + 4 * c, bj), s_jj, ONE,
                        obc_view(obc_c[c], j, bj, e0), ONE));
         }
@@ -852,7 +845,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
           const MutView st = STc[c]->view(i);
           if (nz(c, i, j)) launch_skew_combine(bj, ne, st, w, st, s);
           const MatView s_jj =
-              nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, gather(8 + c), ws) : MatView{ws.zero, bj, 0};
+              nz(c, j, j) ? in_block(*Sc[c], j, j, e0, ne, T[4 + 4 * c], ws) : MatView{ws.zero, bj, 0};
           launch_axpby(bj, bj, ne, ONE, st, ONE, s_jj, qv, s);
           const MatView o2 = obc_view(obc_c[c], j, bj, e0);
           if (o2.ptr) launch_axpby(bj, bj, ne, ONE, qv, ONE, o2, qv, s);
@@ -880,13 +873,14 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       if (want_r) store.add(A.xr, n, n, xr.view(n), 0);
       store.run();
     }
-    // ---- backward sweep (rgf.py:307-404).  Work matrices: P1 0, P2 1, P3 10,
-    // P4 11, the new x_i 12, of component c Y, t1, t2, X_ij from 2 + 4 c on.
+    // ---- backward sweep (rgf.py:307-404).  Work matrices: P1 0, P2 1, P3 10 (then
+    // the new x_i), P4 11, of component c Y, t1, t2, X_ij from 2 + 4 c on; sparse
+    // blocks, which only the first launch reads: A_ij 3, A_ji 5, S_ij in t2.
     for (int i = nb - 2; i >= 0; --i) {
       const int j = i + 1, bi = sizes[i], bj = sizes[j];
-      MatView a_ij = in_block(a, i, j, e0, ne, gather(1), ws);
-      MatView a_ji = in_block(a, j, i, e0, ne, gather(0), ws);
-      const MutView p1 = tv(0, bj), p2 = tv(1, bi), p3 = tv(10, bj), p4 = tv(11, bi), gii = tv(12, bi);
+      MatView a_ij = in_block(a, i, j, e0, ne, T[3], ws);
+      MatView a_ji = in_block(a, j, i, e0, ne, T[5], ws);
+      const MutView p1 = tv(0, bj), p2 = tv(1, bi), p3 = tv(10, bj), p4 = tv(11, bi), gii = tv(10, bi);
       auto y = [&](int c) { return tv(2 + 4 * c, bj); };
       auto t1 = [&](int c) { return tv(3 + 4 * c, bi); };
       auto t2 = [&](int c) { return tv(4 + 4 * c, bj); };
@@ -897,7 +891,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       grp.add(call(bj, bi, bj, ONE, xr.view(j), OP_N, a_ji, OP_N, p2));
       for (int c = 0; c < 2; ++c)
         if (inj[c])
-          grp.add(call(bi, bj, bi, ONE, xr.view(i), OP_N, in_block(*Sc[c], i, j, e0, ne, gather(6 + c), ws), OP_N,
+          grp.add(call(bi, bj, bi, ONE, xr.view(i), OP_N, in_block(*Sc[c], i, j, e0, ne, T[4 + 4 * c], ws), OP_N,
                        y(c)));
       grp.run();
       // P3 = P1 X_jj (only injection and the off-diagonal X^R use it), P4 = P1 P2, t2 = P1 X_j
@@ -906,22 +900,21 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
       for (int c = 0; c < 2; ++c) grp.add(call(bi, bj, bj, ONE, p1, OP_N, Xc[c]->view(j), OP_N, t2(c)));
       grp.run();
       if (want_r_off) {
-        // X^R_ij = -P3 ; X^R_ji = -P2 x_i
-        launch_axpby(bi, bj, ne, MONE, p3, ZERO, {}, tv(12, bj), s);
-        store.add(A.xr, i, j, tv(12, bj), 0);
+        // X^R_ij = -P3 ; X^R_ji = -P2 x_i (in the place of X_0,ij, which follows)
+        launch_axpby(bi, bj, ne, MONE, p3, ZERO, {}, tv(5, bj), s);
+        store.add(A.xr, i, j, tv(5, bj), 0);
         store.run();
-        grp.add(call(bj, bi, bi, MONE, p2, OP_N, xr.view(i), OP_N, tv(12, bi)));
+        grp.add(call(bj, bi, bi, MONE, p2, OP_N, xr.view(i), OP_N, tv(5, bi)));
         grp.run();
-        store.add(A.xr, j, i, tv(12, bi), 0);
+        store.add(A.xr, j, i, tv(5, bi), 0);
         store.run();
       }
-      // t1 = P4 X_i - Y P3^H ; X_ij = Y X_jj^H - t2 - X_i P2^H ; G_ii = x_i + P4 x_i
+      // t1 = P4 X_i - Y P3^H ; X_ij = Y X_jj^H - t2 - X_i P2^H
       for (int c = 0; c < 2; ++c) {
         grp.add(call(bi, bi, bi, ONE, p4, OP_N, Xc[c]->view(i), OP_N, t1(c)));
         if (inj[c]) grp.add(call(bi, bj, bj, ONE, y(c), OP_N, xr.view(j), OP_C, xij(c), t2(c), MONE));
         else grp.add(call(bi, bj, bi, MONE, Xc[c]->view(i), OP_N, p2, OP_C, xij(c), t2(c), MONE));
       }
-      grp.add(call(bi, bi, bi, ONE, p4, OP_N, xr.view(i), OP_N, gii, xr.view(i), ONE));
       grp.run();
       for (int c = 0; c < 2; ++c) {
         if (!inj[c]) continue;
@@ -934,6 +927,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         // X_i += t2 P1^H + t1
         grp.add(call(bi, bi, bj, ONE, t2(c), OP_N, p1, OP_C, Xc[c]->view(i), Xc[c]->view(i), ONE, t1(c), ONE));
       }
+      grp.add(call(bi, bi, bi, ONE, p4, OP_N, xr.view(i), OP_N, gii, xr.view(i), ONE));  // G_ii = x_i + P4 x_i
       grp.run();
       for (int c = 0; c < 2; ++c) {
         store.add(*Oc[c], i, j, xij(c), 0);
@@ -949,7 +943,7 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
         launch_axpby(1, 1, ne, ONE, MatView{cur_out, 1, 1}, ZERO, {}, MutView{A.current + e0 * (nb - 1) + i, 1, nb - 1},
                      s);
       }
-      std::swap(xr.ptr[i], T[12]);
+      std::swap(xr.ptr[i], T[10]);
       if (want_r) store.add(A.xr, i, i, xr.view(i), 0);
       store.run();
     }

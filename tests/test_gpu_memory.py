@@ -9,6 +9,8 @@ import torch
 
 from oracle.rgf_oracle import get_batches
 from quatrex_b200 import _lib
+from quatrex_b200.datastructures import DSDBCOO
+from quatrex_b200.greens_function_solver import RGF
 from quatrex_b200.transport import TransportSolver
 from quatrex_b200.workloads import make_device
 
@@ -60,6 +62,29 @@ def test_sancho_rubio_holds_nine_matrices(n):
 
     panels = n * 32 * CPLX * ne if n > 64 else 0
     assert _peak(call) <= 9 * n * n * CPLX * ne + panels + SLACK
+
+
+@pytest.mark.parametrize("pattern", [False, True])
+@pytest.mark.parametrize("current", [False, True])
+def test_selected_solve_holds_twelve_work_matrices(pattern, current):
+    """Three block stacks (two more of couplings with the currents), twelve work
+    matrices and the inverse's panel scratch, whether the blocks are stored full
+    or as patterns."""
+    nb, b, ne = 6, 96, 20
+    dev = make_device(num_blocks=nb, block_size=b, num_energies=ne, seed=4)
+    d, u, lo = dev.system_blocks()
+    a = DSDBCOO.from_blocks(d, u, lo, device="cuda")
+    if pattern:
+        keep = np.random.default_rng(1).random(len(a.rows)) < 0.5
+        keep |= a.rows == a.cols
+        a = DSDBCOO(a.data[:, torch.from_numpy(keep).cuda()].contiguous(), a.rows[keep], a.cols[keep], a.block_sizes,
+                    a.stack_shape)
+    out = [DSDBCOO.zeros_like(a) for _ in range(3)]
+    solver = RGF(max_batch_size=ne)
+    call = lambda: solver.selected_solve(a, a, a, out=out, return_retarded=True, return_current=current)  # noqa: E731
+    call()  # pattern tables of the operands
+    mats = 3 * nb + 12 + (2 * (nb - 1) if current else 0)
+    assert _peak(call) <= (mats * b * b + b * 32) * CPLX * ne + SLACK
 
 
 def test_leads_in_turn_where_there_is_no_room_for_both():

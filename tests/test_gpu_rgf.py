@@ -17,6 +17,7 @@ import torch
 from scipy import sparse
 
 from oracle import rgf_oracle as orc
+from quatrex_b200 import _lib
 from quatrex_b200.datastructures import DSDBCOO, DSDBCSR
 from quatrex_b200.greens_function_solver import RGF, OBCBlocks
 from quatrex_b200.workloads import make_device
@@ -304,6 +305,61 @@ def test_selected_solve_does_not_depend_on_the_batch(sizes, scatter):
             if current:
                 # (the trace over a block is one CTA per energy in either case)
                 assert torch.equal(one[3][0], big[3][e])
+
+
+@pytest.mark.parametrize("inject", ["none", "some", "all"])
+@pytest.mark.parametrize("sizes", [[8] * 6, [12, 33, 7, 40, 65]])
+@pytest.mark.parametrize("return_current", [False, True])
+def test_sparse_operands_equal_dense_ones(sizes, inject, return_current, monkeypatch):
+    """Blocks stored as patterns are gathered into work matrices that are free
+    at that point of the recursion: every combination of injecting and other
+    steps, with retarded off-diagonal blocks, equals the same values stored as
+    full blocks (their missing entries as zeros) bit for bit."""
+    # the Python layer returns the diagonal blocks; ask for the couplings too
+    monkeypatch.setattr(_lib, "QTX_FLAG_RETURN_RETARDED", _lib.QTX_FLAG_RETURN_RETARDED | _lib.QTX_FLAG_RETARDED_OFFDIAG)
+    rng = np.random.default_rng(sum(sizes))
+    ne, nb = 5, len(sizes)
+
+    def cr(*shape):
+        x = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+        return x * (rng.random(shape[1:]) < 0.6)
+
+    d = [cr(ne, b, b) + 4 * np.sqrt(b) * np.eye(b) for b in sizes]
+    u = [cr(ne, p, q) for p, q in zip(sizes, sizes[1:])]
+    lo = [cr(ne, q, p) for p, q in zip(sizes, sizes[1:])]
+    dense_a = DSDBCOO.from_blocks(d, u, lo, device="cuda")
+    sigma = []
+    for c in range(2):
+        sd = [cr(ne, b, b) for b in sizes]
+        su = [cr(ne, p, q) for p, q in zip(sizes, sizes[1:])]
+        for i in range(nb):  # the two components inject at different blocks
+            if inject == "none" and i > 0 or inject == "some" and i % 3 != c:
+                sd[i] = np.zeros_like(sd[i])
+            if i < nb - 1 and (inject == "none" or inject == "some" and i % 4 != 2 + c):
+                su[i] = np.zeros_like(su[i])
+        sd = [x - x.conj().swapaxes(-1, -2) for x in sd]
+        sl = [-x.conj().swapaxes(-1, -2) for x in su]
+        sigma.append(DSDBCOO.from_blocks(sd, su, sl, device="cuda"))
+
+    def pattern(m):  # without the entries that are zero at every energy
+        keep = (m.data != 0).any(dim=0).cpu().numpy()
+        return DSDBCOO(m.data[:, torch.from_numpy(keep).cuda()].contiguous(), m.rows[keep], m.cols[keep],
+                       m.block_sizes, m.stack_shape)
+
+    solve = RGF(max_batch_size=2).selected_solve
+    full = [DSDBCOO.zeros_like(dense_a) for _ in range(3)]
+    got = [DSDBCOO.zeros_like(dense_a) for _ in range(3)]
+    r_full = solve(dense_a, *sigma, out=full, return_retarded=True, return_current=return_current)
+    r_got = solve(pattern(dense_a), *map(pattern, sigma), out=got, return_retarded=True,
+                  return_current=return_current)
+    for q in range(3):
+        assert torch.equal(full[q].data, got[q].data), q
+    if return_current:
+        assert torch.equal(r_full, r_got)
+    want = np.linalg.inv(dense_a.to_dense())
+    mask = np.zeros(want.shape[1:], dtype=bool)
+    mask[dense_a.rows, dense_a.cols] = True
+    assert _rel(full[2].to_dense(), want * mask) < TOL
 
 
 @pytest.mark.parametrize("b", [4, 40])
