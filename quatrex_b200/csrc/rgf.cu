@@ -501,9 +501,16 @@ struct BlockStack {
   MutView view(int i) const { return MutView{ptr[i], size[i], slot}; }
 };
 
-size_t stack_elems(const std::vector<int>& sizes, int64_t ne) {
-  int bmax = *std::max_element(sizes.begin(), sizes.end());
-  return (size_t)bmax * bmax * ne * sizes.size();
+// Work space of a recursion over `ne` energies at a time: its block stacks and
+// work matrices (a block with a sparse pattern is gathered into one that is free
+// while the block is needed), a zero block, the zero pivots.
+constexpr int INV_TEMPS = 7, SOLVE_TEMPS = 12;
+size_t recursion_bytes(int nb, int bmax, int64_t ne, int mats) {
+  return sizeof(cplx) * (size_t)bmax * bmax * ((size_t)mats * ne + 1) + sizeof(int) * (size_t)ne * nb;
+}
+size_t selected_inv_bytes(int nb, int bmax, int64_t ne) { return recursion_bytes(nb, bmax, ne, nb + INV_TEMPS); }
+size_t selected_solve_bytes(int nb, int bmax, int64_t ne, bool current) {
+  return recursion_bytes(nb, bmax, ne, 3 * nb + SOLVE_TEMPS + (current ? 2 * (nb - 1) : 0));
 }
 
 BlockStack carve(cplx*& cursor, const std::vector<int>& sizes, int64_t ne, int bmax) {
@@ -557,12 +564,11 @@ void selected_inv_impl(qtx_ctx* ctx, const Btd& a, const void* const* obc_r, con
   if (ne_max == 0) return;
 
   const size_t tmp = (size_t)bmax * bmax * ne_max;
-  const size_t total = stack_elems(sizes, ne_max) + 7 * tmp + (size_t)bmax * bmax;
-  DevBuf buf(total * sizeof(cplx) + sizeof(int) * ne_max * nb, s);
+  DevBuf buf(selected_inv_bytes(nb, bmax, ne_max), s);
   cplx* cur = buf.as<cplx>();
   BlockStack x = carve(cur, sizes, ne_max, bmax);
-  cplx* T[7];
-  for (int q = 0; q < 7; ++q) { T[q] = cur; cur += tmp; }
+  cplx* T[INV_TEMPS];
+  for (int q = 0; q < INV_TEMPS; ++q) { T[q] = cur; cur += tmp; }
   Workspace ws{s, ne_max, bmax, cur};
   launch_fill_int(reinterpret_cast<int*>(ws.zero), (int64_t)4 * bmax * bmax, 0, s);
   cur += (size_t)bmax * bmax;
@@ -683,14 +689,9 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
   for (size_t q = 0; q + 1 < offs.size(); ++q) ne_max = std::max(ne_max, offs[q + 1] - offs[q]);
   if (ne_max == 0) return;
 
-  // Work matrices per energy.  A block with a sparse pattern is gathered into
-  // one that is free while the block is needed.
-  const int NT = 12;
   const size_t tmp = (size_t)bmax * bmax * ne_max;
   std::vector<int> cur_sizes(sizes.begin() + 1, sizes.end());
-  size_t total = 3 * stack_elems(sizes, ne_max) + NT * tmp + (size_t)bmax * bmax;
-  if (want_cur) total += 2 * (size_t)bmax * bmax * ne_max * cur_sizes.size();
-  DevBuf buf(total * sizeof(cplx) + sizeof(int) * ne_max * nb, s);
+  DevBuf buf(selected_solve_bytes(nb, bmax, ne_max, want_cur), s);
   cplx* cur = buf.as<cplx>();
   BlockStack xr = carve(cur, sizes, ne_max, bmax);
   BlockStack xl = carve(cur, sizes, ne_max, bmax);
@@ -700,8 +701,8 @@ void selected_solve_impl(qtx_ctx* ctx, const SolveArgs& A, cudaStream_t s) {
     stl = carve(cur, cur_sizes, ne_max, bmax);
     stg = carve(cur, cur_sizes, ne_max, bmax);
   }
-  cplx* T[NT];
-  for (int q = 0; q < NT; ++q) { T[q] = cur; cur += tmp; }
+  cplx* T[SOLVE_TEMPS];
+  for (int q = 0; q < SOLVE_TEMPS; ++q) { T[q] = cur; cur += tmp; }
   Workspace ws{s, ne_max, bmax, cur};
   launch_fill_int(reinterpret_cast<int*>(ws.zero), (int64_t)4 * bmax * bmax, 0, s);
   cur += (size_t)bmax * bmax;
@@ -1628,13 +1629,15 @@ void set_parts(HostArr& a, const qtx_btd_desc* d, bool diag, bool upper, bool lo
   if (a.whole) a.parts.assign(1, {0, a.row_bytes});
 }
 
-// Energies per streamed batch: two staging sets plus the solver's work space
-// (about (3 nb + 32) bmax^2 complex per energy) in 70 % of the free memory.
-int64_t host_batch(int64_t max_batch, int64_t NE, size_t staging_per_energy, int nb, int bmax) {
+// Energies per streamed batch: two staging sets plus the recursion's work space
+// and the scratch of an inverse and of a mixed-precision product in 70 % of the
+// free memory.
+int64_t host_batch(int64_t max_batch, int64_t NE, size_t staging_per_energy, size_t recursion_per_energy, int bmax,
+                   int precision) {
   size_t free_b = 0, total_b = 0;
   QTX_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-  const size_t ws = sizeof(cplx) * (size_t)(3 * nb + 32) * bmax * bmax;
-  const size_t per = 2 * staging_per_energy + ws;
+  size_t per = 2 * staging_per_energy + recursion_per_energy + zinv_workspace_bytes(bmax, 1);
+  if (precision == QTX_PREC_MIXED) per += mixed_workspace_bytes(bmax, bmax, bmax, 1, 1);
   int64_t ne = (int64_t)((double)free_b * 0.7 / (double)std::max<size_t>(per, 1));
   ne = std::max<int64_t>(1, std::min<int64_t>({ne, max_batch, NE}));
   return ne;
@@ -2136,7 +2139,8 @@ qtx_status qtx_selected_inv(qtx_ctx* ctx, const qtx_btd_desc* a_desc, const void
       size_t per_e = 0;
       for (auto& x : arrs) per_e += x.row_bytes;
       const int64_t NE = a_desc->stack_size;
-      const int64_t ne_b = host_batch(max_batch_size, NE, per_e, nb, bmax);
+      const int64_t ne_b =
+          host_batch(max_batch_size, NE, per_e, selected_inv_bytes(nb, bmax, 1), bmax, precision);
       stream_host_batches(ctx, arrs, NE, ne_b, s, [&](int64_t, int64_t ne, int set) {
         qtx_btd_desc ad = batch_desc(a_desc, ne), od = batch_desc(out_desc, ne);
         std::vector<const void*> obc(nb, nullptr);
@@ -2228,7 +2232,8 @@ qtx_status qtx_selected_solve(qtx_ctx* ctx, const qtx_btd_desc* a_desc, const vo
       size_t per_e = 0;
       for (auto& x : arrs) per_e += x.row_bytes;
       const int64_t NE = a_desc->stack_size;
-      const int64_t ne_b = host_batch(max_batch_size, NE, per_e, nb, bmax);
+      const int64_t ne_b =
+          host_batch(max_batch_size, NE, per_e, selected_solve_bytes(nb, bmax, 1, want_cur), bmax, precision);
       stream_host_batches(ctx, arrs, NE, ne_b, s, [&](int64_t, int64_t ne, int set) {
         qtx_btd_desc ad = batch_desc(a_desc, ne), sld = batch_desc(sl_desc, ne), sgd = batch_desc(sg_desc, ne);
         qtx_btd_desc xld = batch_desc(xl_desc, ne), xgd = batch_desc(xg_desc, ne);

@@ -6,6 +6,7 @@ import ctypes
 import numpy as np
 import pytest
 import torch
+from scipy import sparse
 
 from oracle.rgf_oracle import get_batches
 from quatrex_b200 import _lib
@@ -161,3 +162,35 @@ def test_server_takes_the_leads_in_turn_to_fit_the_budget():
         assert lib.qtx_server_destroy(srv) == 0
     for k in KEYS:
         assert torch.equal(out[k], want[k]), k
+
+
+def test_host_stack_larger_than_the_device_memory_left():
+    """A host stack of blocks stored as patterns (small rows, so the recursion's
+    work space decides how many energies fit), with currents, and 2 GB of free
+    device memory: the streamed batches fit, and the results are those of a call
+    with all the memory."""
+    nb, b, ne = 80, 128, 24
+    rng = np.random.default_rng(2)
+    n = nb * b
+    rows = np.concatenate([np.arange(n), np.arange(n - b), np.arange(b, n)])
+    cols = np.concatenate([np.arange(n), np.arange(b, n), np.arange(n - b)])
+    values = rng.standard_normal(len(rows)) + 1j * rng.standard_normal(len(rows)) + 8.0 * (rows == cols)
+    m = DSDBCOO.from_sparray(sparse.coo_matrix((values, (rows, cols)), shape=(n, n)), [b] * nb, (ne,))
+    m.data *= rng.uniform(0.5, 1.5, (ne, 1))
+    solver = RGF(max_batch_size=ne)
+    call = lambda: solver.selected_solve(m, m, m, return_retarded=True, return_current=True)  # noqa: E731
+    want = call()
+    lib, ctx = _lib.load(), _lib.context(0)
+    _lib.check(lib.qtx_ctx_trim(ctx), ctx, "trim")
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    ballast = torch.empty(free - (2 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        got = call()
+    finally:
+        del ballast
+        _lib.check(lib.qtx_ctx_trim(ctx), ctx, "trim")
+        torch.cuda.empty_cache()
+    for q in range(3):
+        assert np.array_equal(got[q].data, want[q].data), q
+    assert np.array_equal(got[3], want[3])
