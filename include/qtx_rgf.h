@@ -115,6 +115,12 @@ qtx_status qtx_ctx_destroy(qtx_ctx* ctx);
 const char* qtx_last_error(const qtx_ctx* ctx);
 /* Device bytes the context may keep for workspaces (0 = no limit). */
 qtx_status qtx_ctx_set_memory_limit(qtx_ctx* ctx, size_t bytes);
+/* Copies of the host-buffer mode (QTX_FLAG_HOST_BUFFERS): parts of rows that
+ * lie more than max_pitch bytes apart are copied row by row instead of as one
+ * pitched copy (0: the device's own limit, above which a pitched copy is
+ * refused), and page_locked = 0 copies straight from the caller's arrays,
+ * without the ring of page-locked slots. */
+qtx_status qtx_ctx_set_host_copies(qtx_ctx* ctx, size_t max_pitch, int32_t page_locked);
 /* Release cached workspaces. */
 qtx_status qtx_ctx_trim(qtx_ctx* ctx);
 /* Library version string. */

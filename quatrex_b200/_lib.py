@@ -135,6 +135,7 @@ SIGNATURES = {
     "qtx_ctx_destroy": (c_int32, [c_void_p]),
     "qtx_last_error": (ctypes.c_char_p, [c_void_p]),
     "qtx_ctx_set_memory_limit": (c_int32, [c_void_p, ctypes.c_size_t]),
+    "qtx_ctx_set_host_copies": (c_int32, [c_void_p, ctypes.c_size_t, c_int32]),
     "qtx_ctx_trim": (c_int32, [c_void_p]),
     "qtx_launch_count": (c_int64, [c_void_p]),
     "qtx_graph_replays": (c_int64, [c_void_p]),

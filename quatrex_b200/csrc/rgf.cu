@@ -202,6 +202,8 @@ struct qtx_ctx {
   int* d_pinned = nullptr;     // their device alias: status words are stored there by a kernel
   cudaEvent_t step_event[2] = {nullptr, nullptr};  // status words of the last two decimation steps stored
   PinRing* ring = nullptr;     // page-locked staging of the host-buffer mode (process-wide pool)
+  bool use_ring = true;
+  size_t max_pitch = 0;        // bytes between rows of one pitched copy, 0: the device's limit
   bool timing = false;
   std::vector<TimedLaunch> timed;
   std::vector<cudaEvent_t> event_pool;
@@ -1643,6 +1645,22 @@ int64_t host_batch(int64_t max_batch, int64_t NE, size_t staging_per_energy, siz
   return ne;
 }
 
+// `len` bytes of each of `rows` rows, spitch bytes apart on the device and
+// dpitch apart in host memory.  A pitched copy of rows further apart than the
+// device's maximum (2 GiB, passed from 172 dense blocks of b = 512 on) is
+// refused, so such rows go one by one.
+void copy_rows_to_host(char* dst, size_t dpitch, const char* src, size_t spitch, size_t len, int64_t rows,
+                       size_t max_pitch, cudaStream_t cs) {
+  if (rows == 1 || (len == spitch && len == dpitch)) {
+    QTX_CUDA_TRY(cudaMemcpyAsync(dst, src, len * rows, cudaMemcpyDeviceToHost, cs));
+  } else if (std::max(spitch, dpitch) > max_pitch) {
+    for (int64_t r = 0; r < rows; ++r)
+      QTX_CUDA_TRY(cudaMemcpyAsync(dst + r * dpitch, src + r * spitch, len, cudaMemcpyDeviceToHost, cs));
+  } else {
+    QTX_CUDA_TRY(cudaMemcpy2DAsync(dst, dpitch, src, spitch, len, rows, cudaMemcpyDeviceToHost, cs));
+  }
+}
+
 // Copies between the caller's pageable arrays and device memory through a
 // PinRing: host memcpy into a slot (split over a few host threads), then an
 // async DMA on `cs`; a slot is reused only after its previous DMA completed.
@@ -1650,6 +1668,7 @@ int64_t host_batch(int64_t max_batch, int64_t NE, size_t staging_per_energy, siz
 struct RingCopier {
   PinRing& R;
   cudaStream_t cs;
+  size_t max_pitch;
   int next = 0;
   struct Pending {  // rows of len bytes, packed in the slot, pitch apart in host memory
     int slot;
@@ -1716,7 +1735,7 @@ struct RingCopier {
     for (int64_t r = 0; r < rows; r += per) {
       const int64_t nr = std::min(per, rows - r);
       const int sl = next_download_slot();
-      QTX_CUDA_TRY(cudaMemcpy2DAsync(R.slot(sl), len, dev + r * pitch, pitch, len, nr, cudaMemcpyDeviceToHost, cs));
+      copy_rows_to_host(R.slot(sl), len, dev + r * pitch, pitch, len, nr, max_pitch, cs);
       QTX_CUDA_TRY(cudaEventRecord(R.ev[sl], cs));
       pending.push_back({sl, host + r * pitch, len, pitch, nr});
     }
@@ -1817,8 +1836,14 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
       cur += ((a.row_bytes * ne_b + 255) / 256) * 256;
     }
   }
-  if (!ctx->ring) ctx->ring = ring_take();
-  bool use_ring = ctx->ring != nullptr;
+  size_t max_pitch = ctx->max_pitch;
+  if (!max_pitch) {
+    int limit = 0;
+    QTX_CUDA_TRY(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxPitch, ctx->device));
+    max_pitch = (size_t)limit;
+  }
+  if (ctx->use_ring && !ctx->ring) ctx->ring = ring_take();
+  bool use_ring = ctx->use_ring && ctx->ring != nullptr;
   if (use_ring)
     for (auto e : ctx->ring->ev) use_ring = use_ring && e != nullptr;
   cudaStream_t cs = nullptr;
@@ -1840,7 +1865,7 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
     QTX_CUDA_TRY(cudaEventRecord(solved, s));
     QTX_CUDA_TRY(cudaStreamWaitEvent(cs, solved, 0));
     if (use_ring) {
-      RingCopier rc{*ctx->ring, cs, 0, {}};
+      RingCopier rc{*ctx->ring, cs, max_pitch, 0, {}};
       CopyWorker w;
       auto upload = [&](int64_t e0, int64_t ne, int set) {
         return w.post([&, e0, ne, set] {
@@ -1893,8 +1918,8 @@ void stream_host_batches(qtx_ctx* ctx, std::vector<HostArr>& arrs, int64_t NE, i
         QTX_CUDA_TRY(cudaStreamWaitEvent(cs, solved, 0));
         for (auto& a : arrs)
           for (const auto& part : a.parts)
-            QTX_CUDA_TRY(cudaMemcpy2DAsync(a.hw + e0 * a.row_bytes + part.first, a.row_bytes, a.dev[set] + part.first,
-                                           a.row_bytes, part.second, ne, cudaMemcpyDeviceToHost, cs));
+            copy_rows_to_host(a.hw + e0 * a.row_bytes + part.first, a.row_bytes, a.dev[set] + part.first, a.row_bytes,
+                              part.second, ne, max_pitch, cs);
       }
     }
     QTX_CUDA_TRY(cudaStreamSynchronize(cs));
@@ -2031,6 +2056,13 @@ const char* qtx_last_error(const qtx_ctx* ctx) { return ctx ? ctx->last_error.c_
 qtx_status qtx_ctx_set_memory_limit(qtx_ctx* ctx, size_t bytes) {
   if (!ctx) return QTX_E_INVAL;
   ctx->mem_limit = bytes;
+  return QTX_OK;
+}
+
+qtx_status qtx_ctx_set_host_copies(qtx_ctx* ctx, size_t max_pitch, int32_t page_locked) {
+  if (!ctx) return QTX_E_INVAL;
+  ctx->max_pitch = max_pitch;
+  ctx->use_ring = page_locked != 0;
   return QTX_OK;
 }
 

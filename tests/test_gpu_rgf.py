@@ -363,10 +363,16 @@ def test_sparse_operands_equal_dense_ones(sizes, inject, return_current, monkeyp
 
 
 @pytest.mark.parametrize("b", [4, 40])
-def test_host_outputs_come_back_in_the_written_parts(b):
+@pytest.mark.parametrize("max_pitch,page_locked", [(0, 1), (1, 1), (0, 0), (1, 0)])
+def test_host_outputs_come_back_in_the_written_parts(b, max_pitch, page_locked, request):
     """Host outputs are not uploaded: the written blocks come back by parts
     (blocks of at least 16 KB) or by whole rows (smaller ones), and what the
-    call does not write keeps its values."""
+    call does not write keeps its values.  A pitch limit of one byte stands for
+    rows further apart than a pitched copy takes (2 GiB): they are copied one
+    by one; with and without the page-locked slots."""
+    lib, ctx = _lib.load(), _lib.context(torch.cuda.current_device())
+    request.addfinalizer(lambda: lib.qtx_ctx_set_host_copies(ctx, 0, 1))
+    assert lib.qtx_ctx_set_host_copies(ctx, max_pitch, page_locked) == _lib.QTX_OK
     dev = make_device(num_blocks=6, block_size=b, num_energies=5, seed=3)
     _, _, _, _, Ah, Zh, ob = _transport_inputs(dev, device=None)
     _, _, _, _, Ad, Zd, _ = _transport_inputs(dev, device="cuda")
