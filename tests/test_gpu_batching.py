@@ -36,8 +36,11 @@ def _close(a, b, tol=1e-12):
         assert np.linalg.norm(x - y) <= tol * max(np.linalg.norm(y), 1e-300), k
 
 
-def test_graph_replay_matches_eager():
-    dev = make_device(num_blocks=6, block_size=32, num_energies=8, seed=3)
+@pytest.mark.parametrize("b", [32, 65, 128])
+def test_graph_replay_matches_eager(b):
+    """(Above b = 64 every inverse of the captured sweep takes and frees its
+    scratch inside the capture.)"""
+    dev = make_device(num_blocks=6, block_size=b, num_energies=8, seed=3)
     eager = TransportSolver(dev, max_batch_size=8).solve(dev.energies, keys=OBSERVABLE_KEYS)
     s = TransportSolver(dev, max_batch_size=8, use_graph=True)
     out = s.allocate_outputs(8, OBSERVABLE_KEYS)
