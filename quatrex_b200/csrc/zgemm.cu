@@ -289,12 +289,16 @@ void launch_t(const Params& p, cudaStream_t stream) {
   qtx_launch(zgemm_dmma_kernel<TILE, OPA, OPB>, grid, THREADS, smem, stream, p);
 }
 
-// Waves of the resident CTAs that `tiles` take.
-template <int TILE>
-int64_t waves(int64_t tiles) {
+int sm_count() {
   int dev = 0, sms = 0;
   QTX_CUDA_TRY(cudaGetDevice(&dev));
   QTX_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  return sms;
+}
+
+// Waves of the resident CTAs that `tiles` take.
+template <int TILE>
+int64_t waves(int64_t tiles, int sms) {
   const int64_t resident = (int64_t)Cfg<TILE>::CTAS_PER_SM * sms;
   return (tiles + resident - 1) / resident;
 }
@@ -310,22 +314,22 @@ int64_t tiles_of(const Params& p) {
 // 9.0 / 17.4 us for 32 matrices of b = 64, 17.9 / 24.0 us for 24 of b = 100,
 // 66 / 86 us for 100 of b = 128, 0.796 / 0.878 ms for 24 of b = 512; 84 / 81
 // us for 16 of b = 256 (two waves against one).
-bool wide_tile(const Params& p) {
+bool wide_tile(const Params& p, int sms) {
   if (p.m > 32 * 65535) return true;  // grid.y
-  return 0.985 * 2.0 * (double)waves<64>(tiles_of<64>(p)) <= (double)waves<32>(tiles_of<32>(p));
+  return 0.985 * 2.0 * (double)waves<64>(tiles_of<64>(p), sms) <= (double)waves<32>(tiles_of<32>(p), sms);
 }
 
 template <int OPA, int OPB>
-void launch_op(const Params& p, cudaStream_t stream) {
-  if (wide_tile(p)) launch_t<64, OPA, OPB>(p, stream);
+void launch_op(const Params& p, int sms, cudaStream_t stream) {
+  if (wide_tile(p, sms)) launch_t<64, OPA, OPB>(p, stream);
   else launch_t<32, OPA, OPB>(p, stream);
 }
 
-void launch_one(const Params& p, cudaStream_t stream) {
-  if (p.op_a == OP_N && p.op_b == OP_N) launch_op<OP_N, OP_N>(p, stream);
-  else if (p.op_a == OP_N && p.op_b == OP_C) launch_op<OP_N, OP_C>(p, stream);
-  else if (p.op_a == OP_C && p.op_b == OP_N) launch_op<OP_C, OP_N>(p, stream);
-  else launch_op<OP_C, OP_C>(p, stream);
+void launch_one(const Params& p, int sms, cudaStream_t stream) {
+  if (p.op_a == OP_N && p.op_b == OP_N) launch_op<OP_N, OP_N>(p, sms, stream);
+  else if (p.op_a == OP_N && p.op_b == OP_C) launch_op<OP_N, OP_C>(p, sms, stream);
+  else if (p.op_a == OP_C && p.op_b == OP_N) launch_op<OP_C, OP_N>(p, sms, stream);
+  else launch_op<OP_C, OP_C>(p, sms, stream);
   qtx_check_launch("zgemm_dmma_kernel");
 }
 
@@ -369,16 +373,17 @@ constexpr int GROUP_WAVES = 4;
 void launch_zgemm_group(const GemmCall* calls, int count, cudaStream_t stream) {
   Group g;
   int n = 0;
+  const int sms = sm_count();
   auto flush = [&]() {
-    if (n == 1) launch_one(g.p[0], stream);
+    if (n == 1) launch_one(g.p[0], sms, stream);
     else if (n > 1) launch_several(g, n, stream);
     n = 0;
   };
   for (int q = 0; q < count; ++q) {
     if (calls[q].m <= 0 || calls[q].n <= 0 || calls[q].batch <= 0) continue;
     const Params p = params_of(calls[q]);
-    if (waves<32>(tiles_of<32>(p)) > GROUP_WAVES) {
-      launch_one(p, stream);
+    if (waves<32>(tiles_of<32>(p), sms) > GROUP_WAVES) {
+      launch_one(p, sms, stream);
       continue;
     }
     g.p[n++] = p;
@@ -389,5 +394,5 @@ void launch_zgemm_group(const GemmCall* calls, int count, cudaStream_t stream) {
 
 void launch_zgemm(const GemmCall& g, cudaStream_t stream) {
   if (g.m <= 0 || g.n <= 0 || g.batch <= 0) return;
-  launch_one(params_of(g), stream);
+  launch_one(params_of(g), sm_count(), stream);
 }

@@ -995,13 +995,16 @@ void launch_split(int n, int64_t batch, MatView a, MutView x, void* scratch, int
     const int w = std::min(W, n - k0);
     qtx_launch(zinv_panel_kernel<TPR, CPT, NW>, gb, 32 * NW, psmem, stream, n, batch, a.ptr, a.ld, a.stride, x.ptr,
                x.ld, x.stride, k0, sc, info, active);
+    qtx_check_launch("zinv_panel_kernel");
     // the first update reads A itself, so an out-of-place call needs no copy
     const MatView from = k0 == 0 ? a : MatView(x);
     qtx_launch(zinv_update_kernel, dim3(nslab, gb), UPD_THREADS, usmem, stream, n, batch, from.ptr, from.ld,
                from.stride, x.ptr, x.ld, x.stride, k0, w, W, sc, active);
+    qtx_check_launch("zinv_update_kernel");
   }
   qtx_launch(zinv_split_unscramble_kernel, dim3((n + UNS_ROWS - 1) / UNS_ROWS, gb), THREADS, xsmem, stream, n, batch,
              x.ptr, x.ld, x.stride, sc, active);
+  qtx_check_launch("zinv_split_unscramble_kernel");
 }
 
 }  // namespace
@@ -1032,7 +1035,6 @@ void launch_zinv(int n, int64_t batch, MatView a, MutView x, int* info, const in
     else if (n <= 256) launch_split<1, 32, 8>(n, batch, a, x, scratch, info, active, stream);
     else if (n <= 384) launch_split<1, 16, 12>(n, batch, a, x, scratch, info, active, stream);
     else launch_split<1, 16, 16>(n, batch, a, x, scratch, info, active, stream);
-    qtx_check_launch("zinv_panel_kernel");
     cudaFreeAsync(scratch, stream);
     return;
   }

@@ -283,6 +283,18 @@ def test_one_launch_and_panel_inverses_agree(tmp_path):
                 assert err < 2 * 4 * n * 2.0**-53 * cond[e], (n, e)
 
 
+@pytest.mark.parametrize("n,panels", [(32, 0), (64, 0), (65, 3), (100, 4), (256, 8), (300, 19), (512, 32)])
+def test_launch_count_of_an_inverse(n, panels):
+    """Every launch counts: one for a register inverse, two per panel and the
+    final unscrambling for the others, and the two of the status word."""
+    a = torch.eye(n, dtype=torch.complex128, device="cuda").repeat(2, 1, 1)
+    x = torch.empty_like(a)
+    lib, ctx = _lib.load(), _lib.context(0)
+    before = lib.qtx_launch_count(ctx)
+    _lib.check(lib.qtx_inv(ctx, n, 2, a.data_ptr(), n * n, x.data_ptr(), n * n, 0), ctx, "inv")
+    assert lib.qtx_launch_count(ctx) - before == 2 + (2 * panels + 1 if panels else 1)
+
+
 @pytest.mark.parametrize("n", [200, 256])
 @pytest.mark.parametrize("batch", [5, 130])
 def test_inverse_output_sixteen_bytes_off(n, batch):
