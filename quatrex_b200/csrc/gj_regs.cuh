@@ -75,12 +75,13 @@ __device__ __forceinline__ int gj_eliminate(cplx (&x)[CPT], int steps, int r_own
       f.y = __shfl_sync(0xffffffffu, f.y, src);
     }
     if (c_own == own) x[0] = cmk(0, 0);
-    // 0: not a candidate; else the bits of |Re| + |Im|, plus one.  The sign bit is
-    // cleared because a NaN may carry one: every candidate's key is then in
-    // [1, 2^63], so a row that was a pivot already is never named again (a NaN
-    // entry is the largest key and becomes the pivot).
+    // 0: not a candidate; else the bits of |Re| + |Im| with the sign bit set.  A
+    // NaN may carry either sign, so that bit must not decide: every candidate's
+    // key is in [2^63, 2^64), in the order of the values, and a row that was a
+    // pivot already is never named again (a NaN entry has the largest key and
+    // becomes the pivot).
     unsigned long long key =
-        used ? 0ull : ((unsigned long long)__double_as_longlong(cabs1(f)) & 0x7fffffffffffffffull) + 1ull;
+        used ? 0ull : (unsigned long long)__double_as_longlong(cabs1(f)) | 0x8000000000000000ull;
     const int best = __ffs(gj_argmax(key)) - 1;  // first lane of the first best row
     int pw = 0;
     if (lane == best) {
