@@ -1088,13 +1088,13 @@ struct TransportWS {
   cplx* C[10];  // g_L, g_R, SigR_L, SigR_R, SigL_L, SigL_R, SigG_L, SigG_R, Gam_L, Gam_R
   cplx *shift = nullptr, *tr = nullptr, *cl = nullptr, *cr = nullptr;
   double *occ_l = nullptr, *occ_r = nullptr;
-  int *info = nullptr, *its = nullptr;
+  int* info = nullptr;
 };
 
 size_t transport_ws_bytes(int nb, int b, int64_t ne_max) {
   const size_t bb = (size_t)b * b, tmp = bb * ne_max;
   const size_t cplx_elems = 2 * bb * std::max(nb - 1, 1) + 3 * (size_t)nb * tmp + 20 * tmp + 4 * ne_max;
-  return sizeof(cplx) * cplx_elems + sizeof(double) * 2 * ne_max + sizeof(int) * (nb + 2) * ne_max + 256;
+  return sizeof(cplx) * cplx_elems + sizeof(double) * 2 * ne_max + sizeof(int) * nb * ne_max + 256;
 }
 
 TransportWS carve_transport_ws(void* mem, int nb, int b, int64_t ne_max) {
@@ -1122,7 +1122,6 @@ TransportWS carve_transport_ws(void* mem, int nb, int b, int64_t ne_max) {
   w.occ_l = reinterpret_cast<double*>(cur);
   w.occ_r = w.occ_l + ne_max;
   w.info = reinterpret_cast<int*>(w.occ_r + ne_max);
-  w.its = w.info + nb * ne_max;
   return w;
 }
 

@@ -41,29 +41,22 @@ namespace {
 constexpr int THREADS = 256;
 constexpr int NWARPS = THREADS / 32;
 
+// Shape of the one-launch form (n > 64).
 struct InvShape {
-  int w;    // panel width
-  int wp;   // panel storage width (multiple of 8)
-  int cw;   // columns per update slab (multiple of 32)
-  int tpr;  // threads per panel row in the elimination
+  int w;   // panel width, a multiple of 8
+  int cw;  // columns per update slab (multiple of 32)
 };
 
 __host__ __device__ inline InvShape inv_shape(int n) {
   InvShape s;
-  s.w = n <= 32 ? n : (n <= 256 ? (n <= 96 ? 16 : 32) : 16);
-  s.wp = (s.w + 7) / 8 * 8;
-  int row_tiles = (n + 31) / 32;
-  int col_tiles = row_tiles >= NWARPS ? 1 : NWARPS / row_tiles;
-  s.cw = 32 * col_tiles;
-  int tpr = 1;
-  while (tpr * 2 * n <= THREADS && tpr * 2 <= s.w) tpr *= 2;
-  s.tpr = tpr;
+  s.w = n > 96 && n <= 256 ? 32 : 16;
+  const int row_tiles = (n + 31) / 32;
+  s.cw = 32 * (row_tiles >= NWARPS ? 1 : NWARPS / row_tiles);
   return s;
 }
 
-// complex elements of the update slabs: pivot rows and panel rows, double
-// buffered (none when one panel covers the matrix)
-__host__ __device__ inline int slab_elems(int n, const InvShape& s) { return s.w >= n ? 0 : 4 * s.w * (s.cw + 2); }
+// complex elements of the update slabs: pivot rows and panel rows, double buffered
+__host__ __device__ inline int slab_elems(const InvShape& s) { return 4 * s.w * (s.cw + 2); }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
   unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -77,13 +70,13 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 inline size_t inv_smem_bytes(int n) {
-  InvShape s = inv_shape(n);
-  size_t panel = (size_t)n * s.wp * sizeof(cplx);
-  size_t slabs = (size_t)slab_elems(n, s) * sizeof(cplx);
-  size_t ints = (size_t)(3 * n + 32 + 4) * sizeof(int);
-  size_t red = 2 * NWARPS * (sizeof(double) + sizeof(int) + sizeof(cplx));
-  size_t pivrow = (size_t)2 * NWARPS * s.wp * sizeof(cplx);  // pivot candidates, two column parities
-  return panel + slabs + ints + red + pivrow + 256;
+  const InvShape s = inv_shape(n);
+  const size_t panel = (size_t)n * s.w * sizeof(cplx);
+  const size_t slabs = (size_t)slab_elems(s) * sizeof(cplx);
+  const size_t ints = (size_t)(3 * n + 32 + 4) * sizeof(int);
+  // pivot candidates of two column parities (several rows a thread)
+  const size_t cand = 2 * NWARPS * (sizeof(double) + sizeof(int) + (1 + s.w) * sizeof(cplx));
+  return panel + slabs + ints + (n > THREADS ? cand : 0) + 256;
 }
 
 // swizzled panel index: row r, column c (c < wp, wp multiple of 8)
@@ -124,7 +117,8 @@ __device__ __forceinline__ void argmax_combine(double& v, int& i, double v2, int
   }
 }
 
-// Shared-memory arrays of one matrix's elimination (see zinv_gj_kernel).
+// Shared-memory arrays of one matrix's elimination (see zinv_gj_kernel); those
+// from red_v on with several rows a thread only.
 struct GjSmem {
   cplx* P;
   int* pos2row;
@@ -137,10 +131,10 @@ struct GjSmem {
   cplx* cand;
 };
 
-__device__ inline GjSmem gj_smem_layout(unsigned char* base, int n, int wp, int slab) {
+__device__ inline GjSmem gj_smem_layout(unsigned char* base, int n, int w, int slab) {
   GjSmem s;
   s.P = reinterpret_cast<cplx*>(base);
-  cplx* Rs = s.P + (size_t)n * wp;
+  cplx* Rs = s.P + (size_t)n * w;
   s.pos2row = reinterpret_cast<int*>(Rs + slab);
   s.row2pos = s.pos2row + n;
   s.perm = s.row2pos + n;  // swap partner of each column (final unscramble)
@@ -159,12 +153,12 @@ __device__ inline GjSmem gj_smem_layout(unsigned char* base, int n, int wp, int 
 // Eliminates a panel of at most CPT columns and of up to RPT * THREADS rows
 // that the threads of the CTA hold RPT rows each (row r0 + q * THREADS in
 // reg[q]): the steps of gj_eliminate for more rows than threads.  Column kk of the
-// register rows is picked by selects.  24 matrices of n = 512 take 11.3 ms; 12.0
+// register rows is picked by selects.  24 matrices of n = 512 take 11.1 ms; 12.0
 // with all columns unrolled and static, 12.8 with one update formula for the
 // pivot row and the others on top, as in gj_eliminate (registers).
 template <int RPT, int CPT>
-__device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, int k0, int w, int WP,
-                                                  const GjSmem& sm, int& zero_pivot) {
+__device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, int k0, int w, const GjSmem& sm,
+                                                  int& zero_pivot) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   bool used[RPT];
 #pragma unroll
@@ -206,7 +200,7 @@ __device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, 
       argmax_combine(bv, bi, v2, i2);
     }
     const int slot = (kk & 1) * NWARPS;
-    cplx* my_cand = sm.cand + (size_t)(slot + warp) * WP;
+    cplx* my_cand = sm.cand + (slot + warp) * CPT;
 #pragma unroll
     for (int q = 0; q < RPT; ++q)
       if (tid + q * THREADS == bi) {
@@ -231,7 +225,7 @@ __device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, 
       argmax_combine(v, p, v2, i2);
     }
     const int pw = (p % THREADS) >> 5;  // the warp that holds row p published it
-    const cplx* prow = sm.cand + (size_t)(slot + pw) * WP;
+    const cplx* prow = sm.cand + (slot + pw) * CPT;
     const cplx piv = sm.red_piv[slot + pw];
     if (piv.x == 0.0 && piv.y == 0.0 && !zero_pivot) zero_pivot = k0 + kk + 1;
     const cplx d = crecip_pivot(piv);
@@ -262,8 +256,9 @@ __device__ __forceinline__ void gj_eliminate_rows(cplx (&reg)[RPT][CPT], int n, 
 // order).  TPR threads a row of CPT columns each, or (TPR = 1) RPT rows a
 // thread.  Ends with a CTA barrier.
 template <int TPR, int RPT, int CPT>
-__device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cplx* X, int64_t ldx, const GjSmem& sm,
+__device__ __forceinline__ void gj_panel(int n, int k0, int w, const cplx* X, int64_t ldx, const GjSmem& sm,
                                          int& zero_pivot) {
+  constexpr int W = TPR * CPT;
   static_assert(TPR == 1 || RPT == 1, "several rows a thread: whole rows");
   cplx* P = sm.P;
   int* pos2row = sm.pos2row;
@@ -275,7 +270,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
     // element in flight at once (asynchronous copies)
     for (int idx = tid; idx < n * w; idx += THREADS) {
       int r = idx / w, c = idx % w;
-      cp_async16(&P[pidx(r, c, WP)], &X[(int64_t)r * ldx + k0 + c], true);
+      cp_async16(&P[pidx(r, c, W)], &X[(int64_t)r * ldx + k0 + c], true);
     }
     cp_async_commit();
     for (int r = tid; r < n; r += THREADS) {
@@ -294,7 +289,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
 #pragma unroll
       for (int j = 0; j < CPT; ++j) {
         const int r = r_own + q * rstride, c = c_own + j * TPR;
-        reg[q][j] = (r < n && c < w) ? P[pidx(r, c, WP)] : cmk(0, 0);
+        reg[q][j] = (r < n && c < w) ? P[pidx(r, c, W)] : cmk(0, 0);
       }
     // rows before k0 are the pivots of earlier panels (rows are in the new order now)
     int turned = 0;
@@ -304,7 +299,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
       if (zero && !zero_pivot) zero_pivot = k0 + zero;
       turned = w / TPR;
     } else {
-      gj_eliminate_rows<RPT, CPT>(reg, n, k0, w, WP, sm, zero_pivot);
+      gj_eliminate_rows<RPT, CPT>(reg, n, k0, w, sm, zero_pivot);
     }
     // classic row-swap semantics of the panel's pivots: position k0 + kk
     // receives row pivs[kk], the displaced row goes to the pivot's position
@@ -326,7 +321,7 @@ __device__ __forceinline__ void gj_panel(int n, int k0, int w, int WP, const cpl
 #pragma unroll
       for (int j = 0; j < CPT; ++j) {
         const int r = r_own + q * rstride, c = ((j + turned) % CPT) * TPR + c_own;
-        if (r < n && c < w) P[pidx(r, c, WP)] = reg[q][j];
+        if (r < n && c < w) P[pidx(r, c, W)] = reg[q][j];
       }
     __syncthreads();
 }
@@ -338,11 +333,12 @@ __global__ void __launch_bounds__(THREADS, 1)
   qtx_grid_dependency();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const InvShape shp = inv_shape(n);
-  const int W = shp.w, WP = shp.wp, CW = shp.cw;
+  constexpr int W = TPR * CPT;  // = shp.w
+  const int CW = shp.cw;
   const int LDR = CW + 2;
-  const GjSmem sm = gj_smem_layout(smem_raw, n, WP, slab_elems(n, shp));
+  const GjSmem sm = gj_smem_layout(smem_raw, n, W, slab_elems(shp));
   cplx* P = sm.P;
-  cplx* Rs = P + (size_t)n * WP;  // two slabs of W x LDR (pivot rows, panel rows)
+  cplx* Rs = P + (size_t)n * W;  // two slabs of W x LDR (pivot rows, panel rows)
   int* pos2row = sm.pos2row;
   int* perm = sm.perm;
 
@@ -365,7 +361,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     for (int k0 = 0; k0 < n; k0 += W) {
       const int w = min(W, n - k0);
-      gj_panel<TPR, RPT, CPT>(n, k0, w, WP, X, ldx, sm, zero_pivot);
+      gj_panel<TPR, RPT, CPT>(n, k0, w, X, ldx, sm, zero_pivot);
 
       // ---- 3. rank-w update of the other columns, slabs of CW columns.
       // Output position i reads X[sigma(i)], and sigma(i) is either i itself or
@@ -489,7 +485,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 int pr = prow_idx[mi][h];
-                af[mi][h] = (pr >= 0 && kc < w) ? P[pidx(pr, kc, WP)] : cmk(0, 0);
+                af[mi][h] = (pr >= 0 && kc < w) ? P[pidx(pr, kc, W)] : cmk(0, 0);
               }
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni) bf[ni] = (kc < w) ? R[kc * LDR + col0 + ni * 8 + g] : cmk(0, 0);
@@ -530,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       // ---- panel columns: final panel values in the new row order
       for (int idx = tid; idx < n * w; idx += THREADS) {
         int i = idx / w, c = idx % w;
-        X[(int64_t)i * ldx + k0 + c] = P[pidx(pos2row[i], c, WP)];
+        X[(int64_t)i * ldx + k0 + c] = P[pidx(pos2row[i], c, W)];
       }
       // rows are now in the new order: the pivot rows so far sit at positions < k0 + w
       __syncthreads();
@@ -550,7 +546,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
     __syncthreads();
     {
-      const int rows_per_slab = max(1, (int)((size_t)n * WP / n));
+      constexpr int rows_per_slab = W;
       for (int r0 = 0; r0 < n; r0 += rows_per_slab) {
         int nr = min(rows_per_slab, n - r0);
         for (int idx = tid; idx < nr * n; idx += THREADS) {
@@ -1038,14 +1034,10 @@ void launch_zinv(int n, int64_t batch, MatView a, MutView x, int* info, const in
     cudaFreeAsync(scratch, stream);
     return;
   }
-  const InvShape s = inv_shape(n);
-  // every panel row / column must be owned by the elimination mapping
-  const int rpt = (n + (THREADS / s.tpr) - 1) / (THREADS / s.tpr);
-  const int cpt = (s.w + s.tpr - 1) / s.tpr;
-  if (s.tpr == 1 && rpt == 1 && cpt <= 32) launch_inv_r<1, 1, 32>(n, batch, a, x, info, active, stream);
-  else if (s.tpr == 1 && rpt == 2 && cpt <= 16) launch_inv_r<1, 2, 16>(n, batch, a, x, info, active, stream);
-  else if (s.tpr == 2 && rpt == 1 && cpt <= 8) launch_inv_r<2, 1, 8>(n, batch, a, x, info, active, stream);
-  else if (s.tpr == 2 && rpt == 1 && cpt <= 16) launch_inv_r<2, 1, 16>(n, batch, a, x, info, active, stream);
-  else throw QtxError(QTX_E_UNSUPPORTED, "qtx inverse: block size outside the supported shapes");
+  // the instances of inv_shape's panel widths: W = TPR * CPT
+  if (n <= 96) launch_inv_r<2, 1, 8>(n, batch, a, x, info, active, stream);
+  else if (n <= 128) launch_inv_r<2, 1, 16>(n, batch, a, x, info, active, stream);
+  else if (n <= 256) launch_inv_r<1, 1, 32>(n, batch, a, x, info, active, stream);
+  else launch_inv_r<1, 2, 16>(n, batch, a, x, info, active, stream);
   qtx_check_launch("zinv_gj_kernel");
 }
