@@ -438,12 +438,12 @@ GemmCall gemm_call(int m, int n, int k, int64_t batch, cplx alpha, MatView a, in
   return g;
 }
 
-// Independent block products of one step of a recursion, in one launch (the
+// Independent block products of one step of a recursion, issued together (the
 // mixed form runs them one by one).  A small product leaves most of the GPU
 // idle and costs its latency whatever else runs beside it (32 matrices of
-// b = 64 are 128 tiles of 592 resident ones); at large sizes the products of
-// a step share their operands in L2 and a single last wave.  The results do
-// not depend on the grouping.
+// b = 64 are 128 tiles of 592 resident ones), so those share a launch; one that
+// fills the GPU for several waves keeps its own (launch_zgemm_group).  The
+// results do not depend on the grouping.
 struct GemmGroup {
   cudaStream_t s;
   int precision;

@@ -21,7 +21,7 @@
 //     8-wide K slices; per output element the K order and the DMMA sequence
 //     are those of zgemm_dmma_kernel.
 //   * cta_inverse: Gauss-Jordan with implicit partial pivoting (gj_regs.cuh),
-//     the matrix in registers with THREADS / BT threads per row, one barrier
+//     the matrix in registers with THREADS / BT threads per row, two barriers
 //     per column, the row and column permutations applied on the store.
 // There are no inter-CTA waits: the only shared state is the work counter
 // and the error flags.
@@ -64,8 +64,8 @@ constexpr size_t smem_bytes() {
   return sizeof(cplx) * GCfg<BT>::REGION + sizeof(Misc<BT>);
 }
 
-// Dynamic shared memory: the product staging ring (or the inverse's pivot
-// candidates) followed by Misc.  The helpers below are separate functions,
+// Dynamic shared memory: the product staging ring (or the inverse's shared
+// state, GjRegs) followed by Misc.  The helpers below are separate functions,
 // so they derive these pointers from the __shared__ symbol themselves: a
 // pointer handed in as an argument would turn every access into a generic one.
 extern __shared__ __align__(16) unsigned char grouped_smem[];

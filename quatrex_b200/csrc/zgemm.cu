@@ -9,9 +9,10 @@
 // K step 16, double-buffered cp.async pipeline, 4 warps, and two CTA tiles:
 //   64x64, warp tile 32x32, two CTAs per SM (80 KB each)
 //   32x32, warp tile 16x16, four CTAs per SM (40 KB each)
-// Bound by the DMMA pipe (87-90 % active in either form where the tiles fill
-// whole waves), so the choice is the one with the shorter last wave: see
-// wide_tile().  Per output element both run the same DMMA sequence, so the
+// Bound by the DMMA pipe where the tiles fill whole waves (89 % active with
+// 64x64 tiles at b = 256, 148 matrices; 83 % with 32x32 ones at b = 96, 592
+// matrices; 67 % at b = 100, where a third of the tiles' area is padding), so
+// the choice is the one with the shorter last wave: see wide_tile().  Per output element both run the same DMMA sequence, so the
 // result does not depend on the tile.
 //
 // Tried and not kept: three real products instead of four (Gauss's identity,
