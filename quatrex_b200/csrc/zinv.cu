@@ -628,8 +628,9 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW)
 // Bounds: the panel by its chain of dependent steps (about 2000 cycles each at
 // 256 rows), the update by the latency of its loads and DMMAs (DMMA pipe 61 %
 // active and 2.2 TB/s of DRAM traffic at b = 256, 148 matrices; 56 % and 3.3
-// TB/s at b = 512, 40 matrices).  Measured on B200, ms per call, against three launches per panel (the pivot rows copied by one of their
-// own) below 80-124 matrices and the one-launch kernel of that time above:
+// TB/s at b = 512, 40 matrices).  Measured on B200, ms per call, against three
+// launches per panel (the pivot rows copied by one of their own) below 80-124
+// matrices and the one-launch kernel of that time above:
 //     b = 100,  24 matrices 0.18 (0.28)     b = 128, 100 matrices 0.27 (0.41)
 //     b = 256,  16 matrices 0.54 (0.82)     b = 256,  64 matrices 0.84 (1.26)
 //     b = 256, 148 matrices 1.31 (1.65)     b = 300,  20 matrices 0.84 (1.43)
