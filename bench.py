@@ -498,6 +498,17 @@ def _mixed_line(args, dev, E, step_energies, stream, local, fp64_value):
                     "Sancho-Rubio in FP64; same outputs as the FP64 line"}
 
 
+def _dropin_bytes(nb, b, ne):
+    """(host to device, device to host) bytes of one drop-in call on host data:
+    the rows of A, Sigma^< and Sigma^> and the six contact blocks go up; every
+    block of G^< and G^> and the diagonal blocks of G^R come back (blocks below
+    16 KB as whole rows, which then go up as well)."""
+    block = 16 * b * b * ne
+    row = (3 * nb - 2) * block
+    whole = 16 * b * b < 16 << 10 and nb > 1
+    return 3 * row + 6 * block + whole * row, 2 * row + (row if whole else nb * block)
+
+
 def _e2e_dropin(args):
     """The plugin call RGF.selected_solve(return_retarded) on NumPy DSDBCOO
     matrices of the nb=64, b=256 device (32 energies, batches of 16): every
@@ -536,9 +547,9 @@ def _e2e_dropin(args):
         solver.selected_solve(A, Z, Z, obc_blocks=ob, out=outs, return_retarded=True)
     torch.cuda.synchronize()
     dt = time.perf_counter() - t0
-    row_bytes = A.data.shape[-1] * 16
-    return {"value": round(ne * steps / dt, 3), "unit": "solves/s", "h2d_bytes_per_step": int(3 * ne * row_bytes),
-            "d2h_bytes_per_step": int(3 * ne * row_bytes), "steps": steps, "warmup": 2,
+    h2d, d2h = _dropin_bytes(nb, b, ne)
+    return {"value": round(ne * steps / dt, 3), "unit": "solves/s", "h2d_bytes_per_step": h2d,
+            "d2h_bytes_per_step": d2h, "steps": steps, "warmup": 2,
             "path": "RGF.selected_solve(a, sigma_lesser, sigma_greater, obc_blocks, out=[xl, xg, xr], "
                     "return_retarded=True) on NumPy DSDBCOO -> qtx_selected_solve with QTX_FLAG_HOST_BUFFERS",
             "config": {"num_blocks": nb, "block_size": b, "energies": ne, "max_batch_size": batch,
@@ -725,12 +736,11 @@ def run_dropin(args):
         torch.cuda.synchronize()
         dt = time.perf_counter() - t0
         lines[where] = ne * args.steps / dt
-    row_bytes = A.data.shape[-1] * 16
+    h2d, d2h = _dropin_bytes(nb, b, ne)
     print(json.dumps({
         "metric": "rgf_energy_solves_per_s", "impl": "ours", "workload": "dropin_selected_solve",
         "value": lines["device"], "unit": "solves/s",
-        "e2e": {"value": lines["host"], "unit": "solves/s", "h2d_bytes_per_step": int(6 * ne * row_bytes),
-                "d2h_bytes_per_step": int(3 * ne * row_bytes),
+        "e2e": {"value": lines["host"], "unit": "solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "path": "NumPy DSDBCOO -> QTX_FLAG_HOST_BUFFERS (streamed batches)"},
         "config": {"num_blocks": nb, "block_size": b, "energies": ne, "max_batch_size": args.dropin_batch,
                    "outputs": "G^<, G^> (all BTD blocks), G^R diagonal", "steps": args.steps},

@@ -29,6 +29,21 @@ def test_reference_arm_json_line():
     assert "nb=64 b=256" in line["config"]["workload"]
 
 
+@pytest.mark.parametrize("nb,b,ne", [(64, 256, 32), (16, 64, 32), (5, 16, 3), (1, 8, 2)])
+def test_dropin_bytes(nb, b, ne):
+    """The bytes of a drop-in call, against the blocks it takes and returns: G^R
+    comes back by diagonal blocks of at least 16 KB, else as whole rows that were
+    sent up first."""
+    import bench
+
+    up, down = bench._dropin_bytes(nb, b, ne)
+    block = 16 * b * b * ne
+    blocks = nb + 2 * (nb - 1)
+    by_parts = nb == 1 or 16 * b * b >= 16384
+    assert up == block * (3 * blocks + 6 + (0 if by_parts else blocks))
+    assert down == block * (2 * blocks + (nb if by_parts else blocks))
+
+
 @pytest.mark.parametrize("nb,its,units", [(64, (22, 22), 3 + 2 + 63 * 19 + 6 + 2 * (7 * 22 + 1)),
                                           (2, (1, 3), 3 + 2 + 19 + 6 + 8 + 22)])
 def test_flop_accounting(nb, its, units):
